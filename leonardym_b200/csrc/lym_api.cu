@@ -190,14 +190,15 @@ void dev_free(lym_context *c, void *p, size_t bytes)
     }
 }
 
-// a zeroed buffer of the given size from the idle blocks, else newly allocated
-void *block_alloc(lym_context *c, size_t bytes)
+// a buffer of the given size from the idle blocks (zeroed unless its user overwrites it whole),
+// else newly allocated (zeroed)
+void *block_alloc(lym_context *c, size_t bytes, bool zeroed = true)
 {
     for (size_t i = 0; i < c->blocks.size(); ++i)
         if (c->blocks[i].first == bytes) {
             void *p = c->blocks[i].second;
             c->blocks.erase(c->blocks.begin() + i);
-            CK(cudaMemsetAsync(p, 0, bytes, c->st));
+            if (zeroed) CK(cudaMemsetAsync(p, 0, bytes, c->st));
             return p;
         }
     return dev_alloc(c, bytes);
@@ -215,7 +216,9 @@ struct DevBuf {
     lym_context *c;
     void *p = nullptr;
     size_t n = 0;
-    DevBuf(lym_context *ctx, size_t bytes) : c(ctx), p(block_alloc(ctx, bytes)), n(bytes) {}
+    DevBuf(lym_context *ctx, size_t bytes, bool zeroed = true) : c(ctx), p(block_alloc(ctx, bytes, zeroed)), n(bytes)
+    {
+    }
     ~DevBuf()
     {
         if (p) block_free(c, p, n);
@@ -3640,10 +3643,10 @@ static int do_fermion_force(lym_context *c, int op_id, int n, const double *cons
         CK(cudaMemcpyAsync(t + 2 * n * sizeof(void *), weights, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
         const int clover = kind_has_clover(op.kind) ? 1 : 0;
         std::unique_ptr<DevBuf> scratch;
-        if (clover) scratch.reset(new DevBuf(c, fermion_force_scratch_bytes(c->g)));
+        if (clover) scratch.reset(new DevBuf(c, fermion_force_scratch_bytes(c->g), false));
         launch_fermion_force(c->g, ge.dev, n, (const double2 *const *)t, (const double2 *const *)(t + n * sizeof(void *)),
                              (const double *)(t + 2 * n * sizeof(void *)), op.kappa, op.csw, clover, (double2 *)dF,
-                             clover ? (double2 *)scratch->p : nullptr, c->st);
+                             clover ? (double *)scratch->p : nullptr, c->st);
         count(c, 1 + clover);
         if (!device_ptr) CK(cudaMemcpyAsync(force, dF, fb, cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));

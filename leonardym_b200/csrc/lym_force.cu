@@ -5,12 +5,25 @@
 // clover-leaf terms with the link products of its setLattice, :225-268, formed on the fly):
 //   force[x][mu] -= weight * F_mu(x),  F = clover / 4 + Wilson.
 // X, Y and the force field are in the reference's AoS layout: spinors double2[V][4][3], force
-// matrices double2[V][4][3][3] column-major ([site][mu][j][i] = F(i, j)).  One thread per
-// (site, mu), everything in FP64.
-#include <cmath>
-#include <complex>
-
+// matrices double2[V][4][3][3] column-major ([site][mu][j][i] = F(i, j)).  Everything in FP64.
+//
+// Wilson part.  With the half spinors h_k(psi) = psi_k - c_k psi_pk and g_k(psi) = psi_k +
+// c_k psi_pk of direction mu (the projections of lym_dslash.cuh), the sum over the spins and
+// both pair orders of the first term is
+//   M = sum_i w_i sum_{k=0,1} h_k(Y_i)(x+mu) g_k(X_i)(x)^+ + h_k(X_i)(x+mu) g_k(Y_i)(x)^+ ,
+// the second term's spin sum is M^+, and F = -kappa (M - (U M U)^+) with U = U_mu(x): the link
+// enters once per (site, mu), not once per pair and spin.
+//
+// Clover part.  gamma5 sigma_{mu nu} acts inside a chirality as +- a Pauli matrix, so the six
+// plane matrices N^{mu nu}(x) of the spinors are i times real combinations of the Hermitian
+//   P_k = sum_ab (sigma_k)_ab sum_i w_i (Y_b X_a^+ + X_b Y_a^+)   (k = 1..3, per chirality),
+// 9 reals each (H below, kappa c_sw and the signs included).  The eight terms of a plane are
+//   i [H(x+mu) V + V H(x) + C S] for the staple V = C E through x+nu, and minus the adjoint of
+// the same expression through x-nu between two U_mu(x)^+, with E = B^+ A^+, C = U_nu(x+mu),
+// B = U_mu(x+nu), A = U_nu(x), S = H(x+mu+nu) E + B^+ (H(x+nu) A^+): 8 matrix products per
+// staple, two of them with a packed Hermitian factor.
 #include "lym_common.cuh"
+#include "lym_dslash.cuh"
 #include "lym_internal.h"
 
 namespace lym {
@@ -19,65 +32,124 @@ namespace {
 
 typedef cx<double> C;
 
-struct M3 {
-    C a[3][3];  // a[i][j] = M(i, j)
+template <class T> struct Mat {
+    T a[3][3];  // a[i][j] = M(i, j)
 };
 
-// (gamma5 (1 - gamma_mu))_{ab}, (gamma5 (1 + gamma_mu))_{ab}, (gamma5 sigma_{mu nu})_{ab} of
-// the chiral basis: gamma_k = [[0, -i s_k], [i s_k, 0]] (k = x, y, z), gamma_t = [[0, 1], [1, 0]],
-// gamma5 = diag(1, 1, -1, -1), sigma_{mu nu} = (i/2) [gamma_mu, gamma_nu] (the reference's
-// Gamma / Sigma tables, utils/Gamma.cpp)
-struct ForceTables {
-    C mg[4][4][4];
-    C pg[4][4][4];
-    C g5s[4][4][4][4];
-};
-__constant__ ForceTables c_ft;
+// r += a b over real and complex factors (adjoint links are real)
+LYM_D void acc(C &r, C a, C b) { fma_c(r, a, b); }
+LYM_D void acc(C &r, double a, C b) { fma_r(r, a, b); }
+LYM_D void acc(C &r, C a, double b) { fma_r(r, b, a); }
+LYM_D void acc(C &r, double a, double b) { r.re = fma(a, b, r.re); }
+LYM_D void acc(double &r, double a, double b) { r = fma(a, b, r); }
+LYM_D double conj(double a) { return a; }
+LYM_D void zero(C &a) { a = C{0.0, 0.0}; }
+LYM_D void zero(double &a) { a = 0.0; }
 
-LYM_D M3 mul(const M3 &A, const M3 &B)
+template <class A, class B> struct Prod {
+    typedef C T;
+};
+template <> struct Prod<double, double> {
+    typedef double T;
+};
+
+template <class T> LYM_D Mat<T> dag(const Mat<T> &A)
 {
-    M3 R;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            C s{0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) fma_c(s, A.a[i][k], B.a[k][j]);
-            R.a[i][j] = s;
-        }
-    return R;
-}
-LYM_D M3 dag(const M3 &A)
-{
-    M3 R;
+    Mat<T> R;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) R.a[i][j] = conj(A.a[j][i]);
     return R;
 }
-LYM_D void mv(const M3 &A, const C x[3], C y[3])
-{
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        C s{0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) fma_c(s, A.a[i][k], x[k]);
-        y[i] = s;
-    }
-}
-// F += s * tensor(x, y), tensor(x, y)(i, j) = y[i] conj(x[j])  (FermionForce.cpp:22-31)
-LYM_D void add_tensor(M3 &F, double s, const C x[3], const C y[3])
+template <class TR, class TA, class TB> LYM_D void mul_add(Mat<TR> &R, const Mat<TA> &A, const Mat<TB> &B)
 {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            C t{0.0, 0.0};
-            fma_cc(t, x[j], y[i]);
-            F.a[i][j] = F.a[i][j] + s * t;
-        }
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc(R.a[i][j], A.a[i][k], B.a[k][j]);
+}
+template <class TA, class TB>
+LYM_D Mat<typename Prod<TA, TB>::T> mul(const Mat<TA> &A, const Mat<TB> &B)
+{
+    Mat<typename Prod<TA, TB>::T> R;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) zero(R.a[i][j]);
+    mul_add(R, A, B);
+    return R;
+}
+
+// a Hermitian matrix: 3 diagonal reals, entries (0,1), (0,2), (1,2)
+struct Herm {
+    double d[3];
+    C o[3];
+    LYM_D C at(int i, int j) const  // i != j
+    {
+        return i < j ? o[i + j - 1] : lym::conj(o[i + j - 1]);
+    }
+};
+// R += H B, R += A H
+template <class T> LYM_D void mul_add(Mat<C> &R, const Herm &H, const Mat<T> &B)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (k == i) acc(R.a[i][j], H.d[i], B.a[k][j]);
+                else acc(R.a[i][j], H.at(i, k), B.a[k][j]);
+            }
+}
+template <class T> LYM_D void mul_add(Mat<C> &R, const Mat<T> &A, const Herm &H)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (k == j) acc(R.a[i][j], A.a[i][k], H.d[j]);
+                else acc(R.a[i][j], A.a[i][k], H.at(k, j));
+            }
+}
+template <class T> LYM_D void zero(Mat<T> &M)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) zero(M.a[i][j]);
+}
+// F(i, j) += y_i conj(x_j)  (FermionForce.cpp:22-31)
+LYM_D void add_outer(Mat<C> &F, const C y[3], const C x[3])
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) fma_cc(F.a[i][j], x[j], y[i]);
+}
+
+template <class T> struct LinkOf;
+template <> struct LinkOf<GaugeD18> {
+    typedef C T;
+};
+template <> struct LinkOf<GaugeD9> {
+    typedef double T;
+};
+template <class Gauge> LYM_D Mat<typename LinkOf<Gauge>::T> load_link(const Gauge &U, int p, int mu, int h)
+{
+    typename Gauge::Link L;
+    U.load(p, mu, h, L);
+    Mat<typename LinkOf<Gauge>::T> M;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) M.a[i][j] = L.u[i][j];
+    return M;
 }
 
 struct ForceArg {
@@ -87,281 +159,50 @@ struct ForceArg {
     const double2 *const *Y;
     const double *w;           // device array [n]
     double2 *force;
-    const double2 *N;  // [V][6][3][3] plane matrices (clover only)
+    double *N;  // plane matrices H [parity][plane][9][stride] (clover only)
     double kappa, csw;
     int clover;
 };
 
-// planes (mu < nu): 01 02 03 12 13 23
-LYM_D int plane_index(int mu, int nu)
-{
-    const int a = mu < nu ? mu : nu, b = mu < nu ? nu : mu;
-    return a == 0 ? b - 1 : (a == 1 ? b + 1 : 5);
-}
-LYM_D M3 load_plane(const double2 *N, int site, int plane)
-{
-    M3 M;
-    const double2 *b = N + ((size_t)site * 6 + plane) * 9;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const double2 w = __ldg(b + k);
-        M.a[k / 3][k % 3] = C{w.x, w.y};
-    }
-    return M;
-}
-
-// N^{mu nu}(x) = i kappa c_sw sum_i w_i sum_{ab} (gamma5 sigma_{mu nu})_{ab} (Y_b X_a^+ + X_b Y_a^+) at
-// every site, for the six planes mu < nu: the spinor part of ImprovedFermionForce's terms, whose
-// term k is then sign_k L_k N(x_k) R_k^+ (tensor(R X_a, L P_Y[a]) + tensor(R Y_a, L P_X[a]) summed
-// over a)
-__global__ void __launch_bounds__(128) clover_outer_kernel(ForceArg a, double2 *N)
-{
-    // one thread per (site, plane): the six threads of a site are neighbours in the warp, so
-    // each spinor word comes from DRAM once and from L1 for the other five
-    const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= 6L * a.g.V) return;
-    const int site = (int)(tid / 6), p = (int)(tid % 6);
-    {
-        const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2), nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
-        M3 acc;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) acc.a[i][j] = C{0.0, 0.0};
-#pragma unroll 1
-        for (int k = 0; k < a.n; ++k) {
-            const double2 *Xp = a.X[k] + (size_t)site * 12, *Yp = a.Y[k] + (size_t)site * 12;
-            const C ikc{0.0, a.kappa * a.csw * a.w[k]};
-#pragma unroll 1
-            for (int al = 0; al < 4; ++al) {
-                C xa[3], ya[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const double2 x = __ldg(Xp + al * 3 + d), y = __ldg(Yp + al * 3 + d);
-                    xa[d] = C{x.x, x.y};
-                    ya[d] = C{y.x, y.y};
-                }
-#pragma unroll 1
-                for (int be = 0; be < 4; ++be) {
-                    const C g = c_ft.g5s[mu][nu][al][be];
-                    if (g.re == 0.0 && g.im == 0.0) continue;
-                    const C c = ikc * g;
-                    C xb[3], yb[3];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const double2 x = __ldg(Xp + be * 3 + d), y = __ldg(Yp + be * 3 + d);
-                        xb[d] = C{x.x, x.y};
-                        yb[d] = C{y.x, y.y};
-                    }
-#pragma unroll
-                    for (int i = 0; i < 3; ++i)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) {
-                            C t{0.0, 0.0};
-                            fma_cc(t, xa[j], yb[i]);
-                            fma_cc(t, ya[j], xb[i]);
-                            fma_c(acc.a[i][j], c, t);
-                        }
-                }
-            }
-        }
-        double2 *o = N + ((size_t)site * 6 + p) * 9;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) o[k] = make_double2(acc.a[k / 3][k % 3].re, acc.a[k / 3][k % 3].im);
-    }
-}
-
-template <class Gauge> struct Ctx {
-    const ForceArg &a;
-    Gauge U;
-    LYM_D int coord_site(const int c[4]) const
-    {
-        return c[3] + a.g.L[3] * (c[2] + a.g.L[2] * (c[1] + a.g.L[1] * c[0]));
-    }
-    LYM_D void coords(int s, int c[4]) const
-    {
-        c[3] = s % a.g.L[3];
-        int r = s / a.g.L[3];
-        c[2] = r % a.g.L[2];
-        r /= a.g.L[2];
-        c[1] = r % a.g.L[1];
-        c[0] = r / a.g.L[1];
-    }
-    // site + d1 e_m1 + d2 e_m2 (periodic in the index)
-    LYM_D int shift(int s, int m1, int d1, int m2 = 0, int d2 = 0) const
-    {
-        int c[4];
-        coords(s, c);
-        c[m1] = (c[m1] + d1 + a.g.L[m1]) % a.g.L[m1];
-        if (d2) c[m2] = (c[m2] + d2 + a.g.L[m2]) % a.g.L[m2];
-        return coord_site(c);
-    }
-    LYM_D M3 link(int s, int mu) const
-    {
-        int c[4];
-        coords(s, c);
-        const int p = (c[0] + c[1] + c[2] + c[3]) & 1;
-        typename Gauge::Link L;
-        U.load(p, mu, s >> 1, L);
-        M3 M;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) M.a[i][j] = as_c(L.u[i][j]);
-        return M;
-    }
-    LYM_D static C as_c(cx<double> z) { return z; }
-    LYM_D static C as_c(double z) { return C{z, 0.0}; }
-    LYM_D static void colour(const double2 *V, int s, int al, C v[3])
-    {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double2 w = __ldg(V + (size_t)s * 12 + al * 3 + d);
-            v[d] = C{w.x, w.y};
-        }
-    }
+// a site by its coordinates: parity and half-site index
+struct Site {
+    int p, h;
 };
-
-// out = coef * sum_beta T[al][beta] V(s, beta), the non-zero entries only
-LYM_D void spin_comb(const C T[4][4], int al, C coef, const double2 *V, int s, C out[3])
+LYM_D Site site_of(const Geom &g, const int c[4])
+{
+    return Site{(c[0] + c[1] + c[2] + c[3]) & 1, lex_of(g, c[0], c[1], c[2], c[3]) >> 1};
+}
+LYM_D void coords_of(const Geom &g, int s, int c[4])
+{
+    c[3] = s % g.L[3];
+    int r = s / g.L[3];
+    c[2] = r % g.L[2];
+    r /= g.L[2];
+    c[1] = r % g.L[1];
+    c[0] = r / g.L[1];
+}
+// c moved by d in direction mu (periodic); mu is not a compile-time constant
+LYM_D void moved(const Geom &g, const int c[4], int mu, int d, int o[4])
 {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) out[d] = C{0.0, 0.0};
-#pragma unroll 1
-    for (int be = 0; be < 4; ++be) {
-        const C w = coef * T[al][be];
-        if (w.re == 0.0 && w.im == 0.0) continue;
-        C v[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double2 z = __ldg(V + (size_t)s * 12 + be * 3 + d);
-            v[d] = C{z.x, z.y};
+    for (int k = 0; k < 4; ++k) {
+        int v = c[k];
+        if (k == mu) {
+            v += d;
+            if (v >= g.L[k]) v -= g.L[k];
+            if (v < 0) v += g.L[k];
         }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) fma_c(out[d], w, v[d]);
+        o[k] = v;
     }
 }
-// the same of U^+ V(s, beta)
-LYM_D void spin_comb_dag(const C T[4][4], int al, C coef, const M3 &U, const double2 *V, int s, C out[3])
+
+// force -= F at the AoS matrix `out`
+LYM_D void subtract(double2 *out, const Mat<C> &F)
 {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) out[d] = C{0.0, 0.0};
-#pragma unroll 1
-    for (int be = 0; be < 4; ++be) {
-        const C w = coef * T[al][be];
-        if (w.re == 0.0 && w.im == 0.0) continue;
-        C v[3], u[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double2 z = __ldg(V + (size_t)s * 12 + be * 3 + d);
-            v[d] = C{z.x, z.y};
-        }
+    for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            C t{0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) fma_cc(t, U.a[k][i], v[k]);
-            u[i] = t;
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) fma_c(out[d], w, u[d]);
-    }
-}
-
-template <class Gauge> __global__ void __launch_bounds__(128) fermion_force_kernel(ForceArg a, Gauge U)
-{
-    const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= 4L * a.g.V) return;
-    const int site = (int)(tid >> 2), mu = (int)(tid & 3);
-    const Ctx<Gauge> cx_{a, U};
-    M3 F;  // sum_i w_i F_i, Wilson part first
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) F.a[i][j] = C{0.0, 0.0};
-    const int xp = cx_.shift(site, mu, +1);
-    const M3 Um = cx_.link(site, mu);
-    // DiracWilsonFermionForce::derivative
-#pragma unroll 1
-    for (int i = 0; i < a.n; ++i) {
-        const double2 *X = a.X[i], *Y = a.Y[i];
-        const C mk{-a.kappa * a.w[i], 0.0};
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {  // (X, Y), then X and Y exchanged
-            const double2 *A = pass ? Y : X, *B = pass ? X : Y;
-#pragma unroll 1
-            for (int al = 0; al < 4; ++al) {
-                C t[3], u[3], v[3];
-                spin_comb(c_ft.mg[mu], al, mk, B, xp, t);
-                Ctx<Gauge>::colour(A, site, al, v);
-                add_tensor(F, 1.0, v, t);
-                spin_comb_dag(c_ft.pg[mu], al, mk, Um, B, site, t);
-                Ctx<Gauge>::colour(A, xp, al, v);
-                mv(Um, v, u);
-                add_tensor(F, -1.0, u, t);
-            }
-        }
-    }
-    if (a.clover) {
-        // ImprovedFermionForce::derivative: term k of plane (mu, nu) adds sign_k L_k N^{mu nu}(x_k) R_k^+
-        // (N from clover_outer_kernel: the spin traces of both pair orders, weights included);
-        // the clover sum / 4
-        M3 Fc;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) Fc.a[i][j] = C{0.0, 0.0};
-#pragma unroll 1
-        for (int nu = 0; nu < 4; ++nu) {
-            if (nu == mu) continue;
-            const int plane = plane_index(mu, nu);
-            const double sgn = mu < nu ? 1.0 : -1.0;  // N^{nu mu} = -N^{mu nu}
-            const int xpn = cx_.shift(site, nu, +1), xmn = cx_.shift(site, nu, -1);
-            const int xpm_mn = cx_.shift(site, mu, +1, nu, -1), xpm_pn = cx_.shift(site, mu, +1, nu, +1);
-            auto add = [&](double sg, const M3 &M) {
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) Fc.a[i][j] = Fc.a[i][j] + (sg * sgn) * M.a[i][j];
-            };
-            // the terms in an order that shares their link products (k = term of
-            // ImprovedFermionForce.cpp; L_k, R_k its matrices): A = U_nu(x+mu) U_mu(x+nu)^+
-            {
-                const M3 Unu_x = cx_.link(site, nu);
-                const M3 A = mul(cx_.link(xp, nu), dag(cx_.link(xpn, mu)));
-                add(+1.0, mul(mul(A, load_plane(a.N, xpn, plane)), dag(Unu_x)));  // k=2: L=A, R=U_nu(x)
-                add(+1.0, mul(mul(A, dag(Unu_x)), load_plane(a.N, site, plane)));  // k=0: L=A U_nu(x)^+
-            }
-            {
-                // D = U_nu(x) U_mu(x+nu)
-                const M3 Unu_xpm = cx_.link(xp, nu);
-                const M3 D = mul(cx_.link(site, nu), cx_.link(xpn, mu));
-                add(+1.0, mul(mul(Unu_xpm, load_plane(a.N, xpm_pn, plane)), dag(D)));  // k=6: L=U_nu(x+mu), R=D
-                add(+1.0, mul(load_plane(a.N, xp, plane), dag(mul(D, dag(Unu_xpm)))));  // k=4: R=D U_nu(x+mu)^+
-            }
-            {
-                // C = U_mu(x)^+ U_nu(x-nu)^+, R7 = U_mu(x) U_nu(x+mu-nu)^+, B = R7 U_mu(x-nu)^+
-                const M3 Umu_xmn = cx_.link(xmn, mu), Unu_xmn = cx_.link(xmn, nu), Unu_xpm_mn = cx_.link(xpm_mn, nu);
-                const M3 C = mul(dag(Um), dag(Unu_xmn));
-                const M3 R7 = mul(Um, dag(Unu_xpm_mn));
-                const M3 L7 = mul(C, Umu_xmn);
-                add(-1.0, mul(mul(L7, load_plane(a.N, xpm_mn, plane)), dag(R7)));  // k=7
-                add(-1.0, mul(mul(mul(L7, Unu_xpm_mn), load_plane(a.N, xp, plane)), dag(Um)));  // k=5: L=L7 U_nu(x+mu-nu), R=U_mu(x)
-                const M3 B = mul(R7, dag(Umu_xmn));
-                add(-1.0, mul(mul(C, load_plane(a.N, xmn, plane)), dag(B)));  // k=3: L=C, R=B
-                add(-1.0, mul(mul(dag(Um), load_plane(a.N, site, plane)), dag(mul(B, Unu_xmn))));  // k=1: L=U_mu(x)^+, R=B U_nu(x-nu)
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) F.a[i][j] = 0.25 * Fc.a[i][j] + F.a[i][j];
-    }
-    double2 *out = a.force + ((size_t)site * 4 + mu) * 9;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
             double2 w = out[j * 3 + i];
             w.x -= F.a[i][j].re;
             w.y -= F.a[i][j].im;
@@ -369,64 +210,357 @@ template <class Gauge> __global__ void __launch_bounds__(128) fermion_force_kern
         }
 }
 
-void upload_tables(cudaStream_t st)
+// ---------------------------------------------------------------- spinors --
+// One block takes 32 consecutive sites (lexicographic).  Per pair it copies X and Y of these
+// sites and of their forward neighbours into shared memory (12 16-byte words a site, so the
+// copies are contiguous 192-byte pieces); warps 0..3 then add the pair to M of direction mu =
+// warp, warps 4 and 5 to the P_k of one chirality (27 reals a thread).  The +t neighbour of a
+// site is the next site of the tile, except at the end of a t line or of the tile: only those
+// are copied for it.  Bound by shared memory (8 x 192 bytes written and 36 x 96 read per site
+// and pair), so the next pair's copies run during this pair's sums, two blocks per SM; the
+// order of the tiles (x slowest, or columns that keep the +x neighbours in L2) made no
+// difference.  Reading the AoS spinors straight into registers instead costs one 32-byte sector
+// per lane and load, with 48 loads per pair, site and direction.
+// 24^3 x 48, 12 pairs: 2.16 ms (2.40 with one stage and all +t neighbours copied), against
+// 3.8 ms for six plane matrices per site plus most of 18.9 ms for the Wilson part per pair.
+constexpr int kTile = 32;
+constexpr int kVecWords = 13;                   // 12 words of a spinor, 1 of padding: conflict-free reads
+constexpr int kRun = kTile * kVecWords;         // words of one vector of the tile
+constexpr int kSpinThreads = 192;
+// X or Y of one pair: own, +x, +y, +z sites, then the extra +t sites
+LYM_HD int extra_t_sites(int Lt) { return (Lt - 1 + kTile - 1) / Lt + 1; }
+LYM_HD int vector_words(int Lt) { return 4 * kRun + extra_t_sites(Lt) * kVecWords; }
+inline int spin_smem(int Lt) { return 2 * 2 * vector_words(Lt) * 16; }  // two stages of X and Y
+
+LYM_D void copy16(double2 *dst, const double2 *src)
 {
-    typedef std::complex<double> Z;
-    const Z I(0.0, 1.0);
-    Z g[4][4][4] = {}, g5[4][4] = {};
-    // gamma_k = [[0, -i s_k], [i s_k, 0]] for k = x, y, z; gamma_t = [[0, 1], [1, 0]]
-    const Z s[3][2][2] = {{{0.0, 1.0}, {1.0, 0.0}}, {{0.0, -I}, {I, 0.0}}, {{1.0, 0.0}, {0.0, -1.0}}};
-    for (int k = 0; k < 3; ++k)
-        for (int i = 0; i < 2; ++i)
-            for (int j = 0; j < 2; ++j) {
-                g[k][i][2 + j] = -I * s[k][i][j];
-                g[k][2 + i][j] = I * s[k][i][j];
-            }
-    for (int i = 0; i < 2; ++i) {
-        g[3][i][2 + i] = 1.0;
-        g[3][2 + i][i] = 1.0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+
+template <int S> LYM_D void half_spinor(const double2 *v, int mu, int k, C o[3])  // psi_k + S c_k psi_pk
+{
+    const int pk = proj_partner(mu, k), code = proj_code(mu, k);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double2 a = v[3 * k + d], b = v[3 * pk + d];
+        const C z = mul_code(code, C{b.x, b.y});
+        o[d] = S > 0 ? C{a.x, a.y} + z : C{a.x, a.y} - z;
     }
-    for (int i = 0; i < 4; ++i) g5[i][i] = i < 2 ? 1.0 : -1.0;
-    ForceTables T;
-    for (int m = 0; m < 4; ++m)
-        for (int a = 0; a < 4; ++a)
-            for (int b = 0; b < 4; ++b) {
-                // gamma5 (1 -+ gamma_mu) = g5[a][a] (delta_ab -+ g[m][a][b])
-                const Z d = a == b ? 1.0 : 0.0;
-                const Z mgz = g5[a][a] * (d - g[m][a][b]), pgz = g5[a][a] * (d + g[m][a][b]);
-                T.mg[m][a][b] = C{mgz.real(), mgz.imag()};
-                T.pg[m][a][b] = C{pgz.real(), pgz.imag()};
+}
+
+// x0: X of the site, xf: X of its +mu neighbour; yo: words from X to Y
+template <int MU> LYM_D void add_wilson(const double2 *x0, const double2 *xf, int yo, double w, Mat<C> &M)
+{
+    const double2 *y0 = x0 + yo, *yf = xf + yo;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            C h[3], g[3];
+            half_spinor<-1>(o ? xf : yf, MU, k, h);
+            half_spinor<+1>(o ? y0 : x0, MU, k, g);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) h[d] = w * h[d];
+            add_outer(M, h, g);
+        }
+}
+
+template <class Gauge, bool CLOVER>
+__global__ void __launch_bounds__(kSpinThreads, 2) spinor_force_kernel(ForceArg a, Gauge U)
+{
+    extern __shared__ __align__(16) double2 sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s0 = blockIdx.x * kTile;
+    const int V = a.g.V, Lt = a.g.L[3];
+    const int yo = vector_words(Lt), t0 = s0 % Lt;
+    // the copies of this thread: word w of the sites j0 and j0 + 16, own and neighbours
+    const int j0 = threadIdx.x / 12, w = threadIdx.x % 12;
+    int src[2][5], slot[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int j = j0 + 16 * q;
+        const int s = min(s0 + j, V - 1);
+        int c[4];
+        coords_of(a.g, s, c);
+        src[q][0] = s;
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu) {
+            int o[4];
+            moved(a.g, c, mu, +1, o);
+            src[q][1 + mu] = lex_of(a.g, o[0], o[1], o[2], o[3]);
+        }
+        slot[q] = (c[3] == Lt - 1 || j == kTile - 1) ? (t0 + j) / Lt : -1;
+    }
+    auto copy_pair = [&](int i, int stage) {
+        const double2 *X = a.X[i] + w, *Y = a.Y[i] + w;
+        double2 *base = sm + stage * 2 * yo + w;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            double2 *d = base + (j0 + 16 * q) * kVecWords;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                copy16(d + r * kRun, X + (size_t)src[q][r] * 12);
+                copy16(d + yo + r * kRun, Y + (size_t)src[q][r] * 12);
             }
-    for (int m = 0; m < 4; ++m)
-        for (int n = 0; n < 4; ++n)
-            for (int a = 0; a < 4; ++a)
-                for (int b = 0; b < 4; ++b) {
-                    Z c = 0.0;
-                    for (int k = 0; k < 4; ++k) c += g[m][a][k] * g[n][k][b] - g[n][a][k] * g[m][k][b];
-                    const Z v = g5[a][a] * 0.5 * I * c;
-                    T.g5s[m][n][a][b] = C{v.real(), v.imag()};
+            if (slot[q] >= 0) {
+                double2 *e = base + 4 * kRun + slot[q] * kVecWords;
+                copy16(e, X + (size_t)src[q][4] * 12);
+                copy16(e + yo, Y + (size_t)src[q][4] * 12);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    const bool t_end = (t0 + lane) % Lt == Lt - 1 || lane == kTile - 1;
+    const int t_word = t_end ? 4 * kRun + (t0 + lane) / Lt * kVecWords : (lane + 1) * kVecWords;
+    Mat<C> M;  // warps 0..3
+    zero(M);
+    double P[27];  // warps 4, 5: M_01 (18), M_00 - M_11 (9, Hermitian)
+#pragma unroll
+    for (int k = 0; k < 27; ++k) P[k] = 0.0;
+    copy_pair(0, 0);
+#pragma unroll 1
+    for (int i = 0; i < a.n; ++i) {
+        if (i + 1 < a.n) {
+            copy_pair(i + 1, (i + 1) & 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        const double2 *st = sm + (i & 1) * 2 * yo, *own = st + lane * kVecWords;
+        const double wi = a.w[i];
+        switch (warp) {
+        case 0: add_wilson<0>(own, own + 1 * kRun, yo, wi, M); break;
+        case 1: add_wilson<1>(own, own + 2 * kRun, yo, wi, M); break;
+        case 2: add_wilson<2>(own, own + 3 * kRun, yo, wi, M); break;
+        case 3: add_wilson<3>(own, st + t_word, yo, wi, M); break;
+        default:
+            if constexpr (CLOVER) {
+                const double2 *x = own + (warp - 4) * 6, *y = x + yo;
+                C x0[3], x1[3], y0[3], y1[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    x0[d] = wi * C{x[d].x, x[d].y};
+                    x1[d] = wi * C{x[3 + d].x, x[3 + d].y};
+                    y0[d] = C{y[d].x, y[d].y};
+                    y1[d] = C{y[3 + d].x, y[3 + d].y};
                 }
-    cudaMemcpyToSymbolAsync(c_ft, &T, sizeof(T), 0, cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);  // T is a host local
+                // M_ab(i, j) = y_b,i conj(x_a,j) + x_b,i conj(y_a,j)
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        C t{P[2 * (3 * r + q)], P[2 * (3 * r + q) + 1]};
+                        fma_cc(t, x0[q], y1[r]);
+                        fma_cc(t, y0[q], x1[r]);
+                        P[2 * (3 * r + q)] = t.re;
+                        P[2 * (3 * r + q) + 1] = t.im;
+                    }
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    P[18 + r] += 2.0 * ((y0[r].re * x0[r].re + y0[r].im * x0[r].im) -
+                                        (y1[r].re * x1[r].re + y1[r].im * x1[r].im));
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                    const int r = e == 2 ? 1 : 0, q = e == 0 ? 1 : 2;
+                    C t{P[21 + 2 * e], P[22 + 2 * e]};
+                    fma_cc(t, x0[q], y0[r]);
+                    fma_cc(t, y0[q], x0[r]);
+                    fma_cc(t, -x1[q], y1[r]);
+                    fma_cc(t, -y1[q], x1[r]);
+                    P[21 + 2 * e] = t.re;
+                    P[22 + 2 * e] = t.im;
+                }
+            }
+        }
+        __syncthreads();  // before a later pair's copies land on these
+    }
+    const int s = s0 + lane;
+    if (warp < 4) {
+        if (s < V) {
+            int c[4];
+            coords_of(a.g, s, c);
+            const Site own = site_of(a.g, c);
+            const auto Um = load_link(U, own.p, warp, own.h);
+            const Mat<C> UMU = mul(mul(Um, M), Um);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) M.a[i][j] = (-a.kappa) * (M.a[i][j] - lym::conj(UMU.a[j][i]));
+            subtract(a.force + ((size_t)s * 4 + warp) * 9, M);
+        }
+    }
+    if constexpr (CLOVER) {
+        // the P_k of both chiralities, then H = kappa c_sw (su P_k(upper) + sl P_k(lower)):
+        // planes 03, 13, 23 (k = x, y, z): su = sl = 1; 12, 02, 01: su = -e, sl = e, e = 1, -1, 1
+        double *ex = reinterpret_cast<double *>(sm);  // [chirality][27][33]
+        if (warp >= 4) {
+#pragma unroll
+            for (int k = 0; k < 27; ++k) ex[((warp - 4) * 27 + k) * 33 + lane] = P[k];
+        }
+        __syncthreads();
+        if (warp < 3 && s < V) {
+            const int k = warp;  // Pauli index; this warp writes its space and its time plane
+            int c[4];
+            coords_of(a.g, s, c);
+            const Site own = site_of(a.g, c);
+            double h[2][9];
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const double *m = ex + b * 27 * 33 + lane;
+                if (k == 2) {
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) h[b][e] = m[(18 + e) * 33];
+                } else {
+                    // P_1 = M_01 + M_01^+, P_2 = -i (M_01 - M_01^+)
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) h[b][r] = 2.0 * m[(8 * r + k) * 33];
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        const int r = e == 2 ? 1 : 0, q = e == 0 ? 1 : 2;
+                        const double ur = m[2 * (3 * r + q) * 33], ui = m[(2 * (3 * r + q) + 1) * 33];
+                        const double lr = m[2 * (3 * q + r) * 33], li = m[(2 * (3 * q + r) + 1) * 33];
+                        h[b][3 + 2 * e] = k == 0 ? ur + lr : ui + li;
+                        h[b][4 + 2 * e] = k == 0 ? ui - li : lr - ur;
+                    }
+                }
+            }
+            const double kc = a.kappa * a.csw, sp = k == 1 ? kc : -kc;
+            const int space = k == 0 ? 3 : (k == 1 ? 1 : 0), time = k == 0 ? 2 : (k == 1 ? 4 : 5);
+            double *ns = a.N + (size_t)((own.p * 6 + space) * 9) * a.g.stride + own.h;
+            double *nt = a.N + (size_t)((own.p * 6 + time) * 9) * a.g.stride + own.h;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                ns[(size_t)e * a.g.stride] = sp * (h[0][e] - h[1][e]);
+                nt[(size_t)e * a.g.stride] = kc * (h[0][e] + h[1][e]);
+            }
+        }
+    }
+}
+
+// ----------------------------------------------------------------- clover --
+// planes (mu < nu): 01 02 03 12 13 23
+LYM_D int plane_index(int mu, int nu)
+{
+    const int a = mu < nu ? mu : nu, b = mu < nu ? nu : mu;
+    return a == 0 ? b - 1 : (a == 1 ? b + 1 : 5);
+}
+LYM_D Herm load_plane(const ForceArg &a, Site s, int plane)
+{
+    const double *b = a.N + (size_t)((s.p * 6 + plane) * 9) * a.g.stride + s.h;
+    double v[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) v[e] = __ldg(b + (size_t)e * a.g.stride);
+    Herm H;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        H.d[e] = v[e];
+        H.o[e] = C{v[3 + 2 * e], v[4 + 2 * e]};
+    }
+    return H;
+}
+
+// acc += sgn (H(x+mu) V + V H(x) + C S), the staple V = C E of plane (mu, nu) through x + nu
+// (UP) or x - nu, with A+ = U_nu(x)^+ or U_nu(x-nu) and C = U_nu(x+mu) or U_nu(x+mu-nu)^+
+template <bool UP, class Gauge>
+LYM_D void add_staple(const ForceArg &a, const Gauge &U, const int c[4], const int cm[4], int mu, int nu, double sgn,
+                      Mat<C> &F)
+{
+    const Geom &g = a.g;
+    const int plane = plane_index(mu, nu);
+    int o[4];
+    const Site x = site_of(g, c), xm = site_of(g, cm);
+    moved(g, c, nu, UP ? +1 : -1, o);
+    const Site xn = site_of(g, o);
+    moved(g, cm, nu, UP ? +1 : -1, o);
+    const Site xmn = site_of(g, o);
+    const auto Al = load_link(U, UP ? x.p : xn.p, nu, UP ? x.h : xn.h);
+    const auto A = UP ? dag(Al) : Al;
+    Mat<C> K;  // H(x+-nu) A + A H(x)
+    zero(K);
+    mul_add(K, load_plane(a, xn, plane), A);
+    mul_add(K, A, load_plane(a, x, plane));
+    const auto B = dag(load_link(U, xn.p, mu, xn.h));
+    Mat<C> S = mul(B, K);
+    const auto E = mul(B, A);
+    mul_add(S, load_plane(a, xmn, plane), E);
+    const auto Cl = load_link(U, UP ? xm.p : xmn.p, nu, UP ? xm.h : xmn.h);
+    const auto Cc = UP ? Cl : dag(Cl);
+    Mat<C> T = mul(Cc, S);
+    mul_add(T, load_plane(a, xm, plane), mul(Cc, E));
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) fma_r(F.a[i][j], sgn, T.a[i][j]);
+}
+
+// One thread per (half-site, mu); a block's four warps take the four directions of 32
+// consecutive half-sites, whose links and plane matrices they share through L1.  Bound by FP64
+// arithmetic (about 20k fused multiply-adds per site, 0.8 ms of the chip at 24^3 x 48), so it
+// runs at 255 registers, two blocks per SM, rather than spill: 1.51 ms there (11 link products
+// and 10 with plane matrices per staple pair before, most of 18.9 ms).  The lower staples come
+// first: their sum L enters as -(U L U)^+.
+template <class Gauge> __global__ void __launch_bounds__(128, 2) clover_force_kernel(ForceArg a, Gauge U)
+{
+    const int h = blockIdx.x * 32 + (threadIdx.x & 31), p = blockIdx.y, mu = threadIdx.x >> 5;
+    if (h >= a.g.Vh) return;
+    int c[4], cm[4];
+    site_coords(a.g, h, p, c);
+    moved(a.g, c, mu, +1, cm);
+    Mat<C> F;
+    zero(F);
+#pragma unroll 1
+    for (int nu = 0; nu < 4; ++nu)
+        if (nu != mu) add_staple<false>(a, U, c, cm, mu, nu, mu < nu ? 1.0 : -1.0, F);
+    {
+        const auto Um = load_link(U, p, mu, h);
+        F = mul(mul(Um, F), Um);
+        F = dag(F);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) F.a[i][j] = -F.a[i][j];
+    }
+#pragma unroll 1
+    for (int nu = 0; nu < 4; ++nu)
+        if (nu != mu) add_staple<true>(a, U, c, cm, mu, nu, mu < nu ? 1.0 : -1.0, F);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) F.a[i][j] = 0.25 * times_i(F.a[i][j]);
+    subtract(a.force + ((size_t)lex_of(a.g, c[0], c[1], c[2], c[3]) * 4 + mu) * 9, F);
+}
+
+template <class Gauge, bool CLOVER> void run_spinor_force(const ForceArg &a, const Gauge &U, cudaStream_t st)
+{
+    const int smem = spin_smem(a.g.L[3]);
+    cudaFuncSetAttribute(spinor_force_kernel<Gauge, CLOVER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    spinor_force_kernel<Gauge, CLOVER><<<(a.g.V + kTile - 1) / kTile, kSpinThreads, smem, st>>>(a, U);
+}
+
+template <class Gauge> void run_force(const ForceArg &a, const Gauge &U, cudaStream_t st)
+{
+    if (a.clover) {
+        run_spinor_force<Gauge, true>(a, U, st);
+        clover_force_kernel<Gauge><<<dim3((a.g.Vh + 31) / 32, 2), 128, 0, st>>>(a, U);
+    } else {
+        run_spinor_force<Gauge, false>(a, U, st);
+    }
 }
 
 }  // namespace
 
-size_t fermion_force_scratch_bytes(const Geom &g) { return (size_t)g.V * 6 * 9 * sizeof(double2); }
+size_t fermion_force_scratch_bytes(const Geom &g) { return (size_t)2 * 6 * 9 * g.stride * sizeof(double); }
 
 void launch_fermion_force(const Geom &g, const GaugeDev &U, int n, const double2 *const *X, const double2 *const *Y,
                           const double *weights, double kappa, double csw, int clover, double2 *force,
-                          double2 *scratch, cudaStream_t st)
+                          double *scratch, cudaStream_t st)
 {
-    upload_tables(st);
-    ForceArg a{g, n, X, Y, weights, force, scratch, kappa, csw, clover};
-    if (clover) clover_outer_kernel<<<(int)((6L * g.V + 127) / 128), 128, 0, st>>>(a, scratch);
-    const long threads = 4L * g.V;
-    const int grid = (int)((threads + 127) / 128);
-    if (U.rep == REP_SU3)
-        fermion_force_kernel<GaugeD18><<<grid, 128, 0, st>>>(a, GaugeD18{(const double2 *)U.d64, g.stride});
-    else
-        fermion_force_kernel<GaugeD9><<<grid, 128, 0, st>>>(a, GaugeD9{(const double *)U.d64, g.stride});
+    const ForceArg a{g, n, X, Y, weights, force, scratch, kappa, csw, clover};
+    if (U.rep == REP_SU3) run_force(a, GaugeD18{(const double2 *)U.d64, g.stride}, st);
+    else run_force(a, GaugeD9{(const double *)U.d64, g.stride}, st);
 }
 
 }  // namespace lym

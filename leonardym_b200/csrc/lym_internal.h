@@ -173,7 +173,7 @@ void launch_dots(const Geom &g, const DotPairs &D, int n, int gamma5, double2 *p
 size_t fermion_force_scratch_bytes(const Geom &g);
 void launch_fermion_force(const Geom &g, const GaugeDev &U, int n, const double2 *const *X, const double2 *const *Y,
                           const double *weights, double kappa, double csw, int clover, double2 *force,
-                          double2 *scratch, cudaStream_t st);
+                          double *scratch, cudaStream_t st);
 // real Z2 noise vector `stream` of generator `seed` (AoS full spinor)
 void launch_z2_noise(const Geom &g, double *out, unsigned long long seed, unsigned long long stream, cudaStream_t st);
 }  // namespace lym

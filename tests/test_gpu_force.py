@@ -96,3 +96,32 @@ def test_force_many_pairs(setup):
     for x, y, wi in zip(Xs, Ys, w):
         ff.derivative(b, x, y, wi)
     assert np.max(np.abs(a - b)) <= 1e-13 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("rep", ["su3", "su2adj"])
+@pytest.mark.parametrize("dims,n", [((2, 2, 2, 2), 1), ((2, 4, 2, 4), 2), ((3, 2, 5, 2), 3), ((2, 2, 3, 10), 1),
+                                    ((4, 2, 2, 34), 2)])
+def test_force_tile_edges(rep, dims, n):
+    # tiles of 32 sites: fewer sites than a tile, a ragged last tile, t lines that end inside a
+    # tile, on its edge and beyond it; extents of 2 (both neighbours the same site) and odd ones
+    kappa, csw = 0.13, 1.2
+    links = synth.fermion_links(dims, rep, 0.3, 17)
+    lat = L.Lattice(dims, rep)
+    try:
+        gid = lat.upload(links)
+        Xs = [synth.gaussian_spinor(dims, 3, 80 + k) for k in range(n)]
+        Ys = [synth.gaussian_spinor(dims, 3, 90 + k) for k in range(n)]
+        w = [0.4 / (k + 1) for k in range(n)]
+        f0 = np.ones((lat.V, 4, 3, 3), np.complex128)
+        for kind, cls in (("Improved", L.ImprovedDiracWilsonOperator), ("DiracWilson", L.DiracWilsonOperator)):
+            op = cls(lat, kappa, csw) if kind == "Improved" else cls(lat, kappa)
+            op.setLattice(gid)
+            f = f0.copy()
+            op.getForce().derivative_many(f, Xs, Ys, w)
+            ref = f0
+            for x, y, wi in zip(Xs, Ys, w):
+                ref = OF.fermion_force(dims, links, x, y, kappa, csw, kind == "Improved", wi, ref)
+            # sums of a few hundred FP64 products of order one
+            assert np.max(np.abs(f - ref)) <= 1e-13 * np.max(np.abs(ref - f0))
+    finally:
+        lat.close()
