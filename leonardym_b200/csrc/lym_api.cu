@@ -371,7 +371,6 @@ void ensure_clover(lym_context *c, OpEntry &op, double *F_out = nullptr)
     }
     CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
     launch_clover_build(c->g, ge.dev, op.kappa * op.csw, op.clover, F_out, c->d_err, c->st);
-    launch_clover_compress(c->g, op.clover, c->st);
     int herr = 0;
     CK(cudaMemcpyAsync(c->h_scal, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -2615,17 +2614,17 @@ static int gauge_store(lym_context *c, int id, const double *links, bool device_
     }
     const size_t per = c->rep == REP_SU3 ? 18 : 9;
     const size_t bytes = (size_t)g.V * 4 * per * sizeof(double);
+    CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
     if (!device_ptr) {
         double *buf = (double *)dev_alloc(c, bytes);
         CK(cudaMemcpyAsync(buf, links, bytes, cudaMemcpyHostToDevice, c->st));
-        launch_upload_gauge(g, c->rep, buf, ge->dev, c->st);
+        launch_store_gauge(g, buf, ge->dev, c->d_err, c->st);
         CK(cudaStreamSynchronize(c->st));
         dev_free(c, buf, bytes);
     } else {
-        launch_upload_gauge(g, c->rep, links, ge->dev, c->st);
+        launch_store_gauge(g, links, ge->dev, c->d_err, c->st);
     }
-    CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
-    launch_compress_gauge(g, ge->dev, c->d_err, c->st);
+    if (ge->dev.link_reals == 8) launch_store_gauge8(g, ge->dev, c->st);
     CK(cudaMemcpyAsync(c->h_scal, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     CK(cudaGetLastError());
@@ -3910,7 +3909,12 @@ int lym_set_link_format(lym_context *c, int reals)
         if (reals == 8 && c->rep != REP_SU3)
             fail(c, LYM_ERR_UNSUPPORTED, "the 8-real link format is for SU(3) fundamental links");
         c->link_reals = reals;
-        for (auto &kv : c->gauges) kv.second.dev.link_reals = reals;
+        for (auto &kv : c->gauges) {
+            // the 8-real words are built for the fields that are read through them
+            if (reals == 8 && kv.second.dev.link_reals != 8) launch_store_gauge8(c->g, kv.second.dev, c->st);
+            kv.second.dev.link_reals = reals;
+        }
+        CK(cudaGetLastError());
         return LYM_OK;
     });
 }

@@ -80,13 +80,16 @@ void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in,
                    int gamma5, cudaStream_t st);
 void launch_pack(const Geom &g, const double *aos, const Spinor &full, cudaStream_t st);
 void launch_unpack(const Geom &g, const Spinor &full, double *aos, cudaStream_t st);
-void launch_upload_gauge(const Geom &g, int rep, const double *aos, GaugeDev &U, cudaStream_t st);
-void launch_compress_gauge(const Geom &g, GaugeDev &U, int *err, cudaStream_t st);
+// every resident format of an AoS link field but the 8-real one (lym_clover.cu); err: bits of
+// links that are not +-SU(3) / +-SO(3)
+void launch_store_gauge(const Geom &g, const double *aos, GaugeDev &U, int *err, cudaStream_t st);
+// the 8-real FP32 links of a stored SU(3) field
+void launch_store_gauge8(const Geom &g, GaugeDev &U, cudaStream_t st);
 void launch_fundamental_to_fermion(const Geom &g, int rep, int bc, const double *gauge_aos, double *fermion_aos,
                                    cudaStream_t st);
+// T and T^-1 in all three precisions (lym_clover.cu), optionally F in the reference's layout
 void launch_clover_build(const Geom &g, const GaugeDev &U, double kc, CloverDev &C, double *F_aos, int *err,
                          cudaStream_t st);
-void launch_clover_compress(const Geom &g, CloverDev &C, cudaStream_t st);
 void launch_neighbour_tables(const Geom &g, int *sup, int *sdn, cudaStream_t st);
 void launch_stencil_index_probe(const Geom &g, int *out, cudaStream_t st);
 void launch_convert(const Geom &g, const Spinor &dst, const Spinor &src, cudaStream_t st);

@@ -192,3 +192,36 @@ def test_upload_fundamental_matches_host_conversion(setup, oracle):
     b.setLattice(g2)
     x = synth.gaussian_spinor(dims, 3, 15)
     assert rel(a.multiply(x), b.multiply(x)) < 1e-14
+
+
+@pytest.mark.parametrize("rep", ["su3", "su2adj"])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 4, 2, 6), (4, 2, 6, 4), (2, 2, 4, 10)])
+@pytest.mark.parametrize("csw", [1.3, 9.0])
+def test_gauge_and_clover_tiles(rep, dims, csw, oracle):
+    """Link formats and clover blocks built in tiles of 32 sites: lattices smaller than a tile,
+    ragged last tiles, extents of 2; a c_sw so large that T is indefinite and its inverse needs
+    the pivoting.  The Schur operator reads T and T^-1 in every precision."""
+    kappa = 0.2
+    links = synth.fermion_links(dims, rep, 0.6, 29)
+    lat = L.Lattice(dims, rep)
+    try:
+        op = L.EvenOddImprovedDiracWilsonOperator(lat, kappa, csw, gamma5=True)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, "EvenOddImproved", kappa, csw, True)
+        F = op.field_strength()
+        Fo = orc.field_strength()
+        assert np.max(np.abs(F - np.asarray(Fo).reshape(F.shape))) < 1e-14
+        x = synth.gaussian_spinor(dims, 3, 31)
+        ref = orc.multiply(x)
+        # the worst condition number of the even blocks bounds the inverse's rounding
+        e = np.eye(12).reshape(12, 4, 3)
+        cols = [orc.even_even_inverse(np.broadcast_to(v, (lat.V, 4, 3)).astype(np.complex128).copy()) for v in e]
+        Ti = np.stack([c.reshape(lat.V, 12) for c in cols], axis=-1)
+        even = np.add.reduce(synth.lex_coords(dims), axis=1) % 2 == 0
+        cond = np.linalg.cond(Ti[even]).max()
+        assert rel(op.multiply(x), ref) < 1e-14 * cond + 1e-14
+        if cond < 1e3:  # the odd sites: the even ones are copied
+            assert rel(op.multiply_precision(x, "single")[~even], ref[~even]) < 1e-6 * cond
+            assert rel(op.multiply_precision(x, "half")[~even], ref[~even]) < 5e-3 * cond
+    finally:
+        lat.close()
