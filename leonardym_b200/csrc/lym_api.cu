@@ -388,40 +388,74 @@ void require_recon(lym_context *c, GaugeEntry &ge, int prec)
              "reduced-precision links need +-SU(3) / +-SO(3) links (unitarity check bits %d)", ge.recon_err);
 }
 
-// full operator: out = G5^g (T in_p - kappa H in_{1-p}) + alpha v2 on both parities
-void apply_full(lym_context *c, OpEntry &op, int prec, const Spinor &out, const Spinor &in, int gamma5,
-                const Spinor *v2, double2 alpha, const int *skip = nullptr)
+// the parts of a full-operator launch that do not depend on the parity
+DslashParams full_params(lym_context *c, OpEntry &op, int prec, int gamma5, double2 alpha, const int *skip)
 {
     GaugeEntry &ge = gauge_of(c, op.gauge_id);
     const bool clov = kind_has_clover(op.kind);
     if (clov) ensure_clover(c, op);
     require_recon(c, ge, prec);
+    DslashParams P;
+    P.g = c->g;
+    P.prec = prec;
+    P.rep = c->rep;
+    P.epi = EPI_XPAY_;
+    P.U = &ge.dev;
+    P.clover = clov ? op.clover.T[prec] : nullptr;
+    P.gamma5 = gamma5;
+    P.b = -op.kappa;
+    P.alpha_re = alpha.x;
+    P.alpha_im = alpha.y;
+    P.skip_if = skip;
+    return P;
+}
+
+// full operator: out = G5^g (T in_p - kappa H in_{1-p}) + alpha v2 on both parities
+void apply_full(lym_context *c, OpEntry &op, int prec, const Spinor &out, const Spinor &in, int gamma5,
+                const Spinor *v2, double2 alpha, const int *skip = nullptr)
+{
+    DslashParams P = full_params(c, op, prec, gamma5, alpha, skip);
+    P.has_v2 = v2 ? 1 : 0;
+    if (prec == PREC_D) {  // one launch over both parities
+        P.parity = 2;
+        P.in = P.y = in;
+        P.out = out;
+        P.v2 = v2 ? *v2 : in;
+        launch_dslash(P, c->st);
+        count(c, 1);
+        return;
+    }
     for (int p = 0; p < 2; ++p) {
-        DslashParams P;
-        P.g = c->g;
-        P.prec = prec;
-        P.rep = c->rep;
-        P.epi = EPI_XPAY_;
         P.parity = p;
         P.in = in.parity(1 - p);
         P.out = out.parity(p);
         P.y = in.parity(p);
-        if (v2) {
-            P.v2 = v2->parity(p);
-            P.has_v2 = 1;
-            P.alpha_re = alpha.x;
-            P.alpha_im = alpha.y;
-        } else {
-            P.v2 = P.y;
-        }
-        P.U = &ge.dev;
-        P.clover = clov ? op.clover.T[prec] : nullptr;
-        P.gamma5 = gamma5;
-        P.b = -op.kappa;
-        P.skip_if = skip;
+        P.v2 = v2 ? v2->parity(p) : P.y;
         launch_dslash(P, c->st);
         count(c, 1);
     }
+}
+
+// the first half of a Schur product: tmp_e = T_ee^{-1} H_eo in_o
+void schur_even_half(lym_context *c, OpEntry &op, int prec, const Spinor &tmp_e, const Spinor &in_o, const int *skip)
+{
+    const bool clov = kind_has_clover(op.kind);
+    DslashParams P;
+    P.g = c->g;
+    P.prec = prec;
+    P.rep = c->rep;
+    P.U = &gauge_of(c, op.gauge_id).dev;
+    P.skip_if = skip;
+    P.epi = clov ? EPI_CLOVINV_ : EPI_SCALE_;
+    P.parity = 0;
+    P.in = in_o;
+    P.out = tmp_e;
+    P.y = tmp_e;
+    P.v2 = tmp_e;
+    P.clover = clov ? op.clover.Tinv[prec] : nullptr;
+    P.a = 1.0;
+    launch_dslash(P, c->st);
+    count(c, 1);
 }
 
 // Schur complement on the odd sites:
@@ -440,17 +474,8 @@ void apply_schur(lym_context *c, OpEntry &op, int prec, const Spinor &out_o, con
     P.rep = c->rep;
     P.U = &ge.dev;
     P.skip_if = skip;
-    // K1: tmp_e = Tinv_ee H_eo in_o
-    P.epi = clov ? EPI_CLOVINV_ : EPI_SCALE_;
-    P.parity = 0;
-    P.in = in_o;
-    P.out = tmp_e;
-    P.y = tmp_e;
-    P.v2 = tmp_e;
-    P.clover = clov ? op.clover.Tinv[prec] : nullptr;
-    P.a = 1.0;
-    launch_dslash(P, c->st);
-    // K2: out_o = G5^g (T_oo in_o - kappa^2 H_oe tmp_e) + alpha v2
+    schur_even_half(c, op, prec, tmp_e, in_o, skip);
+    // out_o = G5^g (T_oo in_o - kappa^2 H_oe tmp_e) + alpha v2
     P.epi = EPI_XPAY_;
     P.parity = 1;
     P.in = tmp_e;
@@ -468,7 +493,7 @@ void apply_schur(lym_context *c, OpEntry &op, int prec, const Spinor &out_o, con
         P.v2 = in_o;
     }
     launch_dslash(P, c->st);
-    count(c, 2);
+    count(c, 1);
 }
 
 // Q in_o = gamma5 S in_o inside the even-odd CG on (gamma5 S)^2, with the CG's vector work in
@@ -489,15 +514,7 @@ void apply_schur_cg(lym_context *c, OpEntry &op, int prec, int mode, const Spino
     P.rep = c->rep;
     P.U = &ge.dev;
     P.skip_if = skip;
-    P.epi = clov ? EPI_CLOVINV_ : EPI_SCALE_;
-    P.parity = 0;
-    P.in = in_o;
-    P.out = tmp_e;
-    P.y = tmp_e;
-    P.v2 = tmp_e;
-    P.clover = clov ? op.clover.Tinv[prec] : nullptr;
-    P.a = 1.0;
-    launch_dslash(P, c->st);
+    schur_even_half(c, op, prec, tmp_e, in_o, skip);
     P.epi = EPI_XPAY_;
     P.parity = 1;
     P.in = tmp_e;
@@ -508,7 +525,7 @@ void apply_schur_cg(lym_context *c, OpEntry &op, int prec, int mode, const Spino
     P.b = -op.kappa * op.kappa;
     P.gamma5 = 1;
     launch_dslash_cg(P, mode, p, x, r, state, c->spartials, c->counter, c->st);
-    count(c, 2);
+    count(c, 1);
 }
 
 bool is_even_odd(int kind) { return kind == LYM_OP_EVEN_ODD_IMPROVED || kind == LYM_OP_SQUARE_EVEN_ODD_IMPROVED; }
@@ -547,6 +564,52 @@ void op_apply(lym_context *c, OpEntry &op, int prec, const Spinor &out, const Sp
     }
     default: fail(c, LYM_ERR_ARGUMENT, "unknown operator kind %d", op.kind);
     }
+}
+
+// op_apply in FP64 with the result, alpha v2 added, written into AoS device vectors by the last
+// stencil launch (v2 may be null, or `out` itself)
+void op_apply_aos(lym_context *c, OpEntry &op, double *out, const Spinor &in, const double *v2, double2 alpha)
+{
+    const int g5 = op.gamma5;
+    DslashParams P = full_params(c, op, PREC_D, g5, alpha, nullptr);
+    P.parity = 2;
+    P.aos_out = out;
+    P.aos_v2 = v2;
+    auto finish = [&]() {
+        launch_dslash(P, c->st);
+        count(c, 1);
+    };
+    if (!is_even_odd(op.kind)) {
+        const bool square = op.kind == LYM_OP_SQUARE_DIRAC_WILSON || op.kind == LYM_OP_SQUARE_IMPROVED;
+        if (!square && op.kind != LYM_OP_DIRAC_WILSON && op.kind != LYM_OP_IMPROVED)
+            fail(c, LYM_ERR_ARGUMENT, "unknown operator kind %d", op.kind);
+        if (!square) {
+            P.in = P.y = in;
+            finish();
+            return;
+        }
+        Vec tmp(c, PREC_D, 2);
+        apply_full(c, op, PREC_D, *tmp, in, g5, nullptr, C2(0.0));
+        P.in = P.y = *tmp;
+        finish();
+        return;
+    }
+    if (op.kind == LYM_OP_EVEN_ODD_IMPROVED && v2)
+        fail(c, LYM_ERR_UNSUPPORTED, "EvenOddImprovedDiracWilsonOperator::multiplyAdd is not implemented");
+    // odd sites: the last Schur product's second stencil; even sites: the input's
+    Vec te(c, PREC_D, 1), to(c, PREC_D, 1);
+    Spinor odd = in.parity(1);
+    if (op.kind == LYM_OP_SQUARE_EVEN_ODD_IMPROVED) {
+        apply_schur(c, op, PREC_D, *to, odd, *te, g5);
+        odd = *to;
+    }
+    schur_even_half(c, op, PREC_D, *te, odd, nullptr);
+    P.in = *te;
+    P.y = odd;
+    P.even = in.parity(0);
+    P.even_copy = 1;
+    P.b = -op.kappa * op.kappa;
+    finish();
 }
 
 // ------------------------------------------------------ host <-> device -----
@@ -2504,7 +2567,7 @@ int lym_context_create(const int dims[4], int rep, int device, lym_context **out
         CK(cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));
         c->partials = (double *)dev_alloc(c, (size_t)kBlasGridMax * kMaxRed * sizeof(double));
         c->bpartials = (double *)dev_alloc(c, (size_t)kBlasGridMax * kMaxBatch * kBatchMaxRed * sizeof(double));
-        c->spartials = (double *)dev_alloc(c, ((size_t)c->g.Vh + 127) / 128 * sizeof(double));
+        c->spartials = (double *)dev_alloc(c, (size_t)split_partials(c->g) * sizeof(double));
         c->nbr = (int *)dev_alloc(c, (size_t)16 * c->g.stride * sizeof(int));
         launch_nbr_table(c->g, c->nbr, c->st);
         c->counter = (unsigned int *)dev_alloc(c, 64);
@@ -2764,20 +2827,31 @@ static int do_multiply(lym_context *c, int op_id, int prec, double *out, const d
     if (prec < PREC_D || prec > PREC_H) return LYM_ERR_ARGUMENT;
     return guarded(c, [&]() {
         OpEntry &op = op_of(c, op_id);
-        Vec a(c, prec, 2), o(c, prec, 2);
-        Vec *w = nullptr;
+        Vec a(c, prec, 2);
         upload_vec(c, *a, v1, device_ptr, 0);
+        const size_t n = (size_t)c->g.V * 24;
+        // the last launch writes the caller's vector itself unless the vectors overlap in part
+        const bool parts = device_ptr && v2 && v2 != out && v2 < out + n && out < v2 + n;
+        if (prec == PREC_D && !parts) {
+            double *dst = device_ptr ? out : staging(c, 2);
+            const double *add = v2;
+            if (v2 && !device_ptr) {
+                CK(cudaMemcpyAsync(staging(c, 1), v2, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
+                add = c->aos[1];
+            }
+            op_apply_aos(c, op, dst, *a, add, alpha);
+            if (!device_ptr) CK(cudaMemcpyAsync(out, dst, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+            CK(cudaStreamSynchronize(c->st));
+            CK(cudaGetLastError());
+            return LYM_OK;
+        }
+        Vec o(c, prec, 2);
+        std::unique_ptr<Vec> w;
         if (v2) {
-            w = new Vec(c, prec, 2);
+            w.reset(new Vec(c, prec, 2));
             upload_vec(c, **w, v2, device_ptr, 1);
         }
-        try {
-            op_apply(c, op, prec, *o, *a, w ? &**w : nullptr, alpha);
-        } catch (...) {
-            delete w;
-            throw;
-        }
-        delete w;
+        op_apply(c, op, prec, *o, *a, w ? &**w : nullptr, alpha);
         download_vec(c, out, *o, device_ptr, 2);
         CK(cudaStreamSynchronize(c->st));
         CK(cudaGetLastError());

@@ -56,11 +56,18 @@ struct DslashParams {
     int prec = PREC_D;
     int rep = REP_SU3;
     int epi = EPI_SCALE_;
-    int parity = 0;          // output parity
+    int parity = 0;          // output parity; 2 (FP64 only): both, the spinors are full ones
     Spinor in;               // view of the input parity (1 - parity)
     Spinor out;              // view of the output parity
     Spinor y;                // same-parity input (EPI_XPAY, EPI_XPAY_INV)
     Spinor v2;               // optional added vector (EPI_XPAY)
+    // FP64 EPI_XPAY with parity 2 may write a caller's AoS vector instead of `out`, adding
+    // alpha times another AoS vector (aos_v2, or null; it may be aos_out itself); with even_copy
+    // the stencil runs on the odd sites only (in, y: half spinors) and the even sites get `even`
+    double *aos_out = nullptr;
+    const double *aos_v2 = nullptr;
+    int even_copy = 0;
+    Spinor even;
     int has_v2 = 0;
     const GaugeDev *U = nullptr;
     const void *clover = nullptr;  // T (EPI_XPAY) or Tinv (EPI_CLOVINV, EPI_XPAY_INV) of this precision
@@ -76,6 +83,12 @@ void launch_dslash(const DslashParams &P, cudaStream_t st);
 // partials: one double per block of the launch
 void launch_dslash_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
                       double *partials, unsigned int *counter, cudaStream_t st);
+// FP64 (lym_split.cu): launch_dslash and launch_dslash_cg end here for PREC_D; the partial sums of
+// a launch_split_cg over either parity or both fit in split_partials doubles
+void launch_split(const DslashParams &P, cudaStream_t st);
+void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
+                     double *partials, unsigned int *counter, cudaStream_t st);
+int split_partials(const Geom &g);
 void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in, const void *clover, int parity,
                    int gamma5, cudaStream_t st);
 void launch_pack(const Geom &g, const double *aos, const Spinor &full, cudaStream_t st);

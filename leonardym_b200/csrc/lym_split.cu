@@ -1,0 +1,423 @@
+// The FP64 Wilson-clover stencil: four threads per site.
+//
+// Thread (k, d) of a site, k, d = 0, 1, takes the half spinor h_k (lym_dslash.cuh) of the
+// directions mu = 2 d, 2 d + 1: it accumulates upper spin k and the lower spin its two
+// directions pair with k (3 - k for d = 0, 2 + k for d = 1), 6 complex numbers instead of the 12
+// of a thread per site, then the lanes of the site add up their parts by shuffles:
+//   spin k      = up(k, 0) + up(k, 1),   spin 2 + k = low(k, 1) + low(1 - k, 0),
+// after which thread (k, d) holds spin 2 d + k and applies its three rows of the clover block of
+// chirality d.  A warp is 8 sites, lane = site + 8 d + 16 k, so that link loads of k = 0, 1 fall
+// on one address and spinor loads on contiguous 128-byte pieces.
+//
+// Why four threads: in FP64 the whole-site form needs 142-180 registers (3 blocks of 128 per SM,
+// 12 warps), too few loads in flight for HBM, and on small lattices too few warps and one long
+// dependent chain per site.  24^3 x 48: both parities in one launch 247 us against
+// 2 x 144 us, one parity 141-149 against 144 us (T^-1 half 130 against 137); 16^3 x 32 adjoint 25
+// and 21 against 26 and 28 us; 8^4 both parities 4.6 against 2 x 6.6 us.  Latency bound (L1 misses;
+// 4.35 TB/s of HBM, 16 warps per SM): 3, 5 or 6 blocks per SM give 253, 270, 312 us there, blocks
+// of 256 or 512 threads 252, 280 us.
+//
+// In "both" mode a launch covers both parities, the same half-sites of either in one block, so
+// that a link read forward by one parity and backward by the other comes from DRAM once; it can
+// write the result straight into the caller's AoS vector (through shared memory, whole sites).
+#include "lym_blas.cuh"
+#include "lym_dslash.cuh"
+#include "lym_internal.h"
+#include "lym_solver_ops.cuh"
+
+namespace lym {
+
+namespace {
+
+typedef cx<double> C;
+
+constexpr int kSplitThreads = 128;
+constexpr int kSplitSites = kSplitThreads / 4;
+
+enum SplitEpi : int {
+    SPLIT_SCALE = EPI_SCALE,
+    SPLIT_CLOVINV = EPI_CLOVINV,
+    SPLIT_XPAY = EPI_XPAY,
+    SPLIT_XPAY_INV = EPI_XPAY_INV,
+    SPLIT_CG_NORM = 10,    // EPI_XPAY with gamma5, |out|^2 reduced (CG_NORM of lym_dslash.cuh)
+    SPLIT_CG_UPDATE = 11,  // A p = EPI_XPAY with gamma5 in registers, x and r updated (CG_UPDATE)
+};
+
+template <class GaugeT> struct SplitArg {
+    Geom g;
+    SpinorD in[2], out[2], y[2], v2[2], x[2], r[2];  // by output parity
+    GaugeT U;
+    const double2 *clover;
+    int parity;  // 0, 1, or 2: both
+    int gamma5, has_v2;
+    double a, b, alpha_re, alpha_im;
+    const int *skip_if;
+    double2 *aos_out;        // AOS: the full result
+    const double2 *aos_v2;   // AOS: the added vector, or null
+    int even_copy;           // AOS: even sites get y (no stencil)
+    const double2 *alpha;    // SPLIT_CG_UPDATE
+    double *partials;        // SPLIT_CG_*: [gridDim.x]
+    unsigned int *counter;
+};
+
+LYM_D C load1(const SpinorD &v, int word, int h)
+{
+    const double2 w = __ldg(v.v + (size_t)word * v.stride + h);
+    return C{w.x, w.y};
+}
+LYM_D C shfl_xor(C z, int m)
+{
+    return C{__shfl_xor_sync(0xffffffffu, z.re, m), __shfl_xor_sync(0xffffffffu, z.im, m)};
+}
+
+// spin 2 d + k of H x at the site (p, h), lexicographic index s, coordinates c
+template <class GaugeT>
+LYM_D void split_hopping(const Geom &g, const SpinorD &in, const GaugeT &U, int p, int h, int s, const int c[4], int k,
+                         int d, C own[3])
+{
+    C up[3], low[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) up[m] = low[m] = C{0.0, 0.0};
+    const int wk = 3 * k, wp = 3 * (d ? 2 + k : 3 - k);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int mu = 2 * d + j;
+        const int cm = d ? c[2 + j] : c[j], L = d ? g.L[2 + j] : g.L[j];
+        const int step = j == 0 ? (d ? g.L[3] : g.L[1] * g.L[2] * g.L[3]) : (d ? 1 : g.L[2] * g.L[3]);
+        // c_mu = -i s (j = 0) or s (j = 1)
+        const double sg = j == 0 ? (d & k ? -1.0 : 1.0) : (d | k ? 1.0 : -1.0);
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            const int hn = (s + (dir == 0 ? (cm == L - 1 ? (1 - L) * step : step) : (cm == 0 ? (L - 1) * step : -step))) >> 1;
+            const double sh = dir == 0 ? -sg : sg;
+            typename GaugeT::Link Lk;
+            if (dir == 0) U.load(p, mu, h, Lk);
+            else U.load(1 - p, mu, hn, Lk);
+            C hv[3], w[3];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const C xk = load1(in, wk + m, hn), xp = load1(in, wp + m, hn);
+                const C z = j == 0 ? times_mi(xp) : xp;
+                hv[m] = xk;
+                fma_r(hv[m], sh, z);
+            }
+            if (dir == 0) mul_u(Lk, hv, w);
+            else mul_ud(Lk, hv, w);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                up[m] = up[m] + w[m];
+                fma_r(low[m], sh, j == 0 ? times_i(w[m]) : w[m]);
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        up[m] = up[m] + shfl_xor(up[m], 8);
+        low[m] = low[m] + shfl_xor(low[m], 24);
+        own[m] = d ? low[m] : up[m];
+    }
+}
+
+// rows 3 k .. 3 k + 2 of the Hermitian 6 x 6 block (parity p, chirality d) applied to the vector
+// (own spin k, other spin 1 - k)
+LYM_D void clover_rows(const double2 *clover, int stride, int p, int h, int k, int d, const C own[3], const C oth[3],
+                       C res[3])
+{
+    const double2 *base = clover + (size_t)((p * 2 + d) * 18) * stride + h;
+    auto word = [&](int w) { return __ldg(base + (size_t)w * stride); };
+    const double2 dm = word(1), de = word(k ? 2 : 0);
+    const double dg[3] = {k ? dm.y : de.x, k ? de.x : de.y, k ? de.y : dm.x};
+    const double2 a10 = word(3 + (k ? 9 : 0)), a20 = word(3 + (k ? 13 : 1)), a21 = word(3 + (k ? 14 : 2));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) res[i] = dg[i] * own[i];
+    const C o10{a10.x, a10.y}, o20{a20.x, a20.y}, o21{a21.x, a21.y};
+    fma_cc(res[0], o10, own[1]);
+    fma_c(res[1], o10, own[0]);
+    fma_cc(res[0], o20, own[2]);
+    fma_c(res[2], o20, own[0]);
+    fma_cc(res[1], o21, own[2]);
+    fma_c(res[2], o21, own[1]);
+    // entries (3 + i, j) for k = 1, their transpose's conjugates for k = 0
+    constexpr int row[3] = {6, 9, 13};  // word of (3 + i, 0): 3 + tri_index(3 + i, 0)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double2 w = word(k ? row[i] + j : row[j] + i);
+            fma_c(res[i], C{w.x, k ? w.y : -w.y}, oth[j]);
+        }
+}
+
+struct NoFin {
+    LYM_D void operator()(double) const {}
+};
+struct AlphaFin {  // alpha = |r|^2 / <p, A p> with <p, A p> = |Q p|^2
+    CGState *s;
+    LYM_D void operator()(double qq) const { s->alpha = make_double2(s->rr / qq, 0.0); }
+};
+struct UpdateFin {  // the scalar step of OpCGUpdate
+    CGState *s;
+    LYM_D void operator()(double rr) const
+    {
+        const double t[1] = {rr};
+        OpCGUpdate<SpinorD, SpinorD, SpinorD, SpinorD> u{SpinorD{}, SpinorD{}, SpinorD{}, SpinorD{}, s};
+        u.finalize(t);
+    }
+};
+
+template <int EPI, bool AOS, class GaugeT, class Fin>
+__global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<GaugeT> arg, const Fin fin)
+{
+    if (arg.skip_if && *arg.skip_if) return;
+    constexpr bool kReduce = EPI == SPLIT_CG_NORM || EPI == SPLIT_CG_UPDATE;
+    constexpr bool kXpay = EPI == SPLIT_XPAY || kReduce;
+    constexpr int kTileWord = 13;  // 12 words of a site, 1 of padding
+    __shared__ __align__(16) double2 tile[AOS ? kSplitSites * kTileWord : 1];
+    const Geom &g = arg.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = (lane >> 3) & 1, k = lane >> 4;
+    const bool both = arg.parity == 2;
+    const int p = both ? warp >> 1 : arg.parity;
+    const int hr = both ? blockIdx.x * (kSplitSites / 2) + (warp & 1) * 8 + (lane & 7)
+                        : blockIdx.x * kSplitSites + warp * 8 + (lane & 7);
+    const bool in = hr < g.Vh;
+    const int h = in ? hr : g.Vh - 1;
+    if (AOS && arg.aos_v2) {
+        for (int i = threadIdx.x; i < kSplitSites * 12; i += kSplitThreads) {
+            const int site = i / 12;
+            if (blockIdx.x * kSplitSites + site < g.V)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(tile + site * kTileWord + i % 12)),
+                             "l"(arg.aos_v2 + (size_t)blockIdx.x * kSplitSites * 12 + i)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    int c[4];
+    site_coords(g, h, p, c);
+    const int s = lex_of(g, c[0], c[1], c[2], c[3]);
+    const int sp = 3 * (2 * d + k), so = 3 * (2 * d + 1 - k);  // words of the own and the other spin
+    C res[3];
+    if (AOS && arg.even_copy && p == 0) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m) res[m] = load1(arg.y[0], sp + m, h);
+    } else {
+        C acc[3];
+        split_hopping(g, arg.in[p], arg.U, p, h, s, c, k, d, acc);
+        C own[3], oth[3];
+        if constexpr (EPI == SPLIT_SCALE) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) res[m] = arg.a * acc[m];
+        } else if constexpr (EPI == SPLIT_CLOVINV || EPI == SPLIT_XPAY_INV) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                if (EPI == SPLIT_CLOVINV) {
+                    own[m] = arg.a * acc[m];
+                } else {
+                    own[m] = load1(arg.y[p], sp + m, h);
+                    fma_r(own[m], arg.b, acc[m]);
+                }
+                oth[m] = shfl_xor(own[m], 16);
+            }
+            clover_rows(arg.clover, g.stride, p, h, k, d, own, oth, res);
+        } else {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) own[m] = load1(arg.y[p], sp + m, h);
+            if (arg.clover) {
+#pragma unroll
+                for (int m = 0; m < 3; ++m) oth[m] = load1(arg.y[p], so + m, h);
+                clover_rows(arg.clover, g.stride, p, h, k, d, own, oth, res);
+            } else {
+#pragma unroll
+                for (int m = 0; m < 3; ++m) res[m] = own[m];
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                fma_r(res[m], arg.b, acc[m]);
+                if (d && arg.gamma5) res[m] = -res[m];
+            }
+        }
+    }
+    if constexpr (kXpay && !kReduce && !AOS) {
+        if (arg.has_v2) {
+            const C al = {arg.alpha_re, arg.alpha_im};
+#pragma unroll
+            for (int m = 0; m < 3; ++m) fma_c(res[m], al, load1(arg.v2[p], sp + m, h));
+        }
+    }
+    if constexpr (AOS) {
+        double2 *t = tile + (s - blockIdx.x * kSplitSites) * kTileWord + sp;
+        if (arg.aos_v2) {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncthreads();
+            const C al = {arg.alpha_re, arg.alpha_im};
+            if (in) {
+#pragma unroll
+                for (int m = 0; m < 3; ++m) fma_c(res[m], al, C{t[m].x, t[m].y});
+            }
+        }
+        if (in) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) t[m] = make_double2(res[m].re, res[m].im);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < kSplitSites * 12; i += kSplitThreads) {
+            const int site = i / 12;
+            if (blockIdx.x * kSplitSites + site < g.V)
+                arg.aos_out[(size_t)blockIdx.x * kSplitSites * 12 + i] = tile[site * kTileWord + i % 12];
+        }
+        return;
+    }
+    double part = 0.0;
+    if (in) {
+        auto put = [&](const SpinorD &v, int m, C z) {
+            v.v[(size_t)(sp + m) * v.stride + h] = make_double2(z.re, z.im);
+        };
+        if constexpr (EPI == SPLIT_CG_UPDATE) {
+            const double2 al2 = *arg.alpha;
+            const C al = {al2.x, al2.y};
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                C xv = load1(arg.x[p], sp + m, h);
+                fma_c(xv, al, load1(arg.v2[p], sp + m, h));
+                const C rv = load1(arg.r[p], sp + m, h) - al * res[m];
+                part += rv.re * rv.re + rv.im * rv.im;
+                put(arg.x[p], m, xv);
+                put(arg.r[p], m, rv);
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                put(arg.out[p], m, res[m]);
+                if (kReduce) part += res[m].re * res[m].re + res[m].im * res[m].im;
+            }
+        }
+    }
+    if constexpr (kReduce) {
+        // fixed-order reduction: warps, the block's warps, then the blocks in order
+        __shared__ double wsum[kSplitThreads / 32];
+        __shared__ bool last;
+        auto block_total = [&](double v) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) wsum[warp] = v;
+            __syncthreads();
+            return (wsum[0] + wsum[1]) + (wsum[2] + wsum[3]);
+        };
+        const double tot = block_total(part);
+        if (threadIdx.x == 0) {
+            arg.partials[blockIdx.x] = tot;
+            __threadfence();
+            last = atomicAdd(arg.counter, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        double t = 0.0;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += kSplitThreads) t += __ldcg(arg.partials + i);
+        const double all = block_total(t);
+        if (threadIdx.x == 0) {
+            fin(all);
+            *arg.counter = 0u;
+        }
+    }
+}
+
+template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const GaugeT &U)
+{
+    SplitArg<GaugeT> a;
+    a.g = P.g;
+    a.U = U;
+    a.parity = P.parity;
+    // views of one parity, or of the full spinors in both mode
+    const bool both = P.parity == 2 && !P.even_copy;
+    for (int p = 0; p < 2; ++p) {
+        a.in[p] = both ? P.in.d(1 - p) : P.in.d();
+        a.out[p] = P.out.v ? (both ? P.out.d(p) : P.out.d()) : SpinorD{};
+        a.y[p] = both ? P.y.d(p) : P.y.d();
+        a.v2[p] = P.v2.v ? (both ? P.v2.d(p) : P.v2.d()) : SpinorD{};
+        a.x[p] = a.r[p] = SpinorD{};
+    }
+    if (P.even_copy) a.y[0] = P.even.d();
+    a.clover = (const double2 *)P.clover;
+    a.gamma5 = P.gamma5;
+    a.has_v2 = P.has_v2;
+    a.a = P.a;
+    a.b = P.b;
+    a.alpha_re = P.alpha_re;
+    a.alpha_im = P.alpha_im;
+    a.skip_if = P.skip_if;
+    a.aos_out = (double2 *)P.aos_out;
+    a.aos_v2 = (const double2 *)P.aos_v2;
+    a.even_copy = P.even_copy;
+    a.alpha = nullptr;
+    a.partials = nullptr;
+    a.counter = nullptr;
+    return a;
+}
+
+int split_blocks(const Geom &g, int parity)
+{
+    const int per = parity == 2 ? kSplitSites / 2 : kSplitSites;
+    return (g.Vh + per - 1) / per;
+}
+
+template <class GaugeT> void run_split(const DslashParams &P, const GaugeT &U, cudaStream_t st)
+{
+    const SplitArg<GaugeT> a = split_arg(P, U);
+    const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
+    if (P.aos_out) {
+        split_kernel<SPLIT_XPAY, true><<<nb, nt, 0, st>>>(a, NoFin{});
+        return;
+    }
+    switch (P.epi) {
+    case EPI_SCALE_: split_kernel<SPLIT_SCALE, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    case EPI_CLOVINV_: split_kernel<SPLIT_CLOVINV, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    case EPI_XPAY_: split_kernel<SPLIT_XPAY, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    default: split_kernel<SPLIT_XPAY_INV, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    }
+}
+
+template <class GaugeT>
+void run_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, CGState *cs,
+                  double *partials, unsigned int *counter, const GaugeT &U, cudaStream_t st)
+{
+    SplitArg<GaugeT> a = split_arg(P, U);
+    for (int q = 0; q < 2; ++q) {
+        const int v = P.parity == 2 ? q : 0;
+        a.v2[q] = p.d(v);
+        a.x[q] = x.d(v);
+        a.r[q] = r.d(v);
+    }
+    a.gamma5 = 1;
+    a.alpha = &cs->alpha;
+    a.partials = partials;
+    a.counter = counter;
+    const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
+    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, AlphaFin{cs});
+    else split_kernel<SPLIT_CG_UPDATE, false><<<nb, nt, 0, st>>>(a, UpdateFin{cs});
+}
+
+}  // namespace
+
+int split_partials(const Geom &g) { return split_blocks(g, 2); }
+
+void launch_split(const DslashParams &P, cudaStream_t st)
+{
+    const int s = P.g.stride;
+    if (P.rep == REP_SU3) run_split(P, GaugeD18{(const double2 *)P.U->d64, s}, st);
+    else run_split(P, GaugeD9{(const double *)P.U->d64, s}, st);
+}
+
+void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
+                     double *partials, unsigned int *counter, cudaStream_t st)
+{
+    const int s = P.g.stride;
+    if (P.rep == REP_SU3)
+        run_split_cg(P, mode, p, x, r, (CGState *)state, partials, counter, GaugeD18{(const double2 *)P.U->d64, s}, st);
+    else
+        run_split_cg(P, mode, p, x, r, (CGState *)state, partials, counter, GaugeD9{(const double *)P.U->d64, s}, st);
+}
+
+}  // namespace lym

@@ -225,3 +225,51 @@ def test_gauge_and_clover_tiles(rep, dims, csw, oracle):
             assert rel(op.multiply_precision(x, "half")[~even], ref[~even]) < 5e-3 * cond
     finally:
         lat.close()
+
+
+@pytest.mark.parametrize("rep", ["su3", "su2adj"])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 2, 10), (4, 2, 6, 6), (2, 2, 2, 34)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_fp64_stencil_tiles(rep, dims, kind, oracle):
+    """The FP64 stencil's tiles of 16 and 32 half-sites: fewer half-sites than a tile, ragged last
+    tiles, extents of 2; results written straight into device vectors, also over an input."""
+    import ctypes as C
+
+    import torch
+    kappa, csw = 0.15, 1.1
+    links = synth.fermion_links(dims, rep, 0.4, 41)
+    lat = L.Lattice(dims, rep)
+    try:
+        op = GPU_CLASS[kind](lat)
+        op.setKappa(kappa)
+        if "Wilson" not in kind:
+            op.setCSW(csw)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, 0.0 if "Wilson" in kind else csw, True)
+        x, y = (synth.gaussian_spinor(dims, 3, 43 + k) for k in range(2))
+        ref, alpha = orc.multiply(x), 0.3 - 0.2j
+        assert rel(op.multiply(x), ref) < 1e-13
+
+        def call(name, out, *args):
+            torch.cuda.synchronize()
+            rc = getattr(L.lib(), name)(lat.handle, op.op_id, *[C.c_void_p(v.data_ptr()) for v in (out, *args[:2])],
+                                        *args[2:])
+            assert rc == 0
+            return out.cpu().numpy()
+
+        dx, dy = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+        assert rel(call("lym_multiply_device", dx, dx), ref) < 1e-13  # over its input
+        if kind == "EvenOddImproved":
+            return
+        refa, a = ref + alpha * y, (alpha.real, alpha.imag)
+        for case in ("apart", "over v2", "over v1"):
+            dx, dy = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+            out = {"apart": torch.empty_like(dx), "over v2": dy, "over v1": dx}[case]
+            assert rel(call("lym_multiply_add_device", out, dx, dy, *a), refa) < 1e-13
+        # v2 and the result overlap in part
+        buf = torch.zeros((lat.V + 1, 4, 3), dtype=torch.complex128, device="cuda")
+        buf[1:] = torch.from_numpy(y).cuda()
+        dx = torch.from_numpy(x).cuda()
+        assert rel(call("lym_multiply_add_device", buf[:-1], dx, buf[1:], *a), refa) < 1e-13
+    finally:
+        lat.close()
