@@ -279,9 +279,11 @@ void count(lym_context *c, int n)
 template <class Op> void run_site(lym_context *c, const Op &op, int nparity, Gate gate = Gate{nullptr, nullptr})
 {
     count(c, 1);
-    int grid = (c->g.Vh + kBlasThreads - 1) / kBlasThreads;
-    grid = std::min(grid, kBlasGridMax);
-    site_kernel<Op><<<grid, kBlasThreads, 0, c->st>>>(op, c->g.Vh, nparity, RedBuf{c->partials, c->counter}, gate);
+    // small vectors take small blocks, so that they reach two blocks on every SM
+    const int n = c->g.Vh * nparity;
+    const int threads = n >= 2 * 148 * kBlasThreads ? kBlasThreads : n >= 148 * kBlasThreads ? 128 : 64;
+    const int grid = std::min((n + threads - 1) / threads, kBlasGridMax);
+    site_kernel<Op><<<grid, threads, 0, c->st>>>(op, c->g.Vh, nparity, RedBuf{c->partials, c->counter}, gate);
 }
 
 double2 C2(double re, double im = 0.0) { return make_double2(re, im); }
@@ -607,7 +609,7 @@ void op_apply_aos(lym_context *c, OpEntry &op, double *out, const Spinor &in, co
     P.in = *te;
     P.y = odd;
     P.even = in.parity(0);
-    P.even_copy = 1;
+    P.even_identity = 1;
     P.b = -op.kappa * op.kappa;
     finish();
 }
@@ -701,11 +703,50 @@ template <class S, class Step> void run_gated_state(lym_context *c, S *d, Step s
     if (!paused) fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %ld iterations", max_iterations);
 }
 
+// A = Q Q (+ shift) with Q Hermitian: the squared kinds with gamma5
+bool is_hermitian_square(const OpEntry &op)
+{
+    return op.gamma5 && (op.kind == LYM_OP_SQUARE_DIRAC_WILSON || op.kind == LYM_OP_SQUARE_IMPROVED ||
+                         op.kind == LYM_OP_SQUARE_EVEN_ODD_IMPROVED);
+}
+
+// One of the two products of a CG iteration on A = Q Q + sigma over full FP64 spinors, with its
+// vector work fused (launch_split_cg): CG_NORM q = Q p (in = p) and alpha; CG_UPDATE A p = Q q
+// + sigma p (in = q), x, r and the step's scalars.  te: a half spinor for the even-odd kind,
+// whose A is 1 + sigma on the even sites.
+void square_cg_half(lym_context *c, OpEntry &op, int mode, const Spinor &q, const Spinor &in, const Spinor &p,
+                    const Spinor &x, const Spinor &r, const Spinor &te, double sigma, void *state, const int *skip)
+{
+    DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), skip);
+    P.parity = 2;
+    P.sigma = sigma;
+    P.in = P.y = in;
+    P.out = q;
+    P.v2 = p;
+    if (op.kind == LYM_OP_SQUARE_EVEN_ODD_IMPROVED) {
+        schur_even_half(c, op, PREC_D, te, in.parity(1), skip);
+        P.in = te;
+        P.y = in.parity(1);
+        P.out = q.parity(1);
+        P.even = p.parity(0);
+        P.even_identity = 1;
+        P.b = -op.kappa * op.kappa;
+    }
+    launch_dslash_cg(P, mode, p, x, r, state, c->spartials, c->counter, c->st);
+    count(c, 1);
+}
+
 // --- CG (ConjugateGradient::solve, inverters/ConjugateGradient.cpp:10-74) ---
+// matvec: A; square: the operator when A = op + sigma with op a Hermitian square (the iteration
+// then runs in 3 launches, 5 even-odd, instead of 7)
 template <class MatVec>
 int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const Spinor &x, const Spinor *guess,
-             double eps, int max_steps, lym_solve_stats *st)
+             double eps, int max_steps, lym_solve_stats *st, OpEntry *square = nullptr, double sigma = 0.0)
 {
+    if (square && !is_hermitian_square(*square)) square = nullptr;
+    std::unique_ptr<Vec> te;
+    if (square && is_even_odd(square->kind)) te.reset(new Vec(c, PREC_D, 1));
+    const Spinor half = te ? **te : Spinor();
     Vec r(c, PREC_D, nparity), p(c, PREC_D, nparity), ap(c, PREC_D, nparity);
     copy(c, x, guess ? *guess : b);
     matvec(*ap, x, nullptr);
@@ -723,10 +764,15 @@ int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const 
     CGState *S = cg_state(c);
     Gate gate{&S->pause, nullptr};
     auto step = [&]() {
-        matvec(*ap, *p, &S->pause);
-        run_site(c, OpCGAlpha<SpinorD, SpinorD>{(*p).d(), (*ap).d(), S}, nparity, gate);
-        run_site(c, OpCGUpdate<SpinorD, SpinorD, SpinorD, SpinorD>{x.d(), (*p).d(), (*r).d(), (*ap).d(), S}, nparity,
-                 gate);
+        if (square) {
+            square_cg_half(c, *square, CG_NORM, *ap, *p, *p, x, *r, half, sigma, S, &S->pause);
+            square_cg_half(c, *square, CG_UPDATE, *ap, *ap, *p, x, *r, half, sigma, S, &S->pause);
+        } else {
+            matvec(*ap, *p, &S->pause);
+            run_site(c, OpCGAlpha<SpinorD, SpinorD>{(*p).d(), (*ap).d(), S}, nparity, gate);
+            run_site(c, OpCGUpdate<SpinorD, SpinorD, SpinorD, SpinorD>{x.d(), (*p).d(), (*r).d(), (*ap).d(), S},
+                     nparity, gate);
+        }
         run_site(c, OpCGDirection<SpinorD, SpinorD>{(*p).d(), (*r).d(), S}, nparity, gate);
     };
     if (max_steps > 0) run_gated_state(c, S, step, 8, max_steps);
@@ -1416,7 +1462,7 @@ int multishift_mmmr(lym_context *c, OpEntry &op, int nshift, const double *shift
         zero(c, *z);
         lym_solve_stats s1;
         memset(&s1, 0, sizeof(s1));
-        flag = cg_solve(c, mv, 2, b, xs[first], &*z, eps, max_steps, &s1) == LYM_OK && flag;
+        flag = cg_solve(c, mv, 2, b, xs[first], &*z, eps, max_steps, &s1, &op, sh) == LYM_OK && flag;
         total += s1.iterations;
         ++first;
     }
@@ -1949,7 +1995,7 @@ int multishift_chrono(lym_context *c, OpEntry &op, int nshift, const double *shi
         }
         lym_solve_stats s1;
         memset(&s1, 0, sizeof(s1));
-        const int rc = cg_solve(c, mv, 2, b, xs[i], &*g, eps, max_steps, &s1);
+        const int rc = cg_solve(c, mv, 2, b, xs[i], &*g, eps, max_steps, &s1, &op, sh);
         ok = ok && rc == LYM_OK;
         total += s1.iterations;
     }
@@ -2957,7 +3003,7 @@ static int do_solve(lym_context *c, int op_id, int solver, double precision, int
                     auto mv = [&](const Spinor &out, const Spinor &in, const int *skip) {
                         op_apply(c, op, PREC_D, out, in, nullptr, C2(0.0), skip);
                     };
-                    rc = cg_solve(c, mv, 2, *b, *x, gp, precision, max_steps, &local);
+                    rc = cg_solve(c, mv, 2, *b, *x, gp, precision, max_steps, &local, &op);
                     break;
                 }
                 case LYM_SOLVER_BICGSTAB: {
@@ -3292,9 +3338,9 @@ static int run_multishift(lym_context *c, OpEntry &op, int algorithm, int nshift
             if (i == 0) {
                 Vec z(c, PREC_D, 2);
                 zero(c, *z);
-                rc = cg_solve(c, mv, 2, b, xv[0], &*z, precision, max_steps, &s1);
+                rc = cg_solve(c, mv, 2, b, xv[0], &*z, precision, max_steps, &s1, &op, sh);
             } else {
-                rc = cg_solve(c, mv, 2, b, xv[i], &xv[i - 1], precision, max_steps, &s1);
+                rc = cg_solve(c, mv, 2, b, xv[i], &xv[i - 1], precision, max_steps, &s1, &op, sh);
             }
             ok = ok && rc == LYM_OK;
             total += s1.iterations;

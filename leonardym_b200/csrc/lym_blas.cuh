@@ -63,8 +63,10 @@ __global__ void __launch_bounds__(kBlasThreads) site_kernel(Op op, int vh, int n
     double acc[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int k = 0; k < (Op::NRED > 0 ? Op::NRED : 1); ++k) acc[k] = 0.0;
-    for (int p = 0; p < nparity; ++p)
-        for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < vh; h += gridDim.x * blockDim.x) op.site(p, h, acc);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < vh * nparity; i += gridDim.x * blockDim.x) {
+        const int p = i >= vh ? 1 : 0;
+        op.site(p, i - p * vh, acc);
+    }
     if constexpr (Op::NRED > 0) {
         __shared__ double smem[(kBlasThreads / 32) * kMaxRed];
         __shared__ bool last;

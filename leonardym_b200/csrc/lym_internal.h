@@ -62,12 +62,14 @@ struct DslashParams {
     Spinor y;                // same-parity input (EPI_XPAY, EPI_XPAY_INV)
     Spinor v2;               // optional added vector (EPI_XPAY)
     // FP64 EPI_XPAY with parity 2 may write a caller's AoS vector instead of `out`, adding
-    // alpha times another AoS vector (aos_v2, or null; it may be aos_out itself); with even_copy
-    // the stencil runs on the odd sites only (in, y: half spinors) and the even sites get `even`
+    // alpha times another AoS vector (aos_v2, or null; it may be aos_out itself).  With
+    // even_identity (parity 2) the stencil runs on the odd sites only (in, out, y: half spinors)
+    // and the even sites get `even`.
     double *aos_out = nullptr;
     const double *aos_v2 = nullptr;
-    int even_copy = 0;
+    int even_identity = 0;
     Spinor even;
+    double sigma = 0.0;  // launch_split_cg: the shift of A
     int has_v2 = 0;
     const GaugeDev *U = nullptr;
     const void *clover = nullptr;  // T (EPI_XPAY) or Tinv (EPI_CLOVINV, EPI_XPAY_INV) of this precision
@@ -83,8 +85,9 @@ void launch_dslash(const DslashParams &P, cudaStream_t st);
 // partials: one double per block of the launch
 void launch_dslash_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
                       double *partials, unsigned int *counter, cudaStream_t st);
-// FP64 (lym_split.cu): launch_dslash and launch_dslash_cg end here for PREC_D; the partial sums of
-// a launch_split_cg over either parity or both fit in split_partials doubles
+// FP64 (lym_split.cu): launch_dslash and launch_dslash_cg end here for PREC_D.  launch_split_cg
+// takes a parity or both (p, x, r full spinors), with the shift sigma; with even_identity A is
+// 1 + sigma on the even sites.  Its partial sums fit in split_partials doubles.
 void launch_split(const DslashParams &P, cudaStream_t st);
 void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
                      double *partials, unsigned int *counter, cudaStream_t st);

@@ -39,8 +39,10 @@ enum SplitEpi : int {
     SPLIT_CLOVINV = EPI_CLOVINV,
     SPLIT_XPAY = EPI_XPAY,
     SPLIT_XPAY_INV = EPI_XPAY_INV,
-    SPLIT_CG_NORM = 10,    // EPI_XPAY with gamma5, |out|^2 reduced (CG_NORM of lym_dslash.cuh)
-    SPLIT_CG_UPDATE = 11,  // A p = EPI_XPAY with gamma5 in registers, x and r updated (CG_UPDATE)
+    // CG on A = Q Q + sigma, Q = gamma5 D or gamma5 S (Hermitian): the vector work of an iteration
+    // inside its two products, as CG_NORM / CG_UPDATE of lym_dslash.cuh
+    SPLIT_CG_NORM = 10,    // q = Q p stored, <p, A p> = |q|^2 + sigma |p|^2 reduced
+    SPLIT_CG_UPDATE = 11,  // A p = Q q + sigma p in registers; x += alpha p, r -= alpha A p, |r|^2
 };
 
 template <class GaugeT> struct SplitArg {
@@ -54,7 +56,9 @@ template <class GaugeT> struct SplitArg {
     const int *skip_if;
     double2 *aos_out;        // AOS: the full result
     const double2 *aos_v2;   // AOS: the added vector, or null
-    int even_copy;           // AOS: even sites get y (no stencil)
+    int even_identity;       // both mode: no stencil on the even sites (AOS: they get y; in
+                             // the CG modes A is 1 + sigma there)
+    double sigma;            // SPLIT_CG_*
     const double2 *alpha;    // SPLIT_CG_UPDATE
     double *partials;        // SPLIT_CG_*: [gridDim.x]
     unsigned int *counter;
@@ -151,9 +155,9 @@ LYM_D void clover_rows(const double2 *clover, int stride, int p, int h, int k, i
 struct NoFin {
     LYM_D void operator()(double) const {}
 };
-struct AlphaFin {  // alpha = |r|^2 / <p, A p> with <p, A p> = |Q p|^2
+struct AlphaFin {  // alpha = |r|^2 / <p, A p>
     CGState *s;
-    LYM_D void operator()(double qq) const { s->alpha = make_double2(s->rr / qq, 0.0); }
+    LYM_D void operator()(double pap) const { s->alpha = make_double2(s->rr / pap, 0.0); }
 };
 struct UpdateFin {  // the scalar step of OpCGUpdate
     CGState *s;
@@ -198,9 +202,13 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
     const int s = lex_of(g, c[0], c[1], c[2], c[3]);
     const int sp = 3 * (2 * d + k), so = 3 * (2 * d + 1 - k);  // words of the own and the other spin
     C res[3];
-    if (AOS && arg.even_copy && p == 0) {
+    C yo[3];  // y (NORM: p) of the own spin
+    const bool identity = (AOS || kReduce) && arg.even_identity && p == 0;
+    if (identity) {
+        if (EPI != SPLIT_CG_UPDATE) {
 #pragma unroll
-        for (int m = 0; m < 3; ++m) res[m] = load1(arg.y[0], sp + m, h);
+            for (int m = 0; m < 3; ++m) res[m] = yo[m] = load1(arg.y[0], sp + m, h);
+        }
     } else {
         C acc[3];
         split_hopping(g, arg.in[p], arg.U, p, h, s, c, k, d, acc);
@@ -222,7 +230,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
             clover_rows(arg.clover, g.stride, p, h, k, d, own, oth, res);
         } else {
 #pragma unroll
-            for (int m = 0; m < 3; ++m) own[m] = load1(arg.y[p], sp + m, h);
+            for (int m = 0; m < 3; ++m) yo[m] = own[m] = load1(arg.y[p], sp + m, h);
             if (arg.clover) {
 #pragma unroll
                 for (int m = 0; m < 3; ++m) oth[m] = load1(arg.y[p], so + m, h);
@@ -278,19 +286,26 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
             const C al = {al2.x, al2.y};
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
-                C xv = load1(arg.x[p], sp + m, h);
-                fma_c(xv, al, load1(arg.v2[p], sp + m, h));
-                const C rv = load1(arg.r[p], sp + m, h) - al * res[m];
+                const C pv = load1(arg.v2[p], sp + m, h);
+                C xv = load1(arg.x[p], sp + m, h), ap = identity ? pv : res[m];
+                fma_c(xv, al, pv);
+                fma_r(ap, arg.sigma, pv);
+                const C rv = load1(arg.r[p], sp + m, h) - al * ap;
                 part += rv.re * rv.re + rv.im * rv.im;
                 put(arg.x[p], m, xv);
                 put(arg.r[p], m, rv);
             }
         } else {
+            double pp = 0.0;
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
-                put(arg.out[p], m, res[m]);
-                if (kReduce) part += res[m].re * res[m].re + res[m].im * res[m].im;
+                if (!identity) put(arg.out[p], m, res[m]);
+                if (kReduce) {
+                    part += res[m].re * res[m].re + res[m].im * res[m].im;
+                    pp += yo[m].re * yo[m].re + yo[m].im * yo[m].im;
+                }
             }
+            if (kReduce && arg.sigma != 0.0) part += arg.sigma * pp;
         }
     }
     if constexpr (kReduce) {
@@ -331,7 +346,7 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     a.U = U;
     a.parity = P.parity;
     // views of one parity, or of the full spinors in both mode
-    const bool both = P.parity == 2 && !P.even_copy;
+    const bool both = P.parity == 2 && !P.even_identity;
     for (int p = 0; p < 2; ++p) {
         a.in[p] = both ? P.in.d(1 - p) : P.in.d();
         a.out[p] = P.out.v ? (both ? P.out.d(p) : P.out.d()) : SpinorD{};
@@ -339,7 +354,7 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
         a.v2[p] = P.v2.v ? (both ? P.v2.d(p) : P.v2.d()) : SpinorD{};
         a.x[p] = a.r[p] = SpinorD{};
     }
-    if (P.even_copy) a.y[0] = P.even.d();
+    if (P.even_identity) a.y[0] = P.even.d();
     a.clover = (const double2 *)P.clover;
     a.gamma5 = P.gamma5;
     a.has_v2 = P.has_v2;
@@ -350,7 +365,8 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     a.skip_if = P.skip_if;
     a.aos_out = (double2 *)P.aos_out;
     a.aos_v2 = (const double2 *)P.aos_v2;
-    a.even_copy = P.even_copy;
+    a.even_identity = P.even_identity;
+    a.sigma = P.sigma;
     a.alpha = nullptr;
     a.partials = nullptr;
     a.counter = nullptr;
