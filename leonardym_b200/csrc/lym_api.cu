@@ -710,12 +710,12 @@ bool is_hermitian_square(const OpEntry &op)
                          op.kind == LYM_OP_SQUARE_EVEN_ODD_IMPROVED);
 }
 
-// One of the two products of a CG iteration on A = Q Q + sigma over full FP64 spinors, with its
-// vector work fused (launch_split_cg): CG_NORM q = Q p (in = p) and alpha; CG_UPDATE A p = Q q
-// + sigma p (in = q), x, r and the step's scalars.  te: a half spinor for the even-odd kind,
-// whose A is 1 + sigma on the even sites.
-void square_cg_half(lym_context *c, OpEntry &op, int mode, const Spinor &q, const Spinor &in, const Spinor &p,
-                    const Spinor &x, const Spinor &r, const Spinor &te, double sigma, void *state, const int *skip)
+// The launch of one of the two products of an iteration on A = Q Q + sigma over full FP64
+// spinors, with the iteration's vector work fused (launch_split_cg, launch_split_ms): q = Q p
+// (in = p), then A p = Q q + sigma p (in = q).  For the even-odd kind, whose A is 1 + sigma on
+// the even sites, the product's first half is launched here (te: a half spinor).
+DslashParams square_half_params(lym_context *c, OpEntry &op, const Spinor &q, const Spinor &in, const Spinor &p,
+                                const Spinor &te, double sigma, const int *skip)
 {
     DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), skip);
     P.parity = 2;
@@ -732,8 +732,7 @@ void square_cg_half(lym_context *c, OpEntry &op, int mode, const Spinor &q, cons
         P.even_identity = 1;
         P.b = -op.kappa * op.kappa;
     }
-    launch_dslash_cg(P, mode, p, x, r, state, c->spartials, c->counter, c->st);
-    count(c, 1);
+    return P;
 }
 
 // --- CG (ConjugateGradient::solve, inverters/ConjugateGradient.cpp:10-74) ---
@@ -765,8 +764,12 @@ int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const 
     Gate gate{&S->pause, nullptr};
     auto step = [&]() {
         if (square) {
-            square_cg_half(c, *square, CG_NORM, *ap, *p, *p, x, *r, half, sigma, S, &S->pause);
-            square_cg_half(c, *square, CG_UPDATE, *ap, *ap, *p, x, *r, half, sigma, S, &S->pause);
+            for (int mode : {CG_NORM, CG_UPDATE}) {
+                const DslashParams P =
+                    square_half_params(c, *square, *ap, mode == CG_NORM ? *p : *ap, *p, half, sigma, &S->pause);
+                launch_dslash_cg(P, mode, *p, x, *r, S, c->spartials, c->counter, c->st);
+                count(c, 1);
+            }
         } else {
             matvec(*ap, *p, &S->pause);
             run_site(c, OpCGAlpha<SpinorD, SpinorD>{(*p).d(), (*ap).d(), S}, nparity, gate);
@@ -1073,7 +1076,41 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
     return rc;
 }
 
-// Multishift CG on (A + shift_i), A Hermitian positive definite (a Square* kind).
+// device arrays of spinor views of a multishift: the residual ring, the solutions (or their
+// accumulators) and the directions
+template <class View> struct MsViews {
+    lym_context *c;
+    View *ring, *x, *p;
+    static constexpr size_t kBytes = (kMsWin + 1 + 2 * kMaxShifts) * sizeof(View);
+    MsViews(lym_context *ctx, const std::vector<View> &hring, const std::vector<View> &hx, const std::vector<View> &hp)
+        : c(ctx), ring((View *)dev_alloc(ctx, kBytes)), x(ring + kMsWin + 1), p(x + kMaxShifts)
+    {
+        try {
+            CK(cudaMemcpyAsync(ring, hring.data(), hring.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+            CK(cudaMemcpyAsync(x, hx.data(), hx.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+            CK(cudaMemcpyAsync(p, hp.data(), hp.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+            CK(cudaStreamSynchronize(c->st));
+        } catch (...) {
+            dev_free(c, ring, kBytes);
+            throw;
+        }
+    }
+    ~MsViews() { dev_free(c, ring, kBytes); }
+    MsViews(const MsViews &) = delete;
+    MsViews &operator=(const MsViews &) = delete;
+    // the window's updates of every shift, then a new window (words: of one vector)
+    template <class W, class R> void flush(MultishiftState *S, int nshift, int words) const
+    {
+        const int grid = std::min((words + kMsFlushThreads - 1) / kMsFlushThreads, 4 * 148);
+        ms_flush_kernel<View, W, R><<<grid, kMsFlushThreads, 0, c->st>>>(MsFlushArg<View>{ring, x, p, S, nshift, words});
+        ms_window_reset_kernel<<<1, 32, 0, c->st>>>(S, nshift);
+        count(c, 2);
+    }
+};
+
+// Multishift CG on (A + shift_i), A Hermitian positive definite (a Square* kind), in FP64.  The
+// shifted x_i and p_i are updated once per kMsWin steps from a ring of residuals
+// (multishift_cg_mixed tells how): 4 of their vectors move per window instead of per step.
 int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts, double eps, int max_steps,
                   const Spinor &b, std::vector<Spinor> &xs, lym_solve_stats *st)
 {
@@ -1082,20 +1119,33 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     for (int i = 1; i < nshift; ++i)
         if (shifts[i] < shifts[base]) base = i;
     const double s0 = shifts[base];
-    std::vector<Vec *> ps;
-    for (int i = 0; i < nshift; ++i) ps.push_back(new Vec(c, PREC_D, 2));
-    Vec r(c, PREC_D, 2), ap(c, PREC_D, 2);
-    std::vector<SpinorD> hx(nshift), hp(nshift);
-    for (int i = 0; i < nshift; ++i) {
-        zero(c, xs[i]);
-        copy(c, **ps[i], b);
-        hx[i] = xs[i].d();
-        hp[i] = (**ps[i]).d();
+    const bool square = is_hermitian_square(op);
+    std::vector<std::unique_ptr<Vec>> owned;
+    auto fresh = [&]() {
+        owned.emplace_back(new Vec(c, PREC_D, 2));
+        return **owned.back();
+    };
+    std::vector<SpinorD> hring, hx, hp;
+    for (int j = 0; j <= kMsWin; ++j) {
+        const Spinor r = fresh();
+        if (j == 0) copy(c, r, b);  // r_0 = b
+        hring.push_back(r.d());
     }
-    copy(c, *r, b);
-    SpinorD *dviews = (SpinorD *)dev_alloc(c, 2 * kMaxShifts * sizeof(SpinorD));
-    CK(cudaMemcpyAsync(dviews, hx.data(), nshift * sizeof(SpinorD), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(dviews + kMaxShifts, hp.data(), nshift * sizeof(SpinorD), cudaMemcpyHostToDevice, c->st));
+    for (int i = 0; i < nshift; ++i) {
+        const Spinor p = fresh();
+        zero(c, xs[i]);
+        copy(c, p, b);
+        hx.push_back(xs[i].d());
+        hp.push_back(p.d());
+    }
+    // the base direction of the current step (the operator's input), and A p or Q p
+    Vec pcur(c, PREC_D, 2), ap(c, PREC_D, 2);
+    std::unique_ptr<Vec> te;
+    if (square && is_even_odd(op.kind)) te.reset(new Vec(c, PREC_D, 1));
+    const Spinor half = te ? **te : Spinor();
+    const Spinor pb = *pcur;
+    copy(c, pb, b);
+    const MsViews<SpinorD> views(c, hring, hx, hp);
     const double bb = norm2_now(c, b);
     // build the clover term and pool the operator's temporaries before graph capture
     op_apply(c, op, PREC_D, *ap, b, &b, C2(s0));
@@ -1107,6 +1157,7 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
         H.sigma[i] = shifts[i] - s0;
         H.zeta[i] = H.zeta_prev[i] = 1.0;
         H.active[i] = 1;
+        H.cp[i][0] = 1.0;
     }
     H.rr = bb;
     H.alpha = 1.0;
@@ -1116,16 +1167,26 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     CK(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(MultishiftState), cudaMemcpyHostToDevice, c->st));
     MultishiftState *S = (MultishiftState *)c->d_state;
     Gate gate{&S->pause, nullptr};
-    const Spinor pb = **ps[base];
+    int nstep = 0;
     auto step = [&]() {
-        op_apply(c, op, PREC_D, *ap, pb, &pb, C2(s0), &S->pause);
-        run_site(c, OpMsAlpha<SpinorD, SpinorD>{pb.d(), (*ap).d(), S}, 2, gate);
-        run_site(c, OpMsResidual<SpinorD, SpinorD>{(*r).d(), (*ap).d(), S}, 2, gate);
-        run_site(c, OpMsUpdate<SpinorD>{dviews, dviews + kMaxShifts, (*r).d(), S, nshift}, 2, gate);
+        if (square) {
+            for (int mode : {CG_NORM, CG_UPDATE}) {
+                const DslashParams P =
+                    square_half_params(c, op, *ap, mode == CG_NORM ? pb : *ap, pb, half, s0, &S->pause);
+                launch_split_ms(P, mode, pb, views.ring, S, c->spartials, c->counter, c->st);
+                count(c, 1);
+            }
+        } else {
+            op_apply(c, op, PREC_D, *ap, pb, &pb, C2(s0), &S->pause);
+            run_site(c, OpMsAlpha<SpinorD, SpinorD>{pb.d(), (*ap).d(), S}, 2, gate);
+            run_site(c, OpMsResidualRing<SpinorD, SpinorD>{views.ring, (*ap).d(), S}, 2, gate);
+        }
+        run_site(c, OpMsBaseDirection<SpinorD, SpinorD>{views.ring, pb.d(), S}, 2, gate);
+        if (++nstep % kMsWin == 0) views.template flush<double2, double>(S, nshift, 2 * 12 * c->g.stride);
     };
     int rc = LYM_OK;
     if (bb > 0 && max_steps > 0) {
-        run_gated_state(c, S, step, 4, max_steps);
+        run_gated_state(c, S, step, kMsWin, max_steps);
         MultishiftState &R = *(MultishiftState *)c->h_state;
         rc = R.converged ? LYM_OK : LYM_NOT_CONVERGED;
         if (st) {
@@ -1135,8 +1196,6 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
             st->last_error = R.rr;
         }
     }
-    for (auto v : ps) delete v;
-    dev_free(c, dviews, 2 * kMaxShifts * sizeof(SpinorD));
     return rc;
 }
 
@@ -1292,23 +1351,7 @@ int multishift_cg_mixed(lym_context *c, OpEntry &op, int rprec, int nshift, cons
         Spinor r0 = **owned.front();
         copy(c, r0, bo);
     }
-    // device arrays of views: ring, accumulators, directions
-    const size_t vb = sizeof(SpinorF);
-    const size_t nview = (kMsWin + 1) + 2 * kMaxShifts;
-    char *dviews = (char *)dev_alloc(c, nview * vb);
-    struct ViewsMem {
-        lym_context *c;
-        void *p;
-        size_t n;
-        ~ViewsMem() { dev_free(c, p, n); }
-    } vmem{c, dviews, nview * vb};
-    SpinorF *d_ring = (SpinorF *)dviews;
-    SpinorF *d_acc = d_ring + (kMsWin + 1);
-    SpinorF *d_p = d_acc + kMaxShifts;
-    CK(cudaMemcpyAsync(d_ring, hring.data(), (kMsWin + 1) * vb, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(d_acc, hacc.data(), nshift * vb, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(d_p, hp.data(), nshift * vb, cudaMemcpyHostToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    const MsViews<SpinorF> views(c, hring, hacc, hp);
     auto pview = [&](int i) {
         Spinor v;
         v.prec = PREC_F;
@@ -1357,19 +1400,12 @@ int multishift_cg_mixed(lym_context *c, OpEntry &op, int rprec, int nshift, cons
     Gate gate{&S->pause, nullptr};
     const Spinor xb = xs[base].parity(1);
     int nstep = 0;
-    const int fgrid = std::min((c->g.Vh + kMsFlushThreads - 1) / kMsFlushThreads, 4 * 148);
-    auto flush = [&]() {
-        MsFlushArg fa{d_ring, d_acc, d_p, S, nshift, c->g.Vh};
-        ms_flush_kernel<<<fgrid, kMsFlushThreads, 0, c->st>>>(fa);
-        ms_window_reset_kernel<<<1, 32, 0, c->st>>>(S, nshift);
-        count(c, 2);
-    };
     auto step = [&]() {
         schur_square_shift(c, op, PREC_F, *ap, pb, *tos, *tes, s0, &S->pause);
         run_site(c, OpMsAlpha<SpinorF, SpinorF>{pb.f(), (*ap).f(), S}, 1, gate);
-        run_site(c, OpMsResidualRing<SpinorF>{d_ring, (*ap).f(), S}, 1, gate);
-        run_site(c, OpMsBaseDirection<SpinorF>{d_ring, pb.f(), S}, 1, gate);
-        if (++nstep % kMsWin == 0) flush();
+        run_site(c, OpMsResidualRing<SpinorF, SpinorF>{views.ring, (*ap).f(), S}, 1, gate);
+        run_site(c, OpMsBaseDirection<SpinorF, SpinorF>{views.ring, pb.f(), S}, 1, gate);
+        if (++nstep % kMsWin == 0) views.template flush<float4, float>(S, nshift, 6 * c->g.stride);
     };
     auto base_true_res = [&]() {
         schur_square_shift(c, op, PREC_D, *u64, xb, *t64, *te64, s0);
@@ -1417,7 +1453,7 @@ int multishift_cg_mixed(lym_context *c, OpEntry &op, int rprec, int nshift, cons
             CK(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(MultishiftState), cudaMemcpyHostToDevice, c->st));
             const Spinor rcur = ring_view(R.iter);
             copy(c, rcur, *r64);
-            run_site(c, OpMsDirection<SpinorF, SpinorF>{d_p, rcur.f(), S, nshift}, 1);
+            run_site(c, OpMsDirection<SpinorF, SpinorF>{views.p, rcur.f(), S, nshift}, 1);
             copy(c, *pcur, pview(base));
         }
     }

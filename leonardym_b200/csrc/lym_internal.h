@@ -91,6 +91,10 @@ void launch_dslash_cg(const DslashParams &P, int mode, const Spinor &p, const Sp
 void launch_split(const DslashParams &P, cudaStream_t st);
 void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
                      double *partials, unsigned int *counter, cudaStream_t st);
+// launch_split_ms: the same two products of a multishift step on both parities (CG_NORM, then
+// the residual: ring, a device array of kMsWin + 1 SpinorD views; state: the MultishiftState).
+void launch_split_ms(const DslashParams &P, int mode, const Spinor &p, const void *ring, void *state, double *partials,
+                     unsigned int *counter, cudaStream_t st);
 int split_partials(const Geom &g);
 void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in, const void *clover, int parity,
                    int gamma5, cudaStream_t st);

@@ -521,7 +521,30 @@ struct MultishiftState {
     double cx[kMaxShifts][kMsWin + 1], cp[kMaxShifts][kMsWin + 1];
 };
 
-// base alpha = rr / <p, Ap>, then the shifted coefficients (Jegerlehner recursions)
+// base alpha = rr / <p, Ap>, then the shifted coefficients (Jegerlehner recursions).
+// On entry s->alpha = alpha_{k-1}, s->beta = beta_k (p_k = r_k + beta_k p_{k-1}),
+// zeta = zeta_k, zeta_prev = zeta_{k-1}.  For (A + sigma) with residuals
+// r^sigma_k = zeta_k r_k the three-term recurrences give
+//   zeta_{k+1} = zeta_k zeta_{k-1} a_{k-1} /
+//                (zeta_{k-1} a_{k-1} (1 + sigma a_k) + a_k b_k (zeta_{k-1} - zeta_k))
+//   a^sigma_k  = a_k zeta_{k+1} / zeta_k.
+LYM_D void ms_alpha_step(MultishiftState *s, double pap)
+{
+    const double a = s->rr / pap;
+    const double am1 = s->alpha;
+    for (int i = 0; i < s->nshift; ++i) {
+        if (s->active[i] == 2) s->active[i] = 0;  // converged at the previous step
+        if (!s->active[i]) continue;
+        const double z = s->zeta[i], zp = s->zeta_prev[i];
+        const double den = zp * am1 * (1.0 + s->sigma[i] * a) + a * s->beta * (zp - z);
+        const double zn = (z * zp * am1) / den;
+        s->alpha_s[i] = a * zn / z;
+        s->zeta_prev[i] = z;
+        s->zeta[i] = zn;
+    }
+    s->alpha_prev = am1;
+    s->alpha = a;
+}
 template <class SP, class SAp> struct OpMsAlpha {
     static constexpr int NRED = 2;
     SP p;
@@ -534,29 +557,7 @@ template <class SP, class SAp> struct OpMsAlpha {
         ap.par(q).template load<double>(h, y);
         dotc(x, y, acc[0], acc[1]);
     }
-    // On entry s->alpha = alpha_{k-1}, s->beta = beta_k (p_k = r_k + beta_k p_{k-1}),
-    // zeta = zeta_k, zeta_prev = zeta_{k-1}.  For (A + sigma) with residuals
-    // r^sigma_k = zeta_k r_k the three-term recurrences give
-    //   zeta_{k+1} = zeta_k zeta_{k-1} a_{k-1} /
-    //                (zeta_{k-1} a_{k-1} (1 + sigma a_k) + a_k b_k (zeta_{k-1} - zeta_k))
-    //   a^sigma_k  = a_k zeta_{k+1} / zeta_k.
-    LYM_D void finalize(const double *t) const
-    {
-        const double a = s->rr / t[0];
-        const double am1 = s->alpha;
-        for (int i = 0; i < s->nshift; ++i) {
-            if (s->active[i] == 2) s->active[i] = 0;  // converged at the previous step
-            if (!s->active[i]) continue;
-            const double z = s->zeta[i], zp = s->zeta_prev[i];
-            const double den = zp * am1 * (1.0 + s->sigma[i] * a) + a * s->beta * (zp - z);
-            const double zn = (z * zp * am1) / den;
-            s->alpha_s[i] = a * zn / z;
-            s->zeta_prev[i] = z;
-            s->zeta[i] = zn;
-        }
-        s->alpha_prev = am1;
-        s->alpha = a;
-    }
+    LYM_D void finalize(const double *t) const { ms_alpha_step(s, t[0]); }
 };
 
 // After r_{k+1}: beta, the shifted betas, per-shift convergence, reliable-update and stop
@@ -586,7 +587,7 @@ LYM_D bool ms_residual_step(MultishiftState *s, double rr_new)
         if (zr < s->eps && i != s->base) s->active[i] = 2;
         else if (zr >= s->eps) any = 1;
     }
-    // the x / p update of this step (OpMsUpdate) still runs; it turns stop into pause
+    // the updates of this step still run; OpMsBaseDirection turns stop into pause
     if (!any) {
         s->converged = 1;
         s->stop = 1;
@@ -600,28 +601,9 @@ LYM_D bool ms_residual_step(MultishiftState *s, double rr_new)
     return true;
 }
 
-// x_i += alpha_i p_i ; r -= alpha Ap ; rr_new
-template <class SR, class SAp> struct OpMsResidual {
-    static constexpr int NRED = 1;
-    SR r;
-    SAp ap;
-    MultishiftState *s;
-    LYM_D void site(int q, int h, double *acc) const
-    {
-        const double a = s->alpha;
-        cx<double> rv[12], av[12];
-        r.par(q).template load<double>(h, rv);
-        ap.par(q).template load<double>(h, av);
-#pragma unroll
-        for (int k = 0; k < 12; ++k) rv[k] = rv[k] - a * av[k];
-        acc[0] += norm2(rv);
-        r.par(q).template store<double>(h, rv);
-    }
-    LYM_D void finalize(const double *t) const { ms_residual_step(s, t[0]); }
-};
-
-// Windowed form of OpMsUpdate's step: x_i += alpha_i p_i and p_i = zeta_i R_m + beta_i p_i
-// applied to the coefficients of x_i and p_i (same conditions as OpMsUpdate), R_m = r_{k+1}.
+// The shifted updates of a step, x_i += alpha_i p_i (a converged shift's last one included) and
+// p_i = zeta_i R_m + beta_i p_i (not after a step that asks for a reliable update), applied to
+// the coefficients of x_i and p_i, R_m = r_{k+1}.
 LYM_D void ms_window_step(MultishiftState *s)
 {
     const int m = s->win;
@@ -642,17 +624,17 @@ LYM_D void ms_window_step(MultishiftState *s)
     s->win = m + 1;
 }
 
-// r_{k+1} = r_k - alpha Ap with the residuals in a ring of kMsWin + 1 FP32 slots (r_k in
-// slot k mod (kMsWin + 1)), |r_{k+1}|^2, then the step's scalars and window coefficients.
-template <class SAp> struct OpMsResidualRing {
+// r_{k+1} = r_k - alpha Ap with the residuals in a ring of kMsWin + 1 slots (r_k in slot
+// k mod (kMsWin + 1)), |r_{k+1}|^2, then the step's scalars and window coefficients.
+template <class SR, class SAp> struct OpMsResidualRing {
     static constexpr int NRED = 1;
-    const SpinorF *ring;
+    const SR *ring;
     SAp ap;
     MultishiftState *s;
     LYM_D void site(int q, int h, double *acc) const
     {
         const int k = s->iter;
-        const SpinorF rin = ring[k % (kMsWin + 1)], rout = ring[(k + 1) % (kMsWin + 1)];
+        const SR rin = ring[k % (kMsWin + 1)], rout = ring[(k + 1) % (kMsWin + 1)];
         const double a = s->alpha;
         cx<double> rv[12], av[12];
         rin.par(q).template load<double>(h, rv);
@@ -670,9 +652,9 @@ template <class SAp> struct OpMsResidualRing {
 
 // the base system's direction, materialised every step for the operator: p = r_{k+1} + beta p
 // (not after a step that asks for a reliable update: the host rebuilds it from the true residual)
-template <class SP> struct OpMsBaseDirection {
+template <class SR, class SP> struct OpMsBaseDirection {
     static constexpr int NRED = 1;  // no sum; finalize ends the step
-    const SpinorF *ring;
+    const SR *ring;
     SP p;
     MultishiftState *s;
     LYM_D void site(int q, int h, double *) const
@@ -694,32 +676,50 @@ template <class SP> struct OpMsBaseDirection {
 
 // Window flush: per shift x_i += cx_i0 P_i + sum_j cx_i(j+1) R_j and (running shifts)
 // P_i = cp_i0 P_i + sum_j cp_i(j+1) R_j, R_j = r_{k0+1+j}: one pass over x_i and P_i
-// per window instead of one per step.  FP32 words streamed one at a time; coefficients in
-// shared memory.  Runs whether or not the state is paused (a pause ends the window early).
-struct MsFlushArg {
-    const SpinorF *ring;  // kMsWin + 1 residual slots
-    const SpinorF *x;     // per-shift FP32 solution accumulators
-    const SpinorF *p;     // per-shift directions
+// per window instead of one per step.  The vectors are streamed as flat arrays of words (the
+// padding of their strides included, which nothing reads); coefficients in shared memory, in the
+// precision of the vectors.  Runs whether or not the state is paused (a pause ends the window
+// early).  HBM bound: 24^3 x 48, 12 FP32 shifts of one parity, 224 us a window.
+template <class View> struct MsFlushArg {
+    const View *ring;  // kMsWin + 1 residual slots
+    const View *x;     // per-shift solutions or their accumulators
+    const View *p;     // per-shift directions
     MultishiftState *s;
     int nshift;
-    int vh;
+    int words;         // of one vector
 };
+
+LYM_D float4 word_scale(float c, float4 v) { return make_float4(c * v.x, c * v.y, c * v.z, c * v.w); }
+LYM_D double2 word_scale(double c, double2 v) { return make_double2(c * v.x, c * v.y); }
+LYM_D void word_add(float4 &a, float c, float4 v)
+{
+    a.x += c * v.x;
+    a.y += c * v.y;
+    a.z += c * v.z;
+    a.w += c * v.w;
+}
+LYM_D void word_add(double2 &a, double c, double2 v)
+{
+    a.x += c * v.x;
+    a.y += c * v.y;
+}
 
 constexpr int kMsFlushThreads = 256;
 
-static __global__ void __launch_bounds__(kMsFlushThreads) ms_flush_kernel(MsFlushArg a)
+template <class View, class W, class R>
+__global__ void __launch_bounds__(kMsFlushThreads) ms_flush_kernel(MsFlushArg<View> a)
 {
-    __shared__ float cxs[kMaxShifts][kMsWin + 1], cps[kMaxShifts][kMsWin + 1];
+    __shared__ R cxs[kMaxShifts][kMsWin + 1], cps[kMaxShifts][kMsWin + 1];
     __shared__ int fl[kMaxShifts];
-    __shared__ float4 *xp[kMaxShifts], *pp[kMaxShifts], *rp[kMsWin];
+    __shared__ W *xp[kMaxShifts], *pp[kMaxShifts], *rp[kMsWin];
     const MultishiftState *s = a.s;
     const int m = s->win;
     if (m == 0) return;
     const int k0 = s->iter - m;
     for (int t = threadIdx.x; t < a.nshift * (kMsWin + 1); t += blockDim.x) {
         const int i = t / (kMsWin + 1), j = t % (kMsWin + 1);
-        cxs[i][j] = (float)s->cx[i][j];
-        cps[i][j] = (float)s->cp[i][j];
+        cxs[i][j] = (R)s->cx[i][j];
+        cps[i][j] = (R)s->cp[i][j];
     }
     for (int i = threadIdx.x; i < a.nshift; i += blockDim.x) {
         fl[i] = (s->xupd[i] ? 1 : 0) | ((s->pupd[i] && s->active[i] == 1) ? 2 : 0);
@@ -728,33 +728,26 @@ static __global__ void __launch_bounds__(kMsFlushThreads) ms_flush_kernel(MsFlus
     }
     for (int j = threadIdx.x; j < m; j += blockDim.x) rp[j] = a.ring[(k0 + 1 + j) % (kMsWin + 1)].v;
     __syncthreads();
-    const int stride = a.ring[0].stride;
-    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < a.vh; h += gridDim.x * blockDim.x) {
-        for (int w = 0; w < 6; ++w) {
-            const size_t o = (size_t)w * stride + h;
-            float4 R[kMsWin];
+    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < a.words; o += gridDim.x * blockDim.x) {
+        W Rj[kMsWin];
 #pragma unroll
-            for (int j = 0; j < kMsWin; ++j)
-                if (j < m) R[j] = rp[j][o];
-            for (int i = 0; i < a.nshift; ++i) {
-                const int f = fl[i];
-                if (!f) continue;
-                const float4 P = pp[i][o];
-                float4 X = xp[i][o], Q;
-                const float c0 = cxs[i][0], d0 = cps[i][0];
-                X.x += c0 * P.x; X.y += c0 * P.y; X.z += c0 * P.z; X.w += c0 * P.w;
-                Q.x = d0 * P.x; Q.y = d0 * P.y; Q.z = d0 * P.z; Q.w = d0 * P.w;
+        for (int j = 0; j < kMsWin; ++j)
+            if (j < m) Rj[j] = rp[j][o];
+        for (int i = 0; i < a.nshift; ++i) {
+            const int f = fl[i];
+            if (!f) continue;
+            const W P = pp[i][o];
+            W X = xp[i][o], Q = word_scale(cps[i][0], P);
+            word_add(X, cxs[i][0], P);
 #pragma unroll
-                for (int j = 0; j < kMsWin; ++j) {
-                    if (j < m) {
-                        const float c = cxs[i][j + 1], d = cps[i][j + 1];
-                        X.x += c * R[j].x; X.y += c * R[j].y; X.z += c * R[j].z; X.w += c * R[j].w;
-                        Q.x += d * R[j].x; Q.y += d * R[j].y; Q.z += d * R[j].z; Q.w += d * R[j].w;
-                    }
+            for (int j = 0; j < kMsWin; ++j) {
+                if (j < m) {
+                    word_add(X, cxs[i][j + 1], Rj[j]);
+                    word_add(Q, cps[i][j + 1], Rj[j]);
                 }
-                xp[i][o] = X;
-                if (f & 2) pp[i][o] = Q;
             }
+            xp[i][o] = X;
+            if (f & 2) pp[i][o] = Q;
         }
     }
 }
@@ -770,44 +763,6 @@ static __global__ void ms_window_reset_kernel(MultishiftState *s, int nshift)
     }
     if (i == 0) s->win = 0;
 }
-
-// per shift: x_i += alpha_i p_i ; p_i = zeta_i r + beta_i p_i  (one launch over all shifts;
-// a step that asks for a reliable update leaves the directions to OpMsDirection)
-template <class SX, class SP = SX, class SR = SX> struct OpMsUpdate {
-    static constexpr int NRED = 1;  // no sum; finalize ends the step
-    SX *x;   // device array of nshift views
-    SP *ps;
-    SR r;
-    MultishiftState *s;
-    int nshift;
-    LYM_D void site(int q, int h, double *) const
-    {
-        cx<double> rv[12];
-        const bool dir = !s->need_update;
-        if (dir) r.par(q).template load<double>(h, rv);
-        for (int i = 0; i < nshift; ++i) {
-            const int act = s->active[i];
-            if (!act) continue;
-            cx<double> xv[12], pv[12];
-            x[i].par(q).template load<double>(h, xv);
-            ps[i].par(q).template load<double>(h, pv);
-            const double ai = s->alpha_s[i];
-#pragma unroll
-            for (int k = 0; k < 12; ++k) fma_r(xv[k], ai, pv[k]);
-            x[i].par(q).template store<double>(h, xv);
-            if (act == 1 && dir) {
-                const double z = s->zeta[i], b = s->beta_s[i];
-#pragma unroll
-                for (int k = 0; k < 12; ++k) pv[k] = z * rv[k] + b * pv[k];
-                ps[i].par(q).template store<double>(h, pv);
-            }
-        }
-    }
-    LYM_D void finalize(const double *) const
-    {
-        if (s->stop) s->pause = 1;
-    }
-};
 
 // p_i = zeta_i r + beta_i p_i for the running shifts (after a reliable update of r)
 template <class SP, class SR> struct OpMsDirection {

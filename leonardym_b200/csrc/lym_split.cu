@@ -43,6 +43,8 @@ enum SplitEpi : int {
     // inside its two products, as CG_NORM / CG_UPDATE of lym_dslash.cuh
     SPLIT_CG_NORM = 10,    // q = Q p stored, <p, A p> = |q|^2 + sigma |p|^2 reduced
     SPLIT_CG_UPDATE = 11,  // A p = Q q + sigma p in registers; x += alpha p, r -= alpha A p, |r|^2
+    // the second product of a multishift step: r_{k+1} = r_k - alpha A p in a ring of residuals
+    SPLIT_MS_RESIDUAL = 12,
 };
 
 template <class GaugeT> struct SplitArg {
@@ -60,6 +62,8 @@ template <class GaugeT> struct SplitArg {
                              // the CG modes A is 1 + sigma there)
     double sigma;            // SPLIT_CG_*
     const double2 *alpha;    // SPLIT_CG_UPDATE
+    const SpinorD *ring;     // SPLIT_MS_RESIDUAL: kMsWin + 1 full spinors
+    const MultishiftState *ms;
     double *partials;        // SPLIT_CG_*: [gridDim.x]
     unsigned int *counter;
 };
@@ -159,6 +163,17 @@ struct AlphaFin {  // alpha = |r|^2 / <p, A p>
     CGState *s;
     LYM_D void operator()(double pap) const { s->alpha = make_double2(s->rr / pap, 0.0); }
 };
+struct MsAlphaFin {
+    MultishiftState *s;
+    LYM_D void operator()(double pap) const { ms_alpha_step(s, pap); }
+};
+struct MsResidualFin {
+    MultishiftState *s;
+    LYM_D void operator()(double rr) const
+    {
+        if (ms_residual_step(s, rr)) ms_window_step(s);
+    }
+};
 struct UpdateFin {  // the scalar step of OpCGUpdate
     CGState *s;
     LYM_D void operator()(double rr) const
@@ -173,7 +188,8 @@ template <int EPI, bool AOS, class GaugeT, class Fin>
 __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<GaugeT> arg, const Fin fin)
 {
     if (arg.skip_if && *arg.skip_if) return;
-    constexpr bool kReduce = EPI == SPLIT_CG_NORM || EPI == SPLIT_CG_UPDATE;
+    constexpr bool kSecond = EPI == SPLIT_CG_UPDATE || EPI == SPLIT_MS_RESIDUAL;  // A p stays in registers
+    constexpr bool kReduce = EPI == SPLIT_CG_NORM || kSecond;
     constexpr bool kXpay = EPI == SPLIT_XPAY || kReduce;
     constexpr int kTileWord = 13;  // 12 words of a site, 1 of padding
     __shared__ __align__(16) double2 tile[AOS ? kSplitSites * kTileWord : 1];
@@ -205,7 +221,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
     C yo[3];  // y (NORM: p) of the own spin
     const bool identity = (AOS || kReduce) && arg.even_identity && p == 0;
     if (identity) {
-        if (EPI != SPLIT_CG_UPDATE) {
+        if (!kSecond) {
 #pragma unroll
             for (int m = 0; m < 3; ++m) res[m] = yo[m] = load1(arg.y[0], sp + m, h);
         }
@@ -295,6 +311,19 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
                 put(arg.x[p], m, xv);
                 put(arg.r[p], m, rv);
             }
+        } else if constexpr (EPI == SPLIT_MS_RESIDUAL) {
+            const int it = arg.ms->iter;
+            const SpinorD rin = arg.ring[it % (kMsWin + 1)].par(p), rout = arg.ring[(it + 1) % (kMsWin + 1)].par(p);
+            const double al = arg.ms->alpha;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const C pv = load1(arg.v2[p], sp + m, h);
+                C ap = identity ? pv : res[m], rv = load1(rin, sp + m, h);
+                fma_r(ap, arg.sigma, pv);
+                fma_r(rv, -al, ap);
+                part += rv.re * rv.re + rv.im * rv.im;
+                put(rout, m, rv);
+            }
         } else {
             double pp = 0.0;
 #pragma unroll
@@ -368,6 +397,8 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     a.even_identity = P.even_identity;
     a.sigma = P.sigma;
     a.alpha = nullptr;
+    a.ring = nullptr;
+    a.ms = nullptr;
     a.partials = nullptr;
     a.counter = nullptr;
     return a;
@@ -415,6 +446,22 @@ void run_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor
     else split_kernel<SPLIT_CG_UPDATE, false><<<nb, nt, 0, st>>>(a, UpdateFin{cs});
 }
 
+template <class GaugeT>
+void run_split_ms(const DslashParams &P, int mode, const Spinor &p, const SpinorD *ring, MultishiftState *ms,
+                  double *partials, unsigned int *counter, const GaugeT &U, cudaStream_t st)
+{
+    SplitArg<GaugeT> a = split_arg(P, U);
+    for (int q = 0; q < 2; ++q) a.v2[q] = p.d(q);
+    a.gamma5 = 1;
+    a.ring = ring;
+    a.ms = ms;
+    a.partials = partials;
+    a.counter = counter;
+    const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
+    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, MsAlphaFin{ms});
+    else split_kernel<SPLIT_MS_RESIDUAL, false><<<nb, nt, 0, st>>>(a, MsResidualFin{ms});
+}
+
 }  // namespace
 
 int split_partials(const Geom &g) { return split_blocks(g, 2); }
@@ -434,6 +481,18 @@ void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spi
         run_split_cg(P, mode, p, x, r, (CGState *)state, partials, counter, GaugeD18{(const double2 *)P.U->d64, s}, st);
     else
         run_split_cg(P, mode, p, x, r, (CGState *)state, partials, counter, GaugeD9{(const double *)P.U->d64, s}, st);
+}
+
+void launch_split_ms(const DslashParams &P, int mode, const Spinor &p, const void *ring, void *state, double *partials,
+                     unsigned int *counter, cudaStream_t st)
+{
+    const int s = P.g.stride;
+    const SpinorD *rv = (const SpinorD *)ring;
+    MultishiftState *ms = (MultishiftState *)state;
+    if (P.rep == REP_SU3)
+        run_split_ms(P, mode, p, rv, ms, partials, counter, GaugeD18{(const double2 *)P.U->d64, s}, st);
+    else
+        run_split_ms(P, mode, p, rv, ms, partials, counter, GaugeD9{(const double *)P.U->d64, s}, st);
 }
 
 }  // namespace lym
