@@ -3582,9 +3582,9 @@ static int do_meson(lym_context *c, const double *const *props, double *pion, do
                 P.p[k] = (const double2 *)staged.back()->p;
             }
         }
-        DevBuf scratch(c, meson_scratch_bytes(c->g)), res(c, 3 * (size_t)Lt * sizeof(double));
+        DevBuf scratch(c, meson_scratch_bytes(c->g), false), res(c, 3 * (size_t)Lt * sizeof(double), false);
         launch_meson_contractions(c->g, P, (double *)scratch.p, (double *)res.p, c->st);
-        count(c, 2);
+        count(c, 3);
         std::vector<double> h(3 * (size_t)Lt);
         CK(cudaMemcpyAsync(h.data(), res.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
