@@ -311,6 +311,23 @@ void copy(lym_context *c, const Spinor &dst, const Spinor &src)
     launch_convert(c->g, dst, src, c->st);
 }
 
+// the FP64 x of one parity plus an accumulator of another precision, which starts again from zero
+void fold(lym_context *c, const Spinor &acc, const Spinor &x)
+{
+    if (acc.prec == PREC_D) run_site(c, OpFoldClear<SpinorD, SpinorD>{acc.d(), x.d()}, 1);
+    else if (acc.prec == PREC_F) run_site(c, OpFoldClear<SpinorF, SpinorD>{acc.f(), x.d()}, 1);
+    else run_site(c, OpFoldClear<SpinorH, SpinorD>{acc.h(), x.d()}, 1);
+}
+
+// CG going on after a reliable update with the FP64 residual rt: r = rt, p = rt + b p (r FP32
+// for reduced-precision p)
+void cg_continue(lym_context *c, const Spinor &r, const Spinor &p, const Spinor &rt, double b)
+{
+    if (p.prec == PREC_D) run_site(c, OpCGContinue<SpinorD, SpinorD, SpinorD>{r.d(), p.d(), rt.d(), b}, 1);
+    else if (p.prec == PREC_F) run_site(c, OpCGContinue<SpinorF, SpinorF, SpinorD>{r.f(), p.f(), rt.d(), b}, 1);
+    else run_site(c, OpCGContinue<SpinorF, SpinorH, SpinorD>{r.f(), p.h(), rt.d(), b}, 1);
+}
+
 void zero(lym_context *c, const Spinor &s) { CK(cudaMemsetAsync(s.v, 0, spinor_bytes(c->g, s.prec, s.nparity), c->st)); }
 
 double norm2_now(lym_context *c, const Spinor &x)
@@ -506,26 +523,14 @@ void apply_schur_cg(lym_context *c, OpEntry &op, int prec, int mode, const Spino
                     const Spinor &tmp_e, const Spinor &p, const Spinor &x, const Spinor &r, void *state,
                     const int *skip)
 {
-    GaugeEntry &ge = gauge_of(c, op.gauge_id);
-    const bool clov = kind_has_clover(op.kind);
-    if (clov) ensure_clover(c, op);
-    require_recon(c, ge, prec);
-    DslashParams P;
-    P.g = c->g;
-    P.prec = prec;
-    P.rep = c->rep;
-    P.U = &ge.dev;
-    P.skip_if = skip;
     schur_even_half(c, op, prec, tmp_e, in_o, skip);
-    P.epi = EPI_XPAY_;
+    DslashParams P = full_params(c, op, prec, 1, C2(0.0), skip);
     P.parity = 1;
     P.in = tmp_e;
     P.out = out_o;
     P.y = in_o;
     P.v2 = p;
-    P.clover = clov ? op.clover.T[prec] : nullptr;
     P.b = -op.kappa * op.kappa;
-    P.gamma5 = 1;
     launch_dslash_cg(P, mode, p, x, r, state, c->spartials, c->counter, c->st);
     count(c, 1);
 }
@@ -661,46 +666,72 @@ void push_state(lym_context *c, size_t bytes)
     CK(cudaMemcpyAsync(c->d_state, c->h_state, bytes, cudaMemcpyHostToDevice, c->st));
 }
 
-// Run `step` (one iteration; every kernel gated on the state's `pause` flag)
-// until the device state pauses.  Batches of iterations are captured once into a
-// CUDA graph and replayed; the host reads the state once per batch.
+// Runs `step` (one iteration; every kernel gated on the state's `pause` flag) until the device
+// state pauses.  `batch` iterations are captured once into a CUDA graph and replayed; the host
+// reads the state once per replay.  A solve that pauses for reliable updates keeps its loop and
+// replays the same graph (capturing and instantiating it again took 0.3-0.4 ms each time).
+template <class S, class Step> class GatedLoop {
+public:
+    GatedLoop(lym_context *ctx, S *state, Step st, int batch_) : c(ctx), d(state), step(st), batch(batch_) {}
+    ~GatedLoop()
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+    }
+    GatedLoop(const GatedLoop &) = delete;
+    GatedLoop &operator=(const GatedLoop &) = delete;
+
+    void run(long max_iterations)
+    {
+        if (!exec) capture();
+        // every iteration pauses the state by itself at its iteration limit; the host
+        // bound below only guards against a state that never pauses
+        const long max_launches = max_iterations / batch + 4;
+        for (long l = 0; l < max_launches; ++l) {
+            CK(cudaGraphLaunch(exec, c->st));
+            c->launches += nodes;
+            CK(cudaMemcpyAsync(c->h_state, d, sizeof(S), cudaMemcpyDeviceToHost, c->st));
+            CK(cudaStreamSynchronize(c->st));
+            if (((S *)c->h_state)->pause) {
+                CK(cudaGetLastError());
+                return;
+            }
+        }
+        CK(cudaGetLastError());
+        fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %ld iterations", max_iterations);
+    }
+
+private:
+    void capture()
+    {
+        cudaGraph_t graph = nullptr;
+        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
+        c->capturing = true;
+        try {
+            for (int k = 0; k < batch; ++k) step();
+        } catch (...) {
+            c->capturing = false;
+            cudaStreamEndCapture(c->st, &graph);
+            if (graph) cudaGraphDestroy(graph);
+            throw;
+        }
+        c->capturing = false;
+        CK(cudaStreamEndCapture(c->st, &graph));
+        const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+        cudaGraphGetNodes(graph, nullptr, &nodes);
+        cudaGraphDestroy(graph);
+        CK(e);
+    }
+    lym_context *c;
+    S *d;
+    Step step;
+    int batch;
+    cudaGraphExec_t exec = nullptr;
+    size_t nodes = 0;
+};
+
 template <class S, class Step> void run_gated_state(lym_context *c, S *d, Step step, int batch, long max_iterations)
 {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
-    c->capturing = true;
-    try {
-        for (int k = 0; k < batch; ++k) step();
-    } catch (...) {
-        c->capturing = false;
-        cudaStreamEndCapture(c->st, &graph);
-        if (graph) cudaGraphDestroy(graph);
-        throw;
-    }
-    c->capturing = false;
-    CK(cudaStreamEndCapture(c->st, &graph));
-    CK(cudaGraphInstantiate(&exec, graph, 0));
-    size_t nodes = 0;
-    cudaGraphGetNodes(graph, nullptr, &nodes);
-    // every iteration pauses the state by itself at its iteration limit; the host
-    // bound below only guards against a state that never pauses
-    const long max_launches = max_iterations / batch + 4;
-    bool paused = false;
-    for (long l = 0; l < max_launches; ++l) {
-        CK(cudaGraphLaunch(exec, c->st));
-        c->launches += nodes;
-        CK(cudaMemcpyAsync(c->h_state, d, sizeof(S), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-        if (((S *)c->h_state)->pause) {
-            paused = true;
-            break;
-        }
-    }
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    CK(cudaGetLastError());
-    if (!paused) fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %ld iterations", max_iterations);
+    GatedLoop<S, Step>(c, d, step, batch).run(max_iterations);
 }
 
 // A = Q Q (+ shift) with Q Hermitian: the squared kinds with gamma5
@@ -977,7 +1008,7 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
     const double delta = sprec == PREC_D ? 0.0 : 0.1;
     OpEntry &eo = op;  // apply_schur takes gamma5 explicitly
     if (kind_has_clover(op.kind)) ensure_clover(c, op);
-    Vec bp(c, PREC_D, 1), rS(c, PREC_D, 1), rN(c, PREC_D, 1), te(c, PREC_D, 1), t1(c, PREC_D, 1);
+    Vec bp(c, PREC_D, 1), rN(c, PREC_D, 1), te(c, PREC_D, 1), t1(c, PREC_D, 1);
     Vec xs(c, sprec == PREC_H ? PREC_F : sprec, 1), rs(c, sprec == PREC_H ? PREC_F : sprec, 1);
     Vec ps(c, sprec, 1), tes(c, sprec, 1), tos(c, sprec, 1);
     const Spinor xo = x.parity(1);
@@ -990,9 +1021,7 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
     // true residuals: r_S = b' - S x, r_N = g5 S g5 r_S ; returns |r_S|^2, |r_N|^2
     auto true_res = [&](double &rrS, double &rrN) {
         apply_schur(c, eo, PREC_D, *t1, xo, *te, 0);
-        run_site(c, OpSubNorm<SpinorD, SpinorD, SpinorD>{(*bp).d(), (*t1).d(), (*rS).d(), c->d_scal}, 1);
-        copy(c, *t1, *rS);
-        gamma5_inplace(c, *t1);
+        run_site(c, OpSubNormG5<SpinorD, SpinorD>{(*bp).d(), (*t1).d(), c->d_scal}, 1);  // t1 = g5 r_S
         apply_schur(c, eo, PREC_D, *rN, *t1, *te, 1);
         run_site(c, OpNorm<SpinorD>{(*rN).d(), c->d_scal + 1}, 1);
         CK(cudaMemcpyAsync(c->h_scal, c->d_scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -1029,14 +1058,14 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
             else if (sprec == PREC_F) run_site(c, OpCGDirection<SpinorF, SpinorF>{(*ps).f(), (*rs).f(), S}, 1, gate);
             else run_site(c, OpCGDirection<SpinorH, SpinorF>{(*ps).h(), (*rs).f(), S}, 1, gate);
         };
+        GatedLoop<CGState, decltype(step)> loop(c, S, step, 8);
         for (int outer = 0; outer < 10000; ++outer) {
-            run_gated_state(c, S, step, 8, (long)max_steps - cg_host(c).iter + 8);
+            loop.run((long)max_steps - cg_host(c).iter + 8);
             CGState R = cg_host(c);
             iters = R.iter;
             if (R.failed) fail(c, LYM_ERR_NUMERIC, "CG produced a non-finite residual");
             // reliable update: x += x_sloppy, recompute the FP64 residuals
-            axpby(c, *xs, xo, C2(1.0), C2(1.0));
-            zero(c, *xs);
+            fold(c, *xs, xo);
             true_res(rrS, rrN);
             ++updates;
             if (rrS < eps_S) {
@@ -1048,7 +1077,6 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
                 // recursion converged but the true residual did not: tighten
                 eps_N = std::max(eps_N * 0.5 * eps_S / rrS, 1e-300);
             }
-            copy(c, *rs, *rN);
             CGState &W = cg_host(c);
             W = R;
             W.beta = rrN / R.rr_prev;
@@ -1059,10 +1087,7 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
             W.converged = 0;
             W.need_update = 0;
             push_state(c, sizeof(CGState));
-            // p = r + beta p with the true residual
-            if (sprec == PREC_D) run_site(c, OpCGDirection<SpinorD, SpinorD>{(*ps).d(), (*rs).d(), S}, 1);
-            else if (sprec == PREC_F) run_site(c, OpCGDirection<SpinorF, SpinorF>{(*ps).f(), (*rs).f(), S}, 1);
-            else run_site(c, OpCGDirection<SpinorH, SpinorF>{(*ps).h(), (*rs).f(), S}, 1);
+            cg_continue(c, *rs, *ps, *rN, W.beta);  // with the true residual
         }
     }
     schur_reconstruct(c, op, b, x);
@@ -1256,13 +1281,13 @@ int shift_cg_mixed(lym_context *c, OpEntry &op, int sprec, double sigma, const S
         else go((*ps).h(), (*aps).h(), (*xs).f(), (*rs).f());
     };
     int rc = LYM_NOT_CONVERGED;
+    GatedLoop<CGState, decltype(step)> loop(c, S, step, 8);
     for (int outer = 0; outer < 100000; ++outer) {
-        run_gated_state(c, S, step, 8, (long)(H.max_iter - cg_host(c).iter) + 8);
+        loop.run((long)(H.max_iter - cg_host(c).iter) + 8);
         CGState R = cg_host(c);
         iters = R.iter;
         if (R.failed) fail(c, LYM_ERR_NUMERIC, "shifted CG produced a non-finite residual");
-        axpby(c, *xs, xo, C2(1.0), C2(1.0));
-        zero(c, *xs);
+        fold(c, *xs, xo);
         rr_true = true_res();
         ++updates;
         if (rr_true < eps) {
@@ -1271,7 +1296,6 @@ int shift_cg_mixed(lym_context *c, OpEntry &op, int sprec, double sigma, const S
         }
         if (R.iter >= R.max_iter) break;
         if (R.converged) eps_rec = std::max(eps_rec * 0.5 * eps / rr_true, 1e-300);
-        copy(c, *rs, *r64);
         CGState &W = cg_host(c);
         W = R;
         W.beta = rr_true / R.rr_prev;
@@ -1282,9 +1306,7 @@ int shift_cg_mixed(lym_context *c, OpEntry &op, int sprec, double sigma, const S
         W.converged = 0;
         W.need_update = 0;
         push_state(c, sizeof(CGState));
-        if (sprec == PREC_D) run_site(c, OpCGDirection<SpinorD, SpinorD>{(*ps).d(), (*rs).d(), S}, 1);
-        else if (sprec == PREC_F) run_site(c, OpCGDirection<SpinorF, SpinorF>{(*ps).f(), (*rs).f(), S}, 1);
-        else run_site(c, OpCGDirection<SpinorH, SpinorF>{(*ps).h(), (*rs).f(), S}, 1);
+        cg_continue(c, *rs, *ps, *r64, W.beta);
     }
     return rc;
 }
@@ -1417,18 +1439,16 @@ int multishift_cg_mixed(lym_context *c, OpEntry &op, int rprec, int nshift, cons
     int iters = 0, updates = 0;
     std::vector<int> was_active(nshift, 1);
     if (!(bbo < eps || bbo == 0.0) && max_steps > 0) {
+        GatedLoop<MultishiftState, decltype(step)> loop(c, S, step, kMsWin);
         for (int outer = 0; outer < 100000; ++outer) {
-            nstep = 0;
-            run_gated_state(c, S, step, kMsWin, (long)max_steps - ((MultishiftState *)c->h_state)->iter + kMsWin);
+            loop.run((long)max_steps - ((MultishiftState *)c->h_state)->iter + kMsWin);
             MultishiftState R = *(MultishiftState *)c->h_state;
             iters = R.iter;
             if (R.failed) fail(c, LYM_ERR_NUMERIC, "multishift CG produced a non-finite residual");
             // fold the accumulators of every shift that ran since the last fold
             for (int i = 0; i < nshift; ++i) {
                 if (!was_active[i]) continue;
-                const Spinor a = **owned[(kMsWin + 1) + 2 * i];
-                axpby(c, a, xs[i].parity(1), C2(1.0), C2(1.0));
-                zero(c, a);
+                fold(c, **owned[(kMsWin + 1) + 2 * i], xs[i].parity(1));
                 was_active[i] = R.active[i] != 0;
             }
             const double rr = base_true_res();
@@ -2103,7 +2123,8 @@ public:
     }
     ~BlockEngine()
     {
-        if (exec) cudaGraphExecDestroy(exec);
+        for (auto e : exec)
+            if (e) cudaGraphExecDestroy(e);
         for (int j = 0; j < nb; ++j) delete slot[j].bp;
         dev_free(c, tables, kTableBytes);
     }
@@ -2181,7 +2202,7 @@ public:
         hs.last_update_its[j] = 0;
         if (algo == ALGO_BICGSTAB) {
             s.best_rr = rrS;
-            restart_bicg(j, rrS);
+            restart_bicg(j, rrS, *rS);
             hs.eps[j] = s.epsS;
         } else {
             axpby_views(c, (*rN).d(), rs.f().slot(j), C2(1.0), C2(0.0));
@@ -2269,9 +2290,13 @@ private:
     int gauge_id = -1;
     bool has_clover = false;
     BatchTile tile;
-    cudaGraphExec_t exec = nullptr;  // kGraphIters captured iterations, replayed
-    size_t nodes = 0;
-    static constexpr int kGraphIters = 8;
+    // captured iterations, replayed: kGraphIters of them, or kShortIters when the last pauses
+    // came sooner (the rest of a replay that pauses is no-op launches: at 14x10x12x22 with 8
+    // slots and FP16 storage the loop pauses every other iteration)
+    static constexpr int kGraphIters = 8, kShortIters = 2;
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    size_t nodes[2] = {0, 0};
+    double run_length = kGraphIters;  // iterations between pauses, averaged
     // the loop pauses once a kParkFraction-th of the busy slots waits for its update
     static constexpr int kParkFraction = LYM_BLOCK_PARK_FRACTION;
     // BiCGStab gives a source up after kMaxStalls reliable updates in a row that did not
@@ -2337,17 +2362,16 @@ private:
         CK(cudaStreamSynchronize(c->st));
         rrS = c->h_scal[0];
     }
-    // BiCGStab (re)start of slot j from the true residual in rS: r = rhat = p = rS
-    // what = S^+ rhat = g5 S g5 rhat (S is gamma5-hermitian), in FP64 into rN and the slot;
-    // returns <what, p> for p = rhat = rS
-    double2 shadow_image(int j)
+    // what = S^+ rhat = g5 S g5 rhat (S is gamma5-hermitian, rhat = res), in FP64 into rN and the slot;
+    // returns <what, p> for p = rhat = res
+    double2 shadow_image(int j, const Spinor &res)
     {
-        copy(c, *t1, *rS);
+        copy(c, *t1, res);
         gamma5_inplace(c, *t1);
         apply_schur(c, *slot[j].op, PREC_D, *rN, *t1, *te, 1);
         axpby_views(c, (*rN).d(), what->f().slot(j), C2(1.0), C2(0.0));
         copy(c, **what_c[j], *rN);
-        run_site(c, OpDot<SpinorD, SpinorD>{(*rN).d(), (*rS).d(), c->d_scal}, 1);
+        run_site(c, OpDot<SpinorD, SpinorD>{(*rN).d(), res.d(), c->d_scal}, 1);
         CK(cudaMemcpyAsync(c->h_scal, c->d_scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
         return make_double2(c->h_scal[0], c->h_scal[1]);
@@ -2360,76 +2384,101 @@ private:
         CK(cudaStreamSynchronize(c->st));
         return make_double2(c->h_scal[0], c->h_scal[1]);
     }
-    // BiCGStab (re)start of slot j from the true residual in rS: r = rhat = p = rS,
-    // rho = |rS|^2, what = S^+ rhat, alpha = rho / <what, p>
-    void restart_bicg(int j, double rrS)
+    // BiCGStab (re)start of slot j from the true residual: r = rhat = p = res,
+    // rho = |res|^2, what = S^+ rhat, alpha = rho / <what, p>
+    void restart_bicg(int j, double rrS, const Spinor &res)
     {
-        axpby_views(c, (*rS).d(), rs.f().slot(j), C2(1.0), C2(0.0));
-        axpby_views(c, (*rS).d(), rhat->f().slot(j), C2(1.0), C2(0.0));
-        copy(c, **rhat_c[j], *rS);
+        axpby_views(c, res.d(), rs.f().slot(j), C2(1.0), C2(0.0));
+        axpby_views(c, res.d(), rhat->f().slot(j), C2(1.0), C2(0.0));
+        copy(c, **rhat_c[j], res);
         set_direction(j, 0.0);
         hs.rho[j] = make_double2(rrS, 0.0);
-        hs.alpha[j] = cdiv(hs.rho[j], shadow_image(j));
+        hs.alpha[j] = cdiv(hs.rho[j], shadow_image(j, res));
         hs.rr[j] = hs.rr_max[j] = rrS;
         hs.restart[j] = 0;
         hs.active[j] = 1;
     }
-    void reliable_update_bicg(int j)
+    // The reliable updates of several parked slots together: their true residuals, then, for
+    // those that go on, the continuation of the recursion, with one host round trip each.
+    static constexpr int kUpdates = 8;  // at most; a residual vector each
+    void reliable_updates_bicg(const std::vector<int> &js)
     {
-        Slot &s = slot[j];
-        // x += the FP32 accumulator (unless a non-finite recursion (restart 2) drops it); the
-        // accumulator counts as zero from the next update pass on
-        if (hs.restart[j] != 2 && !hs.x_reset[j])
-            axpby_views(c, xs.f().slot(j), s.X.parity(1).d(), C2(1.0), C2(1.0));
-        hs.x_reset[j] = 1;
-        double rrS;
-        true_res_S(j, rrS);
-        ++s.updates;
-        hs.last_update_its[j] = hs.its[j];
-        if (rrS < 0.5 * s.best_rr) {
-            s.best_rr = rrS;
-            s.stalls = 0;
-        } else {
-            ++s.stalls;
+        const int n = (int)js.size();
+        std::vector<std::unique_ptr<Vec>> more;  // the first slot's residual is rS
+        std::vector<Spinor> res;
+        for (int i = 0; i < n; ++i) {
+            if (i > 0) more.emplace_back(new Vec(c, PREC_D, 1));
+            res.push_back(i > 0 ? **more.back() : *rS);
+            const int j = js[i];
+            Slot &s = slot[j];
+            // x += the FP32 accumulator (unless a non-finite recursion (restart 2) drops it); the
+            // accumulator counts as zero from the next update pass on
+            if (hs.restart[j] != 2 && !hs.x_reset[j])
+                axpby_views(c, xs.f().slot(j), s.X.parity(1).d(), C2(1.0), C2(1.0));
+            hs.x_reset[j] = 1;
+            apply_schur(c, *s.op, PREC_D, *t1, s.X.parity(1), *te, 0);
+            run_site(c, OpSubNorm<SpinorD, SpinorD, SpinorD>{(**s.bp).d(), (*t1).d(), res[i].d(), c->d_scal + i}, 1);
         }
-        if (hs.restart[j]) ++s.restarts;
-        if (!std::isfinite(rrS)) {
-            s.nonfinite = true;
-            finish(j);
-        } else if (rrS < s.epsS) {
-            s.converged = 1;
-            finish(j);
-        } else if (s.stalls >= kMaxStalls || s.restarts >= kMaxRestarts) {
-            s.gave_up = true;  // BiCGStab does not converge on this source
-            finish(j);
-        } else {
-            if (hs.converged[j]) hs.eps[j] = std::max(hs.eps[j] * 0.5 * s.epsS / rrS, 1e-300);
-            if (hs.restart[j]) {
-                restart_bicg(j, rrS);
+        CK(cudaMemcpyAsync(c->h_scal, c->d_scal, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        double rrs[kUpdates];
+        for (int i = 0; i < n; ++i) rrs[i] = c->h_scal[i];
+        std::vector<int> go;  // indices into js whose recursion continues
+        for (int i = 0; i < n; ++i) {
+            const int j = js[i];
+            Slot &s = slot[j];
+            const double rrS = rrs[i];
+            ++s.updates;
+            hs.last_update_its[j] = hs.its[j];
+            if (rrS < 0.5 * s.best_rr) {
+                s.best_rr = rrS;
+                s.stalls = 0;
             } else {
-                // the recursion goes on with the true residual in place of the recursive
-                // one: p += r_true - r_rec (p was formed from r_rec), r = r_true,
-                // rho = <rhat, r>, alpha = rho / <what, p>
-                if (sprec == PREC_F)
-                    run_site(c, OpBiContinue<SlotF, SlotF, SpinorD, SpinorF, SpinorF>{
-                                    rs.f().slot(j), ps.f().slot(j), (*rS).d(), (**rhat_c[j]).f(), (**what_c[j]).f(),
-                                    c->d_scal}, 1);
-                else
-                    run_site(c, OpBiContinue<SlotF, SlotH, SpinorD, SpinorF, SpinorF>{
-                                    rs.f().slot(j), ps.h().slot(j), (*rS).d(), (**rhat_c[j]).f(), (**what_c[j]).f(),
-                                    c->d_scal}, 1);
-                CK(cudaMemcpyAsync(c->h_scal, c->d_scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-                CK(cudaStreamSynchronize(c->st));
-                hs.rho[j] = make_double2(c->h_scal[0], c->h_scal[1]);
-                const double2 wp = make_double2(c->h_scal[2], c->h_scal[3]);
-                hs.alpha[j] = cdiv(hs.rho[j], wp);
-                hs.rr[j] = hs.rr_max[j] = rrS;
-                hs.active[j] = 1;
+                ++s.stalls;
             }
+            if (hs.restart[j]) ++s.restarts;
+            if (!std::isfinite(rrS)) {
+                s.nonfinite = true;
+                finish(j);
+            } else if (rrS < s.epsS) {
+                s.converged = 1;
+                finish(j);
+            } else if (s.stalls >= kMaxStalls || s.restarts >= kMaxRestarts) {
+                s.gave_up = true;  // BiCGStab does not converge on this source
+                finish(j);
+            } else {
+                if (hs.converged[j]) hs.eps[j] = std::max(hs.eps[j] * 0.5 * s.epsS / rrS, 1e-300);
+                if (hs.restart[j]) restart_bicg(j, rrS, res[i]);
+                else go.push_back(i);
+            }
+            hs.restart[j] = 0;
+            hs.converged[j] = 0;
+            hs.need_update[j] = 0;
         }
-        hs.restart[j] = 0;
-        hs.converged[j] = 0;
-        hs.need_update[j] = 0;
+        if (go.empty()) return;
+        // the recursion goes on with the true residual in place of the recursive one:
+        // p += r_true - r_rec (p was formed from r_rec), r = r_true, rho = <rhat, r>,
+        // alpha = rho / <what, p>
+        for (size_t k = 0; k < go.size(); ++k) {
+            const int j = js[go[k]];
+            const SpinorD rt = res[go[k]].d();
+            double *out = c->d_scal + 4 * k;
+            if (sprec == PREC_F)
+                run_site(c, OpBiContinue<SlotF, SlotF, SpinorD, SpinorF, SpinorF>{
+                                rs.f().slot(j), ps.f().slot(j), rt, (**rhat_c[j]).f(), (**what_c[j]).f(), out}, 1);
+            else
+                run_site(c, OpBiContinue<SlotF, SlotH, SpinorD, SpinorF, SpinorF>{
+                                rs.f().slot(j), ps.h().slot(j), rt, (**rhat_c[j]).f(), (**what_c[j]).f(), out}, 1);
+        }
+        CK(cudaMemcpyAsync(c->h_scal, c->d_scal, 4 * go.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        for (size_t k = 0; k < go.size(); ++k) {
+            const int j = js[go[k]];
+            hs.rho[j] = make_double2(c->h_scal[4 * k], c->h_scal[4 * k + 1]);
+            hs.alpha[j] = cdiv(hs.rho[j], make_double2(c->h_scal[4 * k + 2], c->h_scal[4 * k + 3]));
+            hs.rr[j] = hs.rr_max[j] = rrs[go[k]];
+            hs.active[j] = 1;
+        }
     }
     void set_direction(int j, double b)  // p_j = r_j + b p_j in the precision of p
     {
@@ -2441,54 +2490,66 @@ private:
     {
         const double t0 = wall();
         check_copy_waits(c, tile);
-        for (int j = 0; j < nb; ++j) {
-            Slot &s = slot[j];
-            if (!s.busy || s.finished || !hs.need_update[j]) continue;
-            reliable_update(j);
-            c->engine_stats[6] += 1;
-            if (!s.finished && hs.its[j] >= s.max_iter) finish(j);
+        std::vector<int> parked;
+        for (int j = 0; j < nb; ++j)
+            if (slot[j].busy && !slot[j].finished && hs.need_update[j]) parked.push_back(j);
+        // BiCGStab: as many together as there is scratch for (a residual each, 256 MiB in all)
+        const size_t most = std::max<size_t>(1, ((size_t)256 << 20) / spinor_bytes(c->g, PREC_D, 1));
+        const size_t group = algo == ALGO_BICGSTAB ? std::min<size_t>(kUpdates, most) : 1;
+        for (size_t i = 0; i < parked.size(); i += group) {
+            const std::vector<int> js(parked.begin() + i, parked.begin() + std::min(parked.size(), i + group));
+            if (algo == ALGO_BICGSTAB) reliable_updates_bicg(js);
+            else reliable_update(js[0]);
+            for (int j : js) {
+                c->engine_stats[6] += 1;
+                if (!slot[j].finished && hs.its[j] >= slot[j].max_iter) finish(j);
+            }
         }
         c->engine_stats[1] += wall() - t0;
     }
-    // captures kGraphIters iterations once, then replays them until the state pauses
+    void capture(BatchCGState *S, int which)
+    {
+        cudaGraph_t graph = nullptr;
+        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
+        c->capturing = true;
+        try {
+            for (int k = 0; k < (which ? kShortIters : kGraphIters); ++k) step(S);
+        } catch (...) {
+            c->capturing = false;
+            cudaStreamEndCapture(c->st, &graph);
+            if (graph) cudaGraphDestroy(graph);
+            throw;
+        }
+        c->capturing = false;
+        CK(cudaStreamEndCapture(c->st, &graph));
+        const cudaError_t e = cudaGraphInstantiate(&exec[which], graph, 0);
+        cudaGraphGetNodes(graph, nullptr, &nodes[which]);
+        cudaGraphDestroy(graph);
+        CK(e);
+    }
+    // replays captured iterations until the state pauses
     void run_loop(BatchCGState *S, long max_iterations)
     {
-        if (!exec) {
-            cudaGraph_t graph = nullptr;
-            CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
-            c->capturing = true;
-            try {
-                for (int k = 0; k < kGraphIters; ++k) step(S);
-            } catch (...) {
-                c->capturing = false;
-                cudaStreamEndCapture(c->st, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            c->capturing = false;
-            CK(cudaStreamEndCapture(c->st, &graph));
-            const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphGetNodes(graph, nullptr, &nodes);
-            cudaGraphDestroy(graph);
-            CK(e);
-        }
-        const long max_launches = max_iterations / kGraphIters + 4;
+        const int iter0 = hs.iter;
+        const int which = run_length < kGraphIters / 2 ? 1 : 0;
+        if (!exec[which]) capture(S, which);
+        const long max_launches = max_iterations / (which ? kShortIters : kGraphIters) + 4;
         for (long l = 0; l < max_launches; ++l) {
-            CK(cudaGraphLaunch(exec, c->st));
-            c->launches += nodes;
+            CK(cudaGraphLaunch(exec[which], c->st));
+            c->launches += nodes[which];
             c->engine_stats[4] += 1;
             CK(cudaMemcpyAsync(c->h_state, S, sizeof(BatchCGState), cudaMemcpyDeviceToHost, c->st));
             CK(cudaStreamSynchronize(c->st));
-            if (((BatchCGState *)c->h_state)->pause) return;
+            const BatchCGState &h = *(BatchCGState *)c->h_state;
+            if (h.pause) {
+                run_length = 0.5 * (run_length + (h.iter - iter0));
+                return;
+            }
         }
         fail(c, LYM_ERR_TIMEOUT, "block CG state did not pause within %ld iterations", max_iterations);
     }
-    void reliable_update(int j)
+    void reliable_update(int j)  // CG
     {
-        if (algo == ALGO_BICGSTAB) {
-            reliable_update_bicg(j);
-            return;
-        }
         Slot &s = slot[j];
         // x += the FP32 accumulator (unless a non-finite recursion (restart 2) drops it); the
         // accumulator counts as zero from the next update pass on

@@ -66,16 +66,18 @@ template <class SA, class SX> struct OpFoldClear {
     static constexpr int NRED = 0;
     SA a;
     SX x;
-    LYM_D void site(int p, int h, double *) const  // one component at a time
+    LYM_D void site(int p, int h, double *) const
     {
-        const SA ap = a.par(p);
-        const SX xp = x.par(p);
-#pragma unroll 4
+        cx<double> av[12], xv[12];
+        a.par(p).template load<double>(h, av);
+        x.par(p).template load<double>(h, xv);
+#pragma unroll
         for (int k = 0; k < 12; ++k) {
-            const cx<double> av = ap.get(k, h);
-            xp.put(k, h, xp.get(k, h) + av);
-            ap.put(k, h, cx<double>{0.0, 0.0});
+            xv[k] = xv[k] + av[k];
+            av[k] = cx<double>{0.0, 0.0};
         }
+        x.par(p).template store<double>(h, xv);
+        a.par(p).template store<double>(h, av);
     }
 };
 
@@ -215,6 +217,25 @@ template <class SX, class SY, class SZ> struct OpSubNorm {
         for (int k = 0; k < 12; ++k) u[k] = u[k] - v[k];
         acc[0] += norm2(u);
         z.par(p).template store<double>(h, u);
+    }
+    LYM_D void finalize(const double *t) const { out[0] = t[0]; }
+};
+
+// y = gamma5 (x - y),  out = |y|^2
+template <class SX, class SY> struct OpSubNormG5 {
+    static constexpr int NRED = 1;
+    SX x;
+    SY y;
+    double *out;
+    LYM_D void site(int p, int h, double *acc) const
+    {
+        cx<double> u[12], v[12];
+        x.par(p).template load<double>(h, u);
+        y.par(p).template load<double>(h, v);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) u[k] = k < 6 ? u[k] - v[k] : v[k] - u[k];
+        acc[0] += norm2(u);
+        y.par(p).template store<double>(h, u);
     }
     LYM_D void finalize(const double *t) const { out[0] = t[0]; }
 };
