@@ -118,21 +118,21 @@ __global__ void __launch_bounds__(128) store_gauge8_kernel(Geom g, GaugeDev U)
 // blocks of T = 1 + kappa csw gamma5 C with their inverses
 // (EvenOddImprovedDiracWilsonOperator.cpp:285-317), in FP64, FP32 and FP16.
 //
-// One block takes 32 half-sites of one parity.
+// clover_build_kernel: one block takes 32 half-sites of one parity.
 //   1. Warp pl forms plane pl of each site.  The leaves pair up under F = (Q - Q^+) / 8: a leaf
 //      that ends in U_mu(x)^+ contributes minus the leaf that starts with U_mu(x) would, so the
 //      two leaves at U_mu(x) are one product U_mu(x) (A - B) of staples, and those at U_mu(x-mu)
 //      another: 10 matrix products a plane instead of 12.  F is anti-Hermitian: 9 reals.
-//   2. The entries of T from the six planes, into shared memory.
-//   3. A thread inverts each of the 64 blocks by symmetric sweeps of its packed triangle, which
-//      need no pivoting while the block is positive definite (it is 1 plus the clover term, so
-//      it is but for a very large kappa c_sw).  A block with a pivot that is not positive is
-//      inverted by Gauss-Jordan with partial pivoting instead, a column per lane, six lanes a
-//      block, the pivot column through shared memory.
-//   4. All words of T and T^-1 in the three precisions, coalesced.
-// Bound by FP64 arithmetic in 1.  20^3 x 40: 532 us; all blocks by the pivoted inverse
-// 0.88 ms (its six dependent steps are latency); one thread per site with the matrices in
-// local memory, and a separate pass for the FP32 and FP16 words, 1.77 + 0.10 ms.
+//   2. The entries of T from the six planes, in shared memory.
+//   3. All words of T in the three precisions, coalesced.
+// Bound by FP64 arithmetic in 1.
+// clover_invert_kernel: a thread inverts one block by symmetric sweeps of its packed triangle,
+// in registers.  They need no pivoting while the block is positive definite (it is 1 plus the
+// clover term, so it is but for a very large kappa c_sw); a block with a pivot that is not
+// positive is inverted by Gauss-Jordan with partial pivoting in local memory.  HBM bound.
+// A launch of its own because its dependent steps want many warps, the products many registers:
+// in one launch they took 532 us at 20^3 x 40, against 439 + 77 us; one thread per site with all
+// matrices in local memory, and a separate pass for the FP32 and FP16 words, 1.77 + 0.10 ms.
 struct CloverArg {
     Geom g;
     double kc;
@@ -211,89 +211,65 @@ template <class Gauge> LYM_D void plane_of(const Geom &g, const Gauge &U, const 
     }
 }
 
-// In-place inverse of a 6 x 6 matrix, a column a lane (m: column j of the group's matrix): step
-// col divides by the largest entry at or below the diagonal of column col.  sc: 2 x 7 words of
-// the group.  On return m is column `dest` of the inverse.  False for a zero pivot.
-LYM_D bool invert6(Cd m[6], int j, int &dest, double2 (*sc)[7], bool live)
+// The inverse of the packed Hermitian block by Gauss-Jordan with partial pivoting, its Hermitian
+// part.  False for a zero pivot.
+__device__ __noinline__ bool invert_pivoted(double2 w[18])
 {
-    int pv[6];
-    bool ok = true;
-#pragma unroll
+    Cd m[6][6], inv[6][6];
+    for (int i = 0; i < 6; ++i)
+        for (int j = 0; j < 6; ++j) {
+            inv[i][j] = Cd{i == j ? 1.0 : 0.0, 0.0};
+            if (i == j) {
+                m[i][j] = Cd{(i & 1) ? w[i >> 1].y : w[i >> 1].x, 0.0};
+            } else {
+                const double2 z = w[3 + (i > j ? tri_index(i, j) : tri_index(j, i))];
+                m[i][j] = Cd{z.x, i > j ? z.y : -z.y};
+            }
+        }
     for (int col = 0; col < 6; ++col) {
-        double2 *s = sc[col & 1];
-        if (live && j == col) {
-            int piv = col;
-            double best = fabs(m[col].re) + fabs(m[col].im);
-            Cd d = m[col];
-#pragma unroll
-            for (int r = col + 1; r < 6; ++r) {
-                const double a = fabs(m[r].re) + fabs(m[r].im);
-                if (a > best) {
-                    best = a;
-                    piv = r;
-                    d = m[r];
-                }
+        int piv = col;
+        double best = fabs(m[col][col].re) + fabs(m[col][col].im);
+        for (int r = col + 1; r < 6; ++r) {
+            const double a = fabs(m[r][col].re) + fabs(m[r][col].im);
+            if (a > best) {
+                best = a;
+                piv = r;
             }
-            if (best == 0.0) ok = false;
-            const double dn = d.re * d.re + d.im * d.im;
-#pragma unroll
-            for (int r = 0; r < 6; ++r) {
-                const Cd v = r == piv ? m[col] : m[r];
-                if (r != col) s[r] = make_double2(v.re, v.im);
-            }
-            s[col] = make_double2(d.re / dn, -d.im / dn);
-            s[6] = make_double2((double)piv, 0.0);
         }
-        __syncwarp();
-        const int piv = pv[col] = live ? (int)s[6].x : col;
-        if (piv != col) {
-            const Cd t = m[col];
-#pragma unroll
-            for (int r = col + 1; r < 6; ++r)
-                if (r == piv) {
-                    m[col] = m[r];
-                    m[r] = t;
-                }
+        if (best == 0.0) return false;
+        const Cd d = m[piv][col];
+        const double dn = d.re * d.re + d.im * d.im;
+        const Cd rd{d.re / dn, -d.im / dn};
+        for (int j = 0; j < 6; ++j) {
+            const Cd a = m[piv][j], b = inv[piv][j];
+            m[piv][j] = m[col][j];
+            inv[piv][j] = inv[col][j];
+            m[col][j] = a * rd;
+            inv[col][j] = b * rd;
         }
-        const Cd rd{s[col].x, s[col].y};
-        const bool own = j == col;
-        const Cd t = own ? rd : m[col] * rd;
-        m[col] = t;
-#pragma unroll
         for (int r = 0; r < 6; ++r) {
             if (r == col) continue;
-            const Cd f{s[r].x, s[r].y};
-            const Cd base = own ? Cd{0.0, 0.0} : m[r];
-            m[r] = base - f * t;
+            const Cd f = m[r][col];
+            for (int j = 0; j < 6; ++j) {
+                m[r][j] = m[r][j] - f * m[col][j];
+                inv[r][j] = inv[r][j] - f * inv[col][j];
+            }
         }
     }
-    dest = j;
-#pragma unroll
-    for (int col = 5; col >= 0; --col) {
-        if (dest == col) dest = pv[col];
-        else if (dest == pv[col]) dest = col;
-    }
-    return ok;
+    for (int k = 0; k < 3; ++k) w[k] = make_double2(inv[2 * k][2 * k].re, inv[2 * k + 1][2 * k + 1].re);
+    for (int i = 1; i < 6; ++i)
+        for (int j = 0; j < i; ++j) {
+            const Cd z = 0.5 * (inv[i][j] + conj(inv[j][i]));
+            w[3 + tri_index(i, j)] = make_double2(z.re, z.im);
+        }
+    return true;
 }
 
-// Inverse of the Hermitian block in t (words of site `lane`) into o by sweeps: with D = a_kk,
-// a_ij -= a_ik conj(a_jk) / D, a_ik /= D, a_kk = -1 / D for k = 0..5 leaves minus the inverse.
-// False, and o unwritten, once a pivot is not positive.
-LYM_D bool invert_sweep(const double2 (*t)[kPad], double2 (*o)[kPad], int lane)
+// The inverse of the packed Hermitian block by sweeps: with D = a_kk, a_ij -= a_ik conj(a_jk) / D,
+// a_ik /= D, a_kk = -1 / D for k = 0..5 leaves minus the inverse.  False once a pivot is not
+// positive (d, l then hold no inverse).
+LYM_D bool invert_sweep(double d[6], Cd l[15])
 {
-    double d[6];
-    Cd l[15];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double2 w = t[k][lane];
-        d[2 * k] = w.x;
-        d[2 * k + 1] = w.y;
-    }
-#pragma unroll
-    for (int k = 0; k < 15; ++k) {
-        const double2 w = t[3 + k][lane];
-        l[k] = Cd{w.x, w.y};
-    }
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -320,22 +296,65 @@ LYM_D bool invert_sweep(const double2 (*t)[kPad], double2 (*o)[kPad], int lane)
         }
         d[k] = -r;
     }
-    if (!ok) return false;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) o[k][lane] = make_double2(-d[2 * k], -d[2 * k + 1]);
+    for (int k = 0; k < 6; ++k) d[k] = -d[k];
 #pragma unroll
-    for (int k = 0; k < 15; ++k) o[3 + k][lane] = make_double2(-l[k].re, -l[k].im);
-    return true;
+    for (int k = 0; k < 15; ++k) l[k] = -l[k];
+    return ok;
+}
+
+// word pair k of block pb = 2 parity + chirality of half-site h, in the three precisions
+LYM_D void store_words(double2 *d, float4 *f, uint2 *hf, size_t stride, int pb, int k, int h, double2 x, double2 y)
+{
+    const size_t at = (size_t)pb * 9 + k;
+    d[at * 2 * stride + h] = x;
+    d[(at * 2 + 1) * stride + h] = y;
+    f[at * stride + h] = floats(x, y);
+    hf[at * stride + h] = halves(x, y);
+}
+
+__global__ void __launch_bounds__(128) clover_invert_kernel(CloverArg a)
+{
+    const int h = blockIdx.x * blockDim.x + threadIdx.x, pb = blockIdx.y;
+    if (h >= a.g.Vh) return;
+    const size_t st = a.g.stride;
+    const double2 *t = a.T + (size_t)pb * 18 * st + h;
+    double d[6];
+    Cd l[15];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double2 w = __ldg(t + k * st);
+        d[2 * k] = w.x;
+        d[2 * k + 1] = w.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 15; ++k) {
+        const double2 w = __ldg(t + (3 + k) * st);
+        l[k] = Cd{w.x, w.y};
+    }
+    if (!invert_sweep(d, l)) {
+        double2 w[18];
+        for (int k = 0; k < 18; ++k) w[k] = __ldg(t + k * st);
+        if (!invert_pivoted(w)) atomicOr(a.err, 4);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            d[2 * k] = w[k].x;
+            d[2 * k + 1] = w[k].y;
+        }
+#pragma unroll
+        for (int k = 0; k < 15; ++k) l[k] = Cd{w[3 + k].x, w[3 + k].y};
+    }
+    auto word = [&](int k) {
+        return k < 3 ? make_double2(d[2 * k], d[2 * k + 1]) : make_double2(l[k - 3].re, l[k - 3].im);
+    };
+#pragma unroll
+    for (int k = 0; k < 9; ++k) store_words(a.Ti, a.Tif, a.Tih, st, pb, k, h, word(2 * k), word(2 * k + 1));
 }
 
 template <class Gauge> __global__ void __launch_bounds__(kCloverThreads, 2) clover_build_kernel(CloverArg a, Gauge U)
 {
-    // words of T and of T^-1, [chirality][18][site]; the planes use the space of T^-1 before it
-    __shared__ __align__(16) double2 sT[2][18][kPad], sI[2][18][kPad];
-    __shared__ __align__(16) double2 sc[30][2][7];
-    __shared__ unsigned pivoted[2];
-    static_assert(sizeof(sI) >= sizeof(double) * 6 * 9 * kPad, "planes");
-    double(*f)[9][kPad] = reinterpret_cast<double(*)[9][kPad]>(&sI[0][0][0]);
+    __shared__ __align__(16) double2 sT[2][18][kPad];  // words of T, [chirality][18][site]
+    __shared__ double f[6][9][kPad];                   // planes
     const Geom &g = a.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = blockIdx.y, h = blockIdx.x * kSites + lane;
@@ -396,64 +415,10 @@ template <class Gauge> __global__ void __launch_bounds__(kCloverThreads, 2) clov
         }
     }
     __syncthreads();
-    if (warp < 2) {
-        const unsigned left = __ballot_sync(0xffffffffu, !invert_sweep(sT[warp], sI[warp], lane));
-        if (lane == 0) pivoted[warp] = left;
-    }
-    __syncthreads();
-    // the blocks that need pivoting, five a warp at a time
-    const int grp = lane / 6, j = lane % 6;
-    for (int m0 = 0; (pivoted[0] | pivoted[1]) && m0 < 2 * kSites; m0 += 30) {
-        const int m = m0 + warp * 5 + grp;
-        const int b = min(m, 2 * kSites - 1) / kSites, site = m % kSites;
-        const bool live = lane < 30 && m < 2 * kSites && (pivoted[b] >> site & 1u);
-        Cd v[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            if (i == j) {
-                const double2 w = sT[b][i >> 1][site];
-                v[i] = Cd{(i & 1) ? w.y : w.x, 0.0};
-            } else {
-                const double2 w = sT[b][3 + (i > j ? tri_index(i, j) : tri_index(j, i))][site];
-                v[i] = Cd{w.x, i > j ? w.y : -w.y};
-            }
-        }
-        int q;
-        double2(*s)[7] = sc[warp * 5 + min(grp, 4)];
-        if (!invert6(v, j, q, s, live) && blockIdx.x * kSites + site < g.Vh) atomicOr(a.err, 4);
-        // the Hermitian part, lower triangle: column q writes the entries below its diagonal, then
-        // the columns right of them add their conjugates
-        if (live) {
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                if (i == q) (&sI[b][i >> 1][site].x)[i & 1] = v[i].re;
-                else if (i > q) sI[b][3 + tri_index(i, q)][site] = make_double2(v[i].re, v[i].im);
-            }
-        }
-        __syncwarp();
-        if (live) {
-#pragma unroll
-            for (int i = 0; i < 6; ++i)
-                if (i < q) {
-                    double2 &w = sI[b][3 + tri_index(q, i)][site];
-                    w = make_double2(0.5 * (w.x + v[i].re), 0.5 * (w.y - v[i].im));
-                }
-        }
-        __syncwarp();
-    }
-    __syncthreads();
     if (!in) return;
-    // word pair k of one chirality of T or T^-1 in the three precisions
-    for (int it = warp; it < 36; it += 6) {
-        const int inv = it / 18, b = it / 9 % 2, k = it % 9;
-        const double2 x = inv ? sI[b][2 * k][lane] : sT[b][2 * k][lane];
-        const double2 y = inv ? sI[b][2 * k + 1][lane] : sT[b][2 * k + 1][lane];
-        const size_t st = g.stride, at = (size_t)(p * 2 + b) * 9 + k;
-        double2 *d = (inv ? a.Ti : a.T) + at * 2 * st + h;
-        d[0] = x;
-        d[st] = y;
-        (inv ? a.Tif : a.Tf)[at * st + h] = floats(x, y);
-        (inv ? a.Tih : a.Th)[at * st + h] = halves(x, y);
+    for (int it = warp; it < 18; it += 6) {
+        const int b = it / 9, k = it % 9;
+        store_words(a.T, a.Tf, a.Th, g.stride, 2 * p + b, k, h, sT[b][2 * k][lane], sT[b][2 * k + 1][lane]);
     }
 }
 
@@ -489,6 +454,7 @@ void launch_clover_build(const Geom &g, const GaugeDev &U, double kc, CloverDev 
         clover_build_kernel<<<grid, kCloverThreads, 0, st>>>(a, GaugeD18{(const double2 *)U.d64, g.stride});
     else
         clover_build_kernel<<<grid, kCloverThreads, 0, st>>>(a, GaugeD9{(const double *)U.d64, g.stride});
+    clover_invert_kernel<<<dim3((g.Vh + 127) / 128, 4), 128, 0, st>>>(a);
 }
 
 }  // namespace lym
