@@ -98,8 +98,10 @@ __global__ void __launch_bounds__(kMeasThreads) slice_partial_kernel(const doubl
     for (int t0 = 0; t0 < Lt; t0 += width) {
         const int t = t0 + tl;
         double s = 0.0;
-        if (g < groups && t < Lt)
-            for (int l = l0 + g; l < l1; l += groups) s += v[(size_t)l * Lt + t];
+        if (g < groups && t < Lt) {
+#pragma unroll 8
+            for (int l = l0 + g; l < l1; l += groups) s += __ldg(v + (size_t)l * Lt + t);
+        }
         red[threadIdx.x] = s;
         __syncthreads();
         if (threadIdx.x < width && t < Lt) {
@@ -199,7 +201,7 @@ void launch_z2_noise(const Geom &g, double *out, unsigned long long seed, unsign
     z2_noise_kernel<<<grid, kMeasThreads, 0, st>>>((double2 *)out, n, seed, stream);
 }
 
-constexpr int kSliceChunks = 64;
+constexpr int kSliceChunks = 128;
 
 size_t meson_scratch_bytes(const Geom &g)
 {
