@@ -670,6 +670,11 @@ void push_state(lym_context *c, size_t bytes)
 // state pauses.  `batch` iterations are captured once into a CUDA graph and replayed; the host
 // reads the state once per replay.  A solve that pauses for reliable updates keeps its loop and
 // replays the same graph (capturing and instantiating it again took 0.3-0.4 ms each time).
+inline bool state_paused(const CGState &s) { return s.pause != 0; }
+inline bool state_paused(const BiCGState &s) { return s.pause != 0; }
+inline bool state_paused(const MMMRState &s) { return s.pause != 0; }
+inline bool state_paused(const MultishiftState &s) { return s.pause != 0 || s.stop != 0; }
+
 template <class S, class Step> class GatedLoop {
 public:
     GatedLoop(lym_context *ctx, S *state, Step st, int batch_) : c(ctx), d(state), step(st), batch(batch_) {}
@@ -691,7 +696,7 @@ public:
             c->launches += nodes;
             CK(cudaMemcpyAsync(c->h_state, d, sizeof(S), cudaMemcpyDeviceToHost, c->st));
             CK(cudaStreamSynchronize(c->st));
-            if (((S *)c->h_state)->pause) {
+            if (state_paused(*(S *)c->h_state)) {
                 CK(cudaGetLastError());
                 return;
             }
@@ -1197,14 +1202,14 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
         if (square) {
             for (int mode : {CG_NORM, CG_UPDATE}) {
                 const DslashParams P =
-                    square_half_params(c, op, *ap, mode == CG_NORM ? pb : *ap, pb, half, s0, &S->pause);
+                    square_half_params(c, op, *ap, mode == CG_NORM ? pb : *ap, pb, half, s0, &S->stop);
                 launch_split_ms(P, mode, pb, views.ring, S, c->spartials, c->counter, c->st);
                 count(c, 1);
             }
         } else {
-            op_apply(c, op, PREC_D, *ap, pb, &pb, C2(s0), &S->pause);
-            run_site(c, OpMsAlpha<SpinorD, SpinorD>{pb.d(), (*ap).d(), S}, 2, gate);
-            run_site(c, OpMsResidualRing<SpinorD, SpinorD>{views.ring, (*ap).d(), S}, 2, gate);
+            op_apply(c, op, PREC_D, *ap, pb, &pb, C2(s0), &S->stop);
+            run_site(c, OpMsAlpha<SpinorD, SpinorD>{pb.d(), (*ap).d(), S}, 2, Gate{&S->stop, nullptr, &S->pause});
+            run_site(c, OpMsResidualRing<SpinorD, SpinorD>{views.ring, (*ap).d(), S}, 2, Gate{&S->stop, nullptr});
         }
         run_site(c, OpMsBaseDirection<SpinorD, SpinorD>{views.ring, pb.d(), S}, 2, gate);
         if (++nstep % kMsWin == 0) views.template flush<double2, double>(S, nshift, 2 * 12 * c->g.stride);
@@ -1423,9 +1428,9 @@ int multishift_cg_mixed(lym_context *c, OpEntry &op, int rprec, int nshift, cons
     const Spinor xb = xs[base].parity(1);
     int nstep = 0;
     auto step = [&]() {
-        schur_square_shift(c, op, PREC_F, *ap, pb, *tos, *tes, s0, &S->pause);
-        run_site(c, OpMsAlpha<SpinorF, SpinorF>{pb.f(), (*ap).f(), S}, 1, gate);
-        run_site(c, OpMsResidualRing<SpinorF, SpinorF>{views.ring, (*ap).f(), S}, 1, gate);
+        schur_square_shift(c, op, PREC_F, *ap, pb, *tos, *tes, s0, &S->stop);
+        run_site(c, OpMsAlpha<SpinorF, SpinorF>{pb.f(), (*ap).f(), S}, 1, Gate{&S->stop, nullptr, &S->pause});
+        run_site(c, OpMsResidualRing<SpinorF, SpinorF>{views.ring, (*ap).f(), S}, 1, Gate{&S->stop, nullptr});
         run_site(c, OpMsBaseDirection<SpinorF, SpinorF>{views.ring, pb.f(), S}, 1, gate);
         if (++nstep % kMsWin == 0) views.template flush<float4, float>(S, nshift, 6 * c->g.stride);
     };

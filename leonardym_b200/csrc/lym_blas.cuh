@@ -49,11 +49,27 @@ LYM_D void block_sum(double v[N], double *smem /* [kBlasThreads/32][N] */)
     __syncthreads();
 }
 
-// Skip gates: a kernel does nothing when *skip_if != 0 or (run_if && *run_if == 0).
+// Skip gates: a kernel does nothing when *skip_if != 0 or (run_if && *run_if == 0), except that
+// it then sets *on_skip.
 struct Gate {
     const int *skip_if;
     const int *run_if;
-    LYM_D bool closed() const { return (skip_if && *skip_if) || (run_if && !*run_if); }
+    int *on_skip = nullptr;
+    LYM_D bool closed() const
+    {
+        const bool shut = (skip_if && *skip_if) || (run_if && !*run_if);
+        if (shut && on_skip && blockIdx.x == 0 && threadIdx.x == 0) *on_skip = 1;
+        return shut;
+    }
+};
+
+// Op::finalize runs in one thread, or in every thread of the last block where the functor says
+// so (kParallelFinalize)
+template <class Op, class = void> struct ParallelFinalize {
+    static constexpr bool value = false;
+};
+template <class Op> struct ParallelFinalize<Op, decltype((void)Op::kParallelFinalize)> {
+    static constexpr bool value = Op::kParallelFinalize;
 };
 
 template <class Op>
@@ -88,10 +104,16 @@ __global__ void __launch_bounds__(kBlasThreads) site_kernel(Op op, int vh, int n
 #pragma unroll
                 for (int k = 0; k < Op::NRED; ++k) tot[k] += ((volatile double *)rb.partials)[b * kMaxRed + k];
             block_sum<Op::NRED>(tot, smem);
-            if (threadIdx.x == 0) {
+            if constexpr (ParallelFinalize<Op>::value) {
+                if (threadIdx.x == 0)
+#pragma unroll
+                    for (int k = 0; k < Op::NRED; ++k) smem[k] = tot[k];
+                __syncthreads();
+                op.finalize(smem);
+            } else if (threadIdx.x == 0) {
                 op.finalize(tot);
-                *rb.counter = 0u;
             }
+            if (threadIdx.x == 0) *rb.counter = 0u;
         }
     } else {
         (void)rb;

@@ -549,25 +549,31 @@ struct MultishiftState {
 //   zeta_{k+1} = zeta_k zeta_{k-1} a_{k-1} /
 //                (zeta_{k-1} a_{k-1} (1 + sigma a_k) + a_k b_k (zeta_{k-1} - zeta_k))
 //   a^sigma_k  = a_k zeta_{k+1} / zeta_k.
+// The scalar steps below are called by every thread of the last block, a shift a thread: one
+// thread walking the shifts in global memory took 5-8 us a step with 8 shifts.
 LYM_D void ms_alpha_step(MultishiftState *s, double pap)
 {
-    const double a = s->rr / pap;
-    const double am1 = s->alpha;
-    for (int i = 0; i < s->nshift; ++i) {
-        if (s->active[i] == 2) s->active[i] = 0;  // converged at the previous step
-        if (!s->active[i]) continue;
+    const double a = s->rr / pap, am1 = s->alpha, beta = s->beta;
+    for (int i = threadIdx.x; i < s->nshift; i += blockDim.x) {
+        const int act = s->active[i];
+        if (act == 2) s->active[i] = 0;  // converged at the previous step
+        if (act != 1) continue;
         const double z = s->zeta[i], zp = s->zeta_prev[i];
-        const double den = zp * am1 * (1.0 + s->sigma[i] * a) + a * s->beta * (zp - z);
+        const double den = zp * am1 * (1.0 + s->sigma[i] * a) + a * beta * (zp - z);
         const double zn = (z * zp * am1) / den;
         s->alpha_s[i] = a * zn / z;
         s->zeta_prev[i] = z;
         s->zeta[i] = zn;
     }
-    s->alpha_prev = am1;
-    s->alpha = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s->alpha_prev = am1;
+        s->alpha = a;
+    }
 }
 template <class SP, class SAp> struct OpMsAlpha {
     static constexpr int NRED = 2;
+    static constexpr bool kParallelFinalize = true;
     SP p;
     SAp ap;
     MultishiftState *s;
@@ -581,74 +587,68 @@ template <class SP, class SAp> struct OpMsAlpha {
     LYM_D void finalize(const double *t) const { ms_alpha_step(s, t[0]); }
 };
 
-// After r_{k+1}: beta, the shifted betas, per-shift convergence, reliable-update and stop
-// flags.  False when the residual is not finite (the state is paused).
-LYM_D bool ms_residual_step(MultishiftState *s, double rr_new)
+// After r_{k+1}: beta, the shifted betas, per-shift convergence, reliable-update and stop flags;
+// then the shifted updates of the step, x_i += alpha_i p_i (a converged shift's last one included)
+// and p_i = zeta_i R_m + beta_i p_i (not after a step that asks for a reliable update), applied
+// to the coefficients of x_i and p_i, R_m = r_{k+1}.  A residual that is not finite pauses the
+// state before the updates.
+LYM_D void ms_residual_step(MultishiftState *s, double rr_new)
 {
-    s->iter += 1;
-    s->beta = rr_new / s->rr;
-    s->rr_prev = s->rr;
-    s->rr = rr_new;
-    if (rr_new > s->rr_max) s->rr_max = rr_new;
-    if (!(rr_new == rr_new)) {  // NaN: stop before the update
-        s->failed = 1;
-        s->stop = 1;
-        s->pause = 1;
-        return false;
-    }
+    const double rr = s->rr, beta = rr_new / rr, eps = s->eps, delta2 = s->delta2;
+    const double rr_max = fmax(s->rr_max, rr_new);
+    const int iter = s->iter + 1, m = s->win, base = s->base;
+    const bool bad = !(rr_new == rr_new);
     int any = 0;
-    for (int i = 0; i < s->nshift; ++i) {
-        if (!s->active[i]) continue;
-        // residual of shift i after this step: zeta_{k+1} r_{k+1}
-        const double zr = s->zeta[i] * s->zeta[i] * rr_new;
-        s->beta_s[i] = s->beta * (s->zeta[i] / s->zeta_prev[i]) * (s->zeta[i] / s->zeta_prev[i]);
-        // converged: this step's x update still runs, then the shift is frozen.
-        // The base system (sigma 0, index base) keeps its direction p, which
-        // drives the recursion of all the others.
-        if (zr < s->eps && i != s->base) s->active[i] = 2;
-        else if (zr >= s->eps) any = 1;
-    }
-    // the updates of this step still run; OpMsBaseDirection turns stop into pause
-    if (!any) {
-        s->converged = 1;
-        s->stop = 1;
-        s->need_update = s->delta2 > 0.0;
-    } else if (s->delta2 > 0.0 && rr_new < s->delta2 * s->rr_max) {
-        s->need_update = 1;
-        s->stop = 1;
-    } else if (s->iter >= s->max_iter) {
-        s->stop = 1;
-    }
-    return true;
-}
-
-// The shifted updates of a step, x_i += alpha_i p_i (a converged shift's last one included) and
-// p_i = zeta_i R_m + beta_i p_i (not after a step that asks for a reliable update), applied to
-// the coefficients of x_i and p_i, R_m = r_{k+1}.
-LYM_D void ms_window_step(MultishiftState *s)
-{
-    const int m = s->win;
-    const bool dir = !s->need_update;
-    for (int i = 0; i < s->nshift; ++i) {
-        const int act = s->active[i];
-        if (!act) continue;
-        const double a = s->alpha_s[i];
-        for (int j = 0; j <= m; ++j) s->cx[i][j] += a * s->cp[i][j];
-        s->xupd[i] = 1;
-        if (act == 1 && dir) {
-            const double b = s->beta_s[i];
-            for (int j = 0; j <= m; ++j) s->cp[i][j] *= b;
-            s->cp[i][m + 1] = s->zeta[i];
-            s->pupd[i] = 1;
+    if (!bad)
+        for (int i = threadIdx.x; i < s->nshift; i += blockDim.x) {
+            if (!s->active[i]) continue;
+            // residual of shift i after this step: zeta_{k+1} r_{k+1}
+            const double z = s->zeta[i], f = z / s->zeta_prev[i], zr = z * z * rr_new;
+            s->beta_s[i] = beta * f * f;
+            // converged: this step's x update still runs, then the shift is frozen.
+            // The base system (sigma 0, index base) keeps its direction p, which
+            // drives the recursion of all the others.
+            if (zr < eps && i != base) s->active[i] = 2;
+            else if (zr >= eps) any = 1;
         }
+    any = __syncthreads_or(any);
+    const bool update = !bad && (any ? delta2 > 0.0 && rr_new < delta2 * rr_max : delta2 > 0.0);
+    if (!bad)
+        for (int i = threadIdx.x; i < s->nshift; i += blockDim.x) {
+            const int act = s->active[i];
+            if (!act) continue;
+            const double a = s->alpha_s[i];
+            for (int j = 0; j <= m; ++j) s->cx[i][j] += a * s->cp[i][j];
+            s->xupd[i] = 1;
+            if (act == 1 && !update) {
+                const double b = s->beta_s[i];
+                for (int j = 0; j <= m; ++j) s->cp[i][j] *= b;
+                s->cp[i][m + 1] = s->zeta[i];
+                s->pupd[i] = 1;
+            }
+        }
+    if (threadIdx.x != 0) return;
+    s->iter = iter;
+    s->beta = beta;
+    s->rr_prev = rr;
+    s->rr = rr_new;
+    s->rr_max = rr_max;
+    if (bad) {
+        s->failed = s->stop = s->pause = 1;
+        return;
     }
     s->win = m + 1;
+    // the updates of this step still run; the next step turns stop into pause
+    if (!any) s->converged = 1;
+    if (update) s->need_update = 1;
+    if (!any || update || iter >= s->max_iter) s->stop = 1;
 }
 
 // r_{k+1} = r_k - alpha Ap with the residuals in a ring of kMsWin + 1 slots (r_k in slot
 // k mod (kMsWin + 1)), |r_{k+1}|^2, then the step's scalars and window coefficients.
 template <class SR, class SAp> struct OpMsResidualRing {
     static constexpr int NRED = 1;
+    static constexpr bool kParallelFinalize = true;
     const SR *ring;
     SAp ap;
     MultishiftState *s;
@@ -665,16 +665,15 @@ template <class SR, class SAp> struct OpMsResidualRing {
         acc[0] += norm2(rv);
         rout.par(q).template store<double>(h, rv);
     }
-    LYM_D void finalize(const double *t) const
-    {
-        if (ms_residual_step(s, t[0])) ms_window_step(s);
-    }
+    LYM_D void finalize(const double *t) const { ms_residual_step(s, t[0]); }
 };
 
 // the base system's direction, materialised every step for the operator: p = r_{k+1} + beta p
-// (not after a step that asks for a reliable update: the host rebuilds it from the true residual)
+// (not after a step that asks for a reliable update: the host rebuilds it from the true residual).
+// Gated on `pause`, which the next step's product with <p, A p> sets when it finds the state
+// stopped: this launch runs once after the last residual without a grid-wide last block of its own.
 template <class SR, class SP> struct OpMsBaseDirection {
-    static constexpr int NRED = 1;  // no sum; finalize ends the step
+    static constexpr int NRED = 0;
     const SR *ring;
     SP p;
     MultishiftState *s;
@@ -688,10 +687,6 @@ template <class SR, class SP> struct OpMsBaseDirection {
 #pragma unroll
         for (int c = 0; c < 12; ++c) pv[c] = rv[c] + b * pv[c];
         p.par(q).template store<double>(h, pv);
-    }
-    LYM_D void finalize(const double *) const
-    {
-        if (s->stop) s->pause = 1;
     }
 };
 

@@ -1,21 +1,5 @@
-// The FP64 Wilson-clover stencil: four threads per site.
-//
-// Thread (k, d) of a site, k, d = 0, 1, takes the half spinor h_k (lym_dslash.cuh) of the
-// directions mu = 2 d, 2 d + 1: it accumulates upper spin k and the lower spin its two
-// directions pair with k (3 - k for d = 0, 2 + k for d = 1), 6 complex numbers instead of the 12
-// of a thread per site, then the lanes of the site add up their parts by shuffles:
-//   spin k      = up(k, 0) + up(k, 1),   spin 2 + k = low(k, 1) + low(1 - k, 0),
-// after which thread (k, d) holds spin 2 d + k and applies its three rows of the clover block of
-// chirality d.  A warp is 8 sites, lane = site + 8 d + 16 k, so that link loads of k = 0, 1 fall
-// on one address and spinor loads on contiguous 128-byte pieces.
-//
-// Why four threads: in FP64 the whole-site form needs 142-180 registers (3 blocks of 128 per SM,
-// 12 warps), too few loads in flight for HBM, and on small lattices too few warps and one long
-// dependent chain per site.  24^3 x 48: both parities in one launch 247 us against
-// 2 x 144 us, one parity 141-149 against 144 us (T^-1 half 130 against 137); 16^3 x 32 adjoint 25
-// and 21 against 26 and 28 us; 8^4 both parities 4.6 against 2 x 6.6 us.  Latency bound (L1 misses;
-// 4.35 TB/s of HBM, 16 warps per SM): 3, 5 or 6 blocks per SM give 253, 270, 312 us there, blocks
-// of 256 or 512 threads 252, 280 us.
+// Launches of the FP64 stencil (lym_split.cuh): operator applications, Schur halves, and the
+// products of CG and multishift iterations with their vector work fused.
 //
 // In "both" mode a launch covers both parities, the same half-sites of either in one block, so
 // that a link read forward by one parity and backward by the other comes from DRAM once; it can
@@ -24,15 +8,13 @@
 #include "lym_dslash.cuh"
 #include "lym_internal.h"
 #include "lym_solver_ops.cuh"
+#include "lym_split.cuh"
 
 namespace lym {
 
 namespace {
 
-typedef cx<double> C;
-
-constexpr int kSplitThreads = 128;
-constexpr int kSplitSites = kSplitThreads / 4;
+using namespace split;
 
 enum SplitEpi : int {
     SPLIT_SCALE = EPI_SCALE,
@@ -56,6 +38,7 @@ template <class GaugeT> struct SplitArg {
     int gamma5, has_v2;
     double a, b, alpha_re, alpha_im;
     const int *skip_if;
+    int *on_skip;            // SPLIT_CG_NORM: set when the launch is skipped
     double2 *aos_out;        // AOS: the full result
     const double2 *aos_v2;   // AOS: the added vector, or null
     int even_identity;       // both mode: no stencil on the even sites (AOS: they get y; in
@@ -68,94 +51,6 @@ template <class GaugeT> struct SplitArg {
     unsigned int *counter;
 };
 
-LYM_D C load1(const SpinorD &v, int word, int h)
-{
-    const double2 w = __ldg(v.v + (size_t)word * v.stride + h);
-    return C{w.x, w.y};
-}
-LYM_D C shfl_xor(C z, int m)
-{
-    return C{__shfl_xor_sync(0xffffffffu, z.re, m), __shfl_xor_sync(0xffffffffu, z.im, m)};
-}
-
-// spin 2 d + k of H x at the site (p, h), lexicographic index s, coordinates c
-template <class GaugeT>
-LYM_D void split_hopping(const Geom &g, const SpinorD &in, const GaugeT &U, int p, int h, int s, const int c[4], int k,
-                         int d, C own[3])
-{
-    C up[3], low[3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) up[m] = low[m] = C{0.0, 0.0};
-    const int wk = 3 * k, wp = 3 * (d ? 2 + k : 3 - k);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const int mu = 2 * d + j;
-        const int cm = d ? c[2 + j] : c[j], L = d ? g.L[2 + j] : g.L[j];
-        const int step = j == 0 ? (d ? g.L[3] : g.L[1] * g.L[2] * g.L[3]) : (d ? 1 : g.L[2] * g.L[3]);
-        // c_mu = -i s (j = 0) or s (j = 1)
-        const double sg = j == 0 ? (d & k ? -1.0 : 1.0) : (d | k ? 1.0 : -1.0);
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-            const int hn = (s + (dir == 0 ? (cm == L - 1 ? (1 - L) * step : step) : (cm == 0 ? (L - 1) * step : -step))) >> 1;
-            const double sh = dir == 0 ? -sg : sg;
-            typename GaugeT::Link Lk;
-            if (dir == 0) U.load(p, mu, h, Lk);
-            else U.load(1 - p, mu, hn, Lk);
-            C hv[3], w[3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                const C xk = load1(in, wk + m, hn), xp = load1(in, wp + m, hn);
-                const C z = j == 0 ? times_mi(xp) : xp;
-                hv[m] = xk;
-                fma_r(hv[m], sh, z);
-            }
-            if (dir == 0) mul_u(Lk, hv, w);
-            else mul_ud(Lk, hv, w);
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                up[m] = up[m] + w[m];
-                fma_r(low[m], sh, j == 0 ? times_i(w[m]) : w[m]);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        up[m] = up[m] + shfl_xor(up[m], 8);
-        low[m] = low[m] + shfl_xor(low[m], 24);
-        own[m] = d ? low[m] : up[m];
-    }
-}
-
-// rows 3 k .. 3 k + 2 of the Hermitian 6 x 6 block (parity p, chirality d) applied to the vector
-// (own spin k, other spin 1 - k)
-LYM_D void clover_rows(const double2 *clover, int stride, int p, int h, int k, int d, const C own[3], const C oth[3],
-                       C res[3])
-{
-    const double2 *base = clover + (size_t)((p * 2 + d) * 18) * stride + h;
-    auto word = [&](int w) { return __ldg(base + (size_t)w * stride); };
-    const double2 dm = word(1), de = word(k ? 2 : 0);
-    const double dg[3] = {k ? dm.y : de.x, k ? de.x : de.y, k ? de.y : dm.x};
-    const double2 a10 = word(3 + (k ? 9 : 0)), a20 = word(3 + (k ? 13 : 1)), a21 = word(3 + (k ? 14 : 2));
-#pragma unroll
-    for (int i = 0; i < 3; ++i) res[i] = dg[i] * own[i];
-    const C o10{a10.x, a10.y}, o20{a20.x, a20.y}, o21{a21.x, a21.y};
-    fma_cc(res[0], o10, own[1]);
-    fma_c(res[1], o10, own[0]);
-    fma_cc(res[0], o20, own[2]);
-    fma_c(res[2], o20, own[0]);
-    fma_cc(res[1], o21, own[2]);
-    fma_c(res[2], o21, own[1]);
-    // entries (3 + i, j) for k = 1, their transpose's conjugates for k = 0
-    constexpr int row[3] = {6, 9, 13};  // word of (3 + i, 0): 3 + tri_index(3 + i, 0)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double2 w = word(k ? row[i] + j : row[j] + i);
-            fma_c(res[i], C{w.x, k ? w.y : -w.y}, oth[j]);
-        }
-}
-
 struct NoFin {
     LYM_D void operator()(double) const {}
 };
@@ -164,15 +59,14 @@ struct AlphaFin {  // alpha = |r|^2 / <p, A p>
     LYM_D void operator()(double pap) const { s->alpha = make_double2(s->rr / pap, 0.0); }
 };
 struct MsAlphaFin {
+    static constexpr bool kParallelFinalize = true;
     MultishiftState *s;
     LYM_D void operator()(double pap) const { ms_alpha_step(s, pap); }
 };
 struct MsResidualFin {
     MultishiftState *s;
-    LYM_D void operator()(double rr) const
-    {
-        if (ms_residual_step(s, rr)) ms_window_step(s);
-    }
+    static constexpr bool kParallelFinalize = true;
+    LYM_D void operator()(double rr) const { ms_residual_step(s, rr); }
 };
 struct UpdateFin {  // the scalar step of OpCGUpdate
     CGState *s;
@@ -187,7 +81,10 @@ struct UpdateFin {  // the scalar step of OpCGUpdate
 template <int EPI, bool AOS, class GaugeT, class Fin>
 __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<GaugeT> arg, const Fin fin)
 {
-    if (arg.skip_if && *arg.skip_if) return;
+    if (arg.skip_if && *arg.skip_if) {
+        if (EPI == SPLIT_CG_NORM && arg.on_skip && blockIdx.x == 0 && threadIdx.x == 0) *arg.on_skip = 1;
+        return;
+    }
     constexpr bool kSecond = EPI == SPLIT_CG_UPDATE || EPI == SPLIT_MS_RESIDUAL;  // A p stays in registers
     constexpr bool kReduce = EPI == SPLIT_CG_NORM || kSecond;
     constexpr bool kXpay = EPI == SPLIT_XPAY || kReduce;
@@ -196,22 +93,29 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
     const Geom &g = arg.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int d = (lane >> 3) & 1, k = lane >> 4;
-    const bool both = arg.parity == 2;
-    const int p = both ? warp >> 1 : arg.parity;
-    const int hr = both ? blockIdx.x * (kSplitSites / 2) + (warp & 1) * 8 + (lane & 7)
-                        : blockIdx.x * kSplitSites + warp * 8 + (lane & 7);
+    int p, hr;
+    if (kReduce && arg.even_identity) {
+        // the stencil's blocks, 32 odd half-sites each, then those of the even sites, which only
+        // stream: with both parities in a block half of its warps would idle (10 x 12 x 14 x 18:
+        // norm 15.6 against 16.6 us, residual 19.7 against 21.7)
+        const int odd = (g.Vh + kSplitSites - 1) / kSplitSites, blk = blockIdx.x;
+        p = blk < odd ? 1 : 0;
+        hr = (p ? blk : blk - odd) * kSplitSites + warp * 8 + (lane & 7);
+    } else if (arg.parity == 2) {
+        p = warp >> 1;
+        hr = blockIdx.x * (kSplitSites / 2) + (warp & 1) * 8 + (lane & 7);
+    } else {
+        p = arg.parity;
+        hr = blockIdx.x * kSplitSites + warp * 8 + (lane & 7);
+    }
     const bool in = hr < g.Vh;
     const int h = in ? hr : g.Vh - 1;
     if (AOS && arg.aos_v2) {
         for (int i = threadIdx.x; i < kSplitSites * 12; i += kSplitThreads) {
             const int site = i / 12;
             if (blockIdx.x * kSplitSites + site < g.V)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                                 (unsigned)__cvta_generic_to_shared(tile + site * kTileWord + i % 12)),
-                             "l"(arg.aos_v2 + (size_t)blockIdx.x * kSplitSites * 12 + i)
-                             : "memory");
+                copy16(tile + site * kTileWord + i % 12, arg.aos_v2 + (size_t)blockIdx.x * kSplitSites * 12 + i);
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
     int c[4];
     site_coords(g, h, p, c);
@@ -226,8 +130,11 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
             for (int m = 0; m < 3; ++m) res[m] = yo[m] = load1(arg.y[0], sp + m, h);
         }
     } else {
+        const double2 *const clover = arg.clover + (size_t)((p * 2 + d) * 18) * g.stride + h;
+        auto word = [&](int w) { return __ldg(clover + (size_t)clover_word(w, k) * g.stride); };
         C acc[3];
-        split_hopping(g, arg.in[p], arg.U, p, h, s, c, k, d, acc);
+        const SpinorD x = arg.in[p];
+        split_hopping(g, [&](int w, int sn) { return load1(x, w, sn >> 1); }, arg.U, p, h, s, c, k, d, acc);
         C own[3], oth[3];
         if constexpr (EPI == SPLIT_SCALE) {
 #pragma unroll
@@ -243,14 +150,14 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
                 }
                 oth[m] = shfl_xor(own[m], 16);
             }
-            clover_rows(arg.clover, g.stride, p, h, k, d, own, oth, res);
+            clover_rows(word, k, own, oth, res);
         } else {
 #pragma unroll
             for (int m = 0; m < 3; ++m) yo[m] = own[m] = load1(arg.y[p], sp + m, h);
             if (arg.clover) {
 #pragma unroll
                 for (int m = 0; m < 3; ++m) oth[m] = load1(arg.y[p], so + m, h);
-                clover_rows(arg.clover, g.stride, p, h, k, d, own, oth, res);
+                clover_rows(word, k, own, oth, res);
             } else {
 #pragma unroll
                 for (int m = 0; m < 3; ++m) res[m] = own[m];
@@ -272,7 +179,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
     if constexpr (AOS) {
         double2 *t = tile + (s - blockIdx.x * kSplitSites) * kTileWord + sp;
         if (arg.aos_v2) {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
             const C al = {arg.alpha_re, arg.alpha_im};
             if (in) {
@@ -361,10 +268,8 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
 #pragma unroll 8
         for (int i = threadIdx.x; i < (int)gridDim.x; i += kSplitThreads) t += __ldcg(arg.partials + i);
         const double all = block_total(t);
-        if (threadIdx.x == 0) {
-            fin(all);
-            *arg.counter = 0u;
-        }
+        if (ParallelFinalize<Fin>::value || threadIdx.x == 0) fin(all);
+        if (threadIdx.x == 0) *arg.counter = 0u;
     }
 }
 
@@ -377,9 +282,9 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     // views of one parity, or of the full spinors in both mode
     const bool both = P.parity == 2 && !P.even_identity;
     for (int p = 0; p < 2; ++p) {
-        a.in[p] = both ? P.in.d(1 - p) : P.in.d();
+        a.in[p] = P.in.v ? (both ? P.in.d(1 - p) : P.in.d()) : SpinorD{};
         a.out[p] = P.out.v ? (both ? P.out.d(p) : P.out.d()) : SpinorD{};
-        a.y[p] = both ? P.y.d(p) : P.y.d();
+        a.y[p] = P.y.v ? (both ? P.y.d(p) : P.y.d()) : SpinorD{};
         a.v2[p] = P.v2.v ? (both ? P.v2.d(p) : P.v2.d()) : SpinorD{};
         a.x[p] = a.r[p] = SpinorD{};
     }
@@ -392,6 +297,7 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     a.alpha_re = P.alpha_re;
     a.alpha_im = P.alpha_im;
     a.skip_if = P.skip_if;
+    a.on_skip = nullptr;
     a.aos_out = (double2 *)P.aos_out;
     a.aos_v2 = (const double2 *)P.aos_v2;
     a.even_identity = P.even_identity;
@@ -404,8 +310,10 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     return a;
 }
 
-int split_blocks(const Geom &g, int parity)
+// even_identity with sums: odd and even half-sites in blocks of their own
+int split_blocks(const Geom &g, int parity, bool apart = false)
 {
+    if (apart) return 2 * ((g.Vh + kSplitSites - 1) / kSplitSites);
     const int per = parity == 2 ? kSplitSites / 2 : kSplitSites;
     return (g.Vh + per - 1) / per;
 }
@@ -441,7 +349,7 @@ void run_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor
     a.alpha = &cs->alpha;
     a.partials = partials;
     a.counter = counter;
-    const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
+    const int nb = split_blocks(P.g, P.parity, P.even_identity != 0), nt = kSplitThreads;
     if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, AlphaFin{cs});
     else split_kernel<SPLIT_CG_UPDATE, false><<<nb, nt, 0, st>>>(a, UpdateFin{cs});
 }
@@ -455,16 +363,17 @@ void run_split_ms(const DslashParams &P, int mode, const Spinor &p, const Spinor
     a.gamma5 = 1;
     a.ring = ring;
     a.ms = ms;
+    a.on_skip = &ms->pause;
     a.partials = partials;
     a.counter = counter;
-    const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
+    const int nb = split_blocks(P.g, P.parity, P.even_identity != 0), nt = kSplitThreads;
     if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, MsAlphaFin{ms});
     else split_kernel<SPLIT_MS_RESIDUAL, false><<<nb, nt, 0, st>>>(a, MsResidualFin{ms});
 }
 
 }  // namespace
 
-int split_partials(const Geom &g) { return split_blocks(g, 2); }
+int split_partials(const Geom &g) { return split_blocks(g, 2, true); }
 
 void launch_split(const DslashParams &P, cudaStream_t st)
 {
