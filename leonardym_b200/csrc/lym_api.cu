@@ -92,6 +92,7 @@ struct lym_context {
     int inject_alloc_failures = 0;  // the next n device allocations report failure (tests)
     bool inject_copy_wait = false;  // the next check of the bulk-copy wait word reports a give-up (tests)
     int link_reals = 12;            // FP32 SU(3) link format of the single-RHS stencils: 12 or 8
+    int persist = 0;                // blocks per SM of the one-launch CG (lym_persist.cu), 0: not fitting
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -771,6 +772,35 @@ DslashParams square_half_params(lym_context *c, OpEntry &op, const Spinor &q, co
     return P;
 }
 
+// The iterations of a CG on A = op + sigma (op a squared kind on full spinors) whose state, x, r
+// and scratch p, q are set up, by cooperative launches of kPersistSteps iterations.
+void persist_cg(lym_context *c, OpEntry &op, double sigma, const Spinor &x, const Spinor &r, const Spinor &p,
+                const Spinor &q, int max_steps)
+{
+    constexpr int kPersistSteps = 512;  // bounds a launch to some ms
+    DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
+    P.sigma = sigma;
+    Vec p1(c, PREC_D, 2);
+    CGState *S = cg_state(c);
+    int *err = c->d_err + 2;
+    CK(cudaMemsetAsync(err, 0, sizeof(int), c->st));
+    // one such launch at a time in the process: two grids that each wait for all their blocks must
+    // not share the GPU's block slots
+    static std::mutex one_launch;
+    for (long done = 0; done < (long)max_steps + kPersistSteps; done += kPersistSteps) {
+        std::lock_guard<std::mutex> lock(one_launch);
+        CK(launch_cg_persist(P, c->persist, p, *p1, x, r, q, S, c->spartials, c->counter + 8, err, kPersistSteps, c->st));
+        count(c, 1);
+        CK(cudaMemcpyAsync(c->h_scal, err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        pull_state(c, sizeof(CGState));
+        int e = 0;
+        memcpy(&e, c->h_scal, sizeof(int));
+        if (e) fail(c, LYM_ERR_TIMEOUT, "a wait between the blocks of the one-launch CG gave up");
+        if (cg_host(c).pause) return;
+    }
+    fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %d iterations", max_steps);
+}
+
 // --- CG (ConjugateGradient::solve, inverters/ConjugateGradient.cpp:10-74) ---
 // matvec: A; square: the operator when A = op + sigma with op a Hermitian square (the iteration
 // then runs in 3 launches, 5 even-odd, instead of 7)
@@ -814,8 +844,9 @@ int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const 
         }
         run_site(c, OpCGDirection<SpinorD, SpinorD>{(*p).d(), (*r).d(), S}, nparity, gate);
     };
-    if (max_steps > 0) run_gated_state(c, S, step, 8, max_steps);
-    else pull_state(c, sizeof(CGState));
+    if (max_steps <= 0) pull_state(c, sizeof(CGState));
+    else if (square && c->persist && !is_even_odd(square->kind)) persist_cg(c, *square, sigma, x, *r, *p, *ap, max_steps);
+    else run_gated_state(c, S, step, 8, max_steps);
     CGState &R = cg_host(c);
     if (st) {
         st->converged = R.converged;
@@ -2715,7 +2746,9 @@ int lym_context_create(const int dims[4], int rep, int device, lym_context **out
         CK(cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));
         c->partials = (double *)dev_alloc(c, (size_t)kBlasGridMax * kMaxRed * sizeof(double));
         c->bpartials = (double *)dev_alloc(c, (size_t)kBlasGridMax * kMaxBatch * kBatchMaxRed * sizeof(double));
-        c->spartials = (double *)dev_alloc(c, (size_t)split_partials(c->g) * sizeof(double));
+        c->persist = cg_persist_residency(c->g, c->rep, c->device);
+        const int nsum = std::max(split_partials(c->g), c->persist ? cg_persist_partials(c->g) : 0);
+        c->spartials = (double *)dev_alloc(c, (size_t)nsum * sizeof(double));
         c->nbr = (int *)dev_alloc(c, (size_t)16 * c->g.stride * sizeof(int));
         launch_nbr_table(c->g, c->nbr, c->st);
         c->counter = (unsigned int *)dev_alloc(c, 64);

@@ -96,6 +96,17 @@ void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spi
 void launch_split_ms(const DslashParams &P, int mode, const Spinor &p, const void *ring, void *state, double *partials,
                      unsigned int *counter, cudaStream_t st);
 int split_partials(const Geom &g);
+// CG on Q Q + sigma over both parities in one cooperative launch of at most `steps` iterations
+// (lym_persist.cu), where the lattice's blocks are all resident at once (cg_persist_residency
+// not 0: the argument minb).
+// P: the full operator, sigma; p0, p1, q: scratch spinors; r: the residual of x; state: the
+// CGState; partials: cg_persist_partials doubles; arrived, err: a word each (err is set to 1
+// when a wait between the blocks gave up)
+int cg_persist_residency(const Geom &g, int rep, int device);
+int cg_persist_partials(const Geom &g);
+cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0, const Spinor &p1, const Spinor &x,
+                              const Spinor &r, const Spinor &q, void *state, double *partials, unsigned int *arrived,
+                              int *err, int steps, cudaStream_t st);
 void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in, const void *clover, int parity,
                    int gamma5, cudaStream_t st);
 void launch_pack(const Geom &g, const double *aos, const Spinor &full, cudaStream_t st);

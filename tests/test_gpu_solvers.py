@@ -370,3 +370,51 @@ def test_rhmc_action_energy_and_force_solves(setup, oracle):
         for x, y, xr, yr in zip(X, Y, xo, yo):
             assert rel(x, xr) < 1e-8
             assert rel(y, yr) < 1e-8
+
+
+@pytest.mark.parametrize("rep", ["su3", "su2adj"])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 2, 6), (4, 4, 2, 10), (4, 4, 4, 6)])
+@pytest.mark.parametrize("kind", ["SquareDiracWilson", "SquareImproved", "SquareEvenOddImproved"])
+def test_fused_square_cg(rep, dims, kind, oracle):
+    """CG on the squared operators, whose vector work runs inside the products (Wilson and clover:
+    the whole solve in one launch): fewer half-sites than a block, ragged last blocks, a shift, and
+    more iterations than one launch runs."""
+    kappa, csw = (0.12, 1.0) if rep == "su3" else (0.15, 1.2)
+    links = synth.fermion_links(dims, rep, 0.3, 71)
+    lat = L.Lattice(dims, rep)
+    try:
+        cls = {"SquareDiracWilson": L.SquareDiracWilsonOperator, "SquareImproved": L.SquareImprovedDiracWilsonOperator,
+               "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind]
+        op = cls(lat)
+        op.setKappa(kappa)
+        clover = kind != "SquareDiracWilson"
+        if clover:
+            op.setCSW(csw)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, csw if clover else 0.0, True)
+        b = synth.gaussian_spinor(dims, 3, 72)
+        eps = 1e-22 * float(np.vdot(b, b).real)
+        cg = L.ConjugateGradient()
+        cg.setPrecision(eps)
+        x = lat.new_vector()
+        assert cg.solve(op, b, x)
+        rc, xo, steps = oracle.cg(orc, b, eps, 3000)
+        assert abs(cg.getLastSteps() - steps) <= 2
+        assert rel(x, xo) < 1e-9 and rel(orc.multiply(x), b) < 1.1e-11
+        # one step of the reference, then a run past the iterations of a launch (no stop)
+        cg.setMaximumSteps(1)
+        cg.setPrecision(0.0)
+        assert not cg.solve(op, b, x)
+        assert rel(x, oracle.cg(orc, b, 0.0, 1)[1]) < 1e-12
+        if dims == (4, 4, 4, 6) and kind != "SquareEvenOddImproved":  # |r|^2 stays above 1e-150
+            cg.setMaximumSteps(530)
+            assert not cg.solve(op, b, x) and cg.stats.iterations == 530
+            assert rel(orc.multiply(x), b) < 1e-12
+        # with shifts, one CG each
+        ms = L.MultishiftSolver.getInstance("mass_estrapolation")
+        ms.setPrecision(eps)
+        sols = []
+        assert ms.solve(op, b, sols, [0.0, 0.3])
+        assert rel(orc.multiply(sols[1]) + 0.3 * sols[1], b) < 1.1e-11
+    finally:
+        lat.close()
