@@ -62,9 +62,11 @@ struct DslashParams {
     Spinor y;                // same-parity input (EPI_XPAY, EPI_XPAY_INV)
     Spinor v2;               // optional added vector (EPI_XPAY)
     // FP64 EPI_XPAY with parity 2 may write a caller's AoS vector instead of `out`, adding
-    // alpha times another AoS vector (aos_v2, or null; it may be aos_out itself).  With
+    // alpha times another AoS vector (aos_v2, or null; it may be aos_out itself), and read its
+    // input from one (aos_in instead of in and y; it must not overlap aos_out).  With
     // even_identity (parity 2) the stencil runs on the odd sites only (in, out, y: half spinors)
     // and the even sites get `even`.
+    const double *aos_in = nullptr;
     double *aos_out = nullptr;
     const double *aos_v2 = nullptr;
     int even_identity = 0;

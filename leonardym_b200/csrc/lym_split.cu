@@ -39,6 +39,7 @@ template <class GaugeT> struct SplitArg {
     double a, b, alpha_re, alpha_im;
     const int *skip_if;
     int *on_skip;            // SPLIT_CG_NORM: set when the launch is skipped
+    const double2 *aos_in;   // IN_AOS
     double2 *aos_out;        // AOS: the full result
     const double2 *aos_v2;   // AOS: the added vector, or null
     int even_identity;       // both mode: no stencil on the even sites (AOS: they get y; in
@@ -78,7 +79,15 @@ struct UpdateFin {  // the scalar step of OpCGUpdate
     }
 };
 
-template <int EPI, bool AOS, class GaugeT, class Fin>
+// where a launch reads its input: packed spinors, or (SPLIT_XPAY to AoS) the caller's AoS vector
+enum SplitIn : int { IN_PACKED = 0, IN_AOS = 1 };
+LYM_D C load_aos(const double2 *v, int word, int s)
+{
+    const double2 w = __ldg(v + (size_t)s * 12 + word);
+    return C{w.x, w.y};
+}
+
+template <int EPI, bool AOS, int IN, class GaugeT, class Fin>
 __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<GaugeT> arg, const Fin fin)
 {
     if (arg.skip_if && *arg.skip_if) {
@@ -133,8 +142,14 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
         const double2 *const clover = arg.clover + (size_t)((p * 2 + d) * 18) * g.stride + h;
         auto word = [&](int w) { return __ldg(clover + (size_t)clover_word(w, k) * g.stride); };
         C acc[3];
-        const SpinorD x = arg.in[p];
-        split_hopping(g, [&](int w, int sn) { return load1(x, w, sn >> 1); }, arg.U, p, h, s, c, k, d, acc);
+        if constexpr (IN == IN_AOS) {
+            split_hopping(g, [&](int w, int sn) { return load_aos(arg.aos_in, w, sn); }, arg.U, p, h, s, c, k, d, acc);
+        } else {
+            const SpinorD x = arg.in[p];
+            split_hopping(g, [&](int w, int sn) { return load1(x, w, sn >> 1); }, arg.U, p, h, s, c, k, d, acc);
+        }
+        // y of the site: an AoS input is its own y
+        auto y = [&](int w) { return IN == IN_AOS ? load_aos(arg.aos_in, w, s) : load1(arg.y[p], w, h); };
         C own[3], oth[3];
         if constexpr (EPI == SPLIT_SCALE) {
 #pragma unroll
@@ -145,7 +160,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
                 if (EPI == SPLIT_CLOVINV) {
                     own[m] = arg.a * acc[m];
                 } else {
-                    own[m] = load1(arg.y[p], sp + m, h);
+                    own[m] = y(sp + m);
                     fma_r(own[m], arg.b, acc[m]);
                 }
                 oth[m] = shfl_xor(own[m], 16);
@@ -153,10 +168,10 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
             clover_rows(word, k, own, oth, res);
         } else {
 #pragma unroll
-            for (int m = 0; m < 3; ++m) yo[m] = own[m] = load1(arg.y[p], sp + m, h);
+            for (int m = 0; m < 3; ++m) yo[m] = own[m] = y(sp + m);
             if (arg.clover) {
 #pragma unroll
-                for (int m = 0; m < 3; ++m) oth[m] = load1(arg.y[p], so + m, h);
+                for (int m = 0; m < 3; ++m) oth[m] = y(so + m);
                 clover_rows(word, k, own, oth, res);
             } else {
 #pragma unroll
@@ -298,6 +313,7 @@ template <class GaugeT> SplitArg<GaugeT> split_arg(const DslashParams &P, const 
     a.alpha_im = P.alpha_im;
     a.skip_if = P.skip_if;
     a.on_skip = nullptr;
+    a.aos_in = (const double2 *)P.aos_in;
     a.aos_out = (double2 *)P.aos_out;
     a.aos_v2 = (const double2 *)P.aos_v2;
     a.even_identity = P.even_identity;
@@ -323,14 +339,15 @@ template <class GaugeT> void run_split(const DslashParams &P, const GaugeT &U, c
     const SplitArg<GaugeT> a = split_arg(P, U);
     const int nb = split_blocks(P.g, P.parity), nt = kSplitThreads;
     if (P.aos_out) {
-        split_kernel<SPLIT_XPAY, true><<<nb, nt, 0, st>>>(a, NoFin{});
+        if (P.aos_in) split_kernel<SPLIT_XPAY, true, IN_AOS><<<nb, nt, 0, st>>>(a, NoFin{});
+        else split_kernel<SPLIT_XPAY, true, IN_PACKED><<<nb, nt, 0, st>>>(a, NoFin{});
         return;
     }
     switch (P.epi) {
-    case EPI_SCALE_: split_kernel<SPLIT_SCALE, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
-    case EPI_CLOVINV_: split_kernel<SPLIT_CLOVINV, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
-    case EPI_XPAY_: split_kernel<SPLIT_XPAY, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
-    default: split_kernel<SPLIT_XPAY_INV, false><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    case EPI_SCALE_: split_kernel<SPLIT_SCALE, false, IN_PACKED><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    case EPI_CLOVINV_: split_kernel<SPLIT_CLOVINV, false, IN_PACKED><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    case EPI_XPAY_: split_kernel<SPLIT_XPAY, false, IN_PACKED><<<nb, nt, 0, st>>>(a, NoFin{}); break;
+    default: split_kernel<SPLIT_XPAY_INV, false, IN_PACKED><<<nb, nt, 0, st>>>(a, NoFin{}); break;
     }
 }
 
@@ -350,8 +367,8 @@ void run_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spinor
     a.partials = partials;
     a.counter = counter;
     const int nb = split_blocks(P.g, P.parity, P.even_identity != 0), nt = kSplitThreads;
-    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, AlphaFin{cs});
-    else split_kernel<SPLIT_CG_UPDATE, false><<<nb, nt, 0, st>>>(a, UpdateFin{cs});
+    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false, IN_PACKED><<<nb, nt, 0, st>>>(a, AlphaFin{cs});
+    else split_kernel<SPLIT_CG_UPDATE, false, IN_PACKED><<<nb, nt, 0, st>>>(a, UpdateFin{cs});
 }
 
 template <class GaugeT>
@@ -367,8 +384,8 @@ void run_split_ms(const DslashParams &P, int mode, const Spinor &p, const Spinor
     a.partials = partials;
     a.counter = counter;
     const int nb = split_blocks(P.g, P.parity, P.even_identity != 0), nt = kSplitThreads;
-    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false><<<nb, nt, 0, st>>>(a, MsAlphaFin{ms});
-    else split_kernel<SPLIT_MS_RESIDUAL, false><<<nb, nt, 0, st>>>(a, MsResidualFin{ms});
+    if (mode == CG_NORM) split_kernel<SPLIT_CG_NORM, false, IN_PACKED><<<nb, nt, 0, st>>>(a, MsAlphaFin{ms});
+    else split_kernel<SPLIT_MS_RESIDUAL, false, IN_PACKED><<<nb, nt, 0, st>>>(a, MsResidualFin{ms});
 }
 
 }  // namespace

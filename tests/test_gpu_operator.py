@@ -273,3 +273,34 @@ def test_fp64_stencil_tiles(rep, dims, kind, oracle):
         assert rel(call("lym_multiply_add_device", buf[:-1], dx, buf[1:], *a), refa) < 1e-13
     finally:
         lat.close()
+
+
+@pytest.mark.parametrize("dims", [(8, 8, 8, 24), (8, 8, 8, 26)])
+@pytest.mark.parametrize("kind,rep", [("DiracWilson", "su3"), ("Improved", "su3"), ("Improved", "su2adj")])
+def test_input_read_in_place_or_packed(kind, rep, dims, oracle):
+    """Either side of the size up to which an application reads the caller's vector in the stencil
+    itself; a result over the input is packed first on both."""
+    import ctypes as C
+
+    import torch
+    kappa, csw = 0.13, 1.0
+    links = synth.fermion_links(dims, rep, 0.4, 47)
+    lat = L.Lattice(dims, rep)
+    try:
+        op = GPU_CLASS[kind](lat)
+        op.setKappa(kappa)
+        if kind != "DiracWilson":
+            op.setCSW(csw)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, 0.0 if kind == "DiracWilson" else csw, True)
+        x = synth.gaussian_spinor(dims, 3, 48)
+        ref = orc.multiply(x)
+        for over in (False, True):
+            dx = torch.from_numpy(x).cuda()
+            out = dx if over else torch.empty_like(dx)
+            torch.cuda.synchronize()
+            assert L.lib().lym_multiply_device(lat.handle, op.op_id, C.c_void_p(out.data_ptr()),
+                                               C.c_void_p(dx.data_ptr())) == 0
+            assert rel(out.cpu().numpy(), ref) < 1e-13
+    finally:
+        lat.close()
