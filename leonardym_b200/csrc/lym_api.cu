@@ -1041,7 +1041,9 @@ int eo_bicgstab(lym_context *c, OpEntry &op, const Spinor &b, const Spinor &x, c
 int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor &x, const Spinor *guess, double tol,
           int max_steps, lym_solve_stats *st)
 {
-    const double delta = sprec == PREC_D ? 0.0 : 0.1;
+    // FP32 keeps its recursion over two decades of the residual: adjoint 16^3 x 32, 6 updates instead
+    // of 11 at delta 0.1, 109 iterations with either, 8.0 against 9.3 ms
+    const double delta = sprec == PREC_D ? 0.0 : sprec == PREC_F ? 0.01 : 0.1;
     OpEntry &eo = op;  // apply_schur takes gamma5 explicitly
     if (kind_has_clover(op.kind)) ensure_clover(c, op);
     Vec bp(c, PREC_D, 1), rN(c, PREC_D, 1), te(c, PREC_D, 1), t1(c, PREC_D, 1);
