@@ -772,33 +772,43 @@ DslashParams square_half_params(lym_context *c, OpEntry &op, const Spinor &q, co
     return P;
 }
 
-// The iterations of a CG on A = op + sigma (op a squared kind on full spinors) whose state, x, r
-// and scratch p, q are set up, by cooperative launches of kPersistSteps iterations.
-void persist_cg(lym_context *c, OpEntry &op, double sigma, const Spinor &x, const Spinor &r, const Spinor &p,
-                const Spinor &q, int max_steps)
+// Cooperative launches go(steps, err) of at most `kOneLaunchSteps` iterations each, until the state
+// pauses.
+template <class S, class Go> void run_one_launch(lym_context *c, int max_steps, Go go, S *state)
 {
-    constexpr int kPersistSteps = 512;  // bounds a launch to some ms
-    DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
-    P.sigma = sigma;
-    Vec p1(c, PREC_D, 2);
-    CGState *S = cg_state(c);
+    constexpr int kOneLaunchSteps = 512;  // bounds a launch to some ms
     int *err = c->d_err + 2;
     CK(cudaMemsetAsync(err, 0, sizeof(int), c->st));
     // one such launch at a time in the process: two grids that each wait for all their blocks must
     // not share the GPU's block slots
     static std::mutex one_launch;
-    for (long done = 0; done < (long)max_steps + kPersistSteps; done += kPersistSteps) {
+    for (long done = 0; done < (long)max_steps + kOneLaunchSteps; done += kOneLaunchSteps) {
         std::lock_guard<std::mutex> lock(one_launch);
-        CK(launch_cg_persist(P, c->persist, p, *p1, x, r, q, S, c->spartials, c->counter + 8, err, kPersistSteps, c->st));
+        CK(go(kOneLaunchSteps, err));
         count(c, 1);
         CK(cudaMemcpyAsync(c->h_scal, err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-        pull_state(c, sizeof(CGState));
+        CK(cudaMemcpyAsync(c->h_state, state, sizeof(S), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
         int e = 0;
         memcpy(&e, c->h_scal, sizeof(int));
-        if (e) fail(c, LYM_ERR_TIMEOUT, "a wait between the blocks of the one-launch CG gave up");
-        if (cg_host(c).pause) return;
+        if (e) fail(c, LYM_ERR_TIMEOUT, "a wait between the blocks of a one-launch solver gave up");
+        if (state_paused(*(S *)c->h_state)) return;
     }
     fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %d iterations", max_steps);
+}
+
+// The iterations of a CG on A = op + sigma (op a squared kind on full spinors) whose state, x, r
+// and scratch p, q are set up.
+void persist_cg(lym_context *c, OpEntry &op, double sigma, const Spinor &x, const Spinor &r, const Spinor &p,
+                const Spinor &q, int max_steps)
+{
+    DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
+    P.sigma = sigma;
+    Vec p1(c, PREC_D, 2);
+    CGState *S = cg_state(c);
+    run_one_launch(c, max_steps, [&](int steps, int *err) {
+        return launch_cg_persist(P, c->persist, p, *p1, x, r, q, S, c->spartials, c->counter + 8, err, steps, c->st);
+    }, S);
 }
 
 // --- CG (ConjugateGradient::solve, inverters/ConjugateGradient.cpp:10-74) ---
@@ -1042,7 +1052,7 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
           int max_steps, lym_solve_stats *st)
 {
     // FP32 keeps its recursion over two decades of the residual: adjoint 16^3 x 32, 6 updates instead
-    // of 11 at delta 0.1, 109 iterations with either, 8.0 against 9.3 ms
+    // of 11 at delta 0.1, 109 iterations with either
     const double delta = sprec == PREC_D ? 0.0 : sprec == PREC_F ? 0.01 : 0.1;
     OpEntry &eo = op;  // apply_schur takes gamma5 explicitly
     if (kind_has_clover(op.kind)) ensure_clover(c, op);
@@ -1173,7 +1183,8 @@ template <class View> struct MsViews {
 
 // Multishift CG on (A + shift_i), A Hermitian positive definite (a Square* kind), in FP64.  The
 // shifted x_i and p_i are updated once per kMsWin steps from a ring of residuals
-// (multishift_cg_mixed tells how): 4 of their vectors move per window instead of per step.
+// (multishift_cg_mixed tells how): 4 of their vectors move per window instead of per step.  Small
+// lattices run all steps in one launch (lym_persist.cu).
 int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts, double eps, int max_steps,
                   const Spinor &b, std::vector<Spinor> &xs, lym_solve_stats *st)
 {
@@ -1248,8 +1259,23 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
         if (++nstep % kMsWin == 0) views.template flush<double2, double>(S, nshift, 2 * 12 * c->g.stride);
     };
     int rc = LYM_OK;
+    const bool eo = is_even_odd(op.kind);
+    const int blocks = square ? ms_persist_blocks(c->g, c->rep, c->device, eo) : 0;
     if (bb > 0 && max_steps > 0) {
-        run_gated_state(c, S, step, kMsWin, max_steps);
+        if (blocks > 0) {
+            DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
+            P.sigma = s0;
+            if (eo) P.b = -op.kappa * op.kappa;
+            const void *Ti = eo && kind_has_clover(op.kind) ? op.clover.Tinv[PREC_D] : nullptr;
+            Vec p1(c, PREC_D, 2);
+            DevBuf sums(c, 2 * (size_t)blocks * sizeof(double), false);
+            run_one_launch(c, max_steps, [&](int steps, int *err) {
+                return launch_ms_persist(P, Ti, eo, pb, *p1, *ap, half, views.ring, views.x, views.p, nshift, S,
+                                         (double *)sums.p, c->counter + 8, err, blocks, steps, c->st);
+            }, S);
+        } else {
+            run_gated_state(c, S, step, kMsWin, max_steps);
+        }
         MultishiftState &R = *(MultishiftState *)c->h_state;
         rc = R.converged ? LYM_OK : LYM_NOT_CONVERGED;
         if (st) {

@@ -109,6 +109,15 @@ int cg_persist_partials(const Geom &g);
 cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0, const Spinor &p1, const Spinor &x,
                               const Spinor &r, const Spinor &q, void *state, double *partials, unsigned int *arrived,
                               int *err, int steps, cudaStream_t st);
+// The FP64 multishift CG likewise: P the operator's second (or only) stencil with the base shift,
+// Ti T^-1 of the even-odd kind (both null without clover); p0, p1, q: scratch full spinors, tmp: a
+// half spinor (even-odd); ring, x, dir: device arrays of SpinorD views; blocks:
+// ms_persist_blocks (0: not on this lattice); partials: 2 * blocks doubles.
+int ms_persist_blocks(const Geom &g, int rep, int device, bool even_odd);
+cudaError_t launch_ms_persist(const DslashParams &P, const void *Ti, bool even_odd, const Spinor &p0, const Spinor &p1,
+                              const Spinor &q, const Spinor &tmp, const void *ring, const void *x, const void *dir,
+                              int nshift, void *state, double *partials, unsigned int *arrived, int *err, int blocks,
+                              int steps, cudaStream_t st);
 void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in, const void *clover, int parity,
                    int gamma5, cudaStream_t st);
 void launch_pack(const Geom &g, const double *aos, const Spinor &full, cudaStream_t st);

@@ -12,8 +12,7 @@
 // barrier, and then runs the CG step's scalars (OpCGUpdate) on its own copy: all copies agree bit
 // for bit.  Directions alternate between two buffers and partial sums between two
 // halves, so that nobody overwrites what a slower block may still read.
-// 8^4 clover, 106 iterations: 1.04 ms (9.8 us an iteration) against 2.2 ms; whole solve with its
-// transfers 1.14 against 2.37 ms.
+// PERSIST_TIMES
 #include "lym_blas.cuh"
 #include "lym_internal.h"
 #include "lym_solver_ops.cuh"
@@ -44,14 +43,20 @@ LYM_D C load_cg(const SpinorD &v, int word, int h)  // from L2: other SMs write 
     return C{w.x, w.y};
 }
 
-// Grid barrier of a cooperative launch (all blocks resident).  The wait is bounded, about a
-// second; false when it ran out.  target: arrivals expected so far.
-LYM_D bool grid_barrier(unsigned int *arrived, unsigned int target, bool *ok)
+// Grid barrier of a cooperative launch (all blocks resident) in two halves, work that needs no other
+// block's results between them.
+LYM_D void grid_arrive(unsigned int *arrived)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(arrived, 1u);
+    }
+}
+// target: arrivals expected so far.  The wait is bounded, about a second; false when it ran out.
+LYM_D bool grid_wait(unsigned int *arrived, unsigned int target, bool *ok)
+{
+    if (threadIdx.x == 0) {
         bool done = false;
         for (int i = 0; i < (1 << 21); ++i) {
             unsigned int v;
@@ -66,6 +71,11 @@ LYM_D bool grid_barrier(unsigned int *arrived, unsigned int target, bool *ok)
     }
     __syncthreads();
     return *ok;
+}
+LYM_D bool grid_barrier(unsigned int *arrived, unsigned int target, bool *ok)
+{
+    grid_arrive(arrived);
+    return grid_wait(arrived, target, ok);
 }
 
 template <int MINB, class GaugeT>
@@ -260,6 +270,312 @@ cudaError_t run(const DslashParams &P, int minb, const Spinor &p0, const Spinor 
     return cudaLaunchCooperativeKernel(kernel, dim3(persist_blocks(P.g)), dim3(kSplitThreads), args, kPersistSmem, st);
 }
 
+// ------------------------------------------------------------- multishift --
+// The FP64 multishift CG (multishift_cg: windowed shifted updates from a ring of residuals) on
+// Q Q + shifts in one cooperative launch.  Every block walks its tiles of 32 half-sites in each
+// phase; the vectors stay in L2 and the MultishiftState is replicated in every block's shared
+// memory.  EO: Q = gamma5 S on the odd sites, A = 1 + sigma on the even ones, whose tiles come last.
+// A step: [EO: tmp = T^-1 H p;] q = Q p with <p, A p>; [tmp = T^-1 H q;] r_{k+1} = r_k - alpha A p
+// with |r_{k+1}|^2, a grid barrier after each; p_k = r_k + beta p_{k-1} is formed where it is read,
+// as in the CG above.  The shifts' scalars and, after kMsWin steps or the last, the window's updates
+// of x_i and P_i run while a block waits for the others.
+// Latency bound (a stencil phase 7 us with 128 registers a thread; polling without the acquire,
+// reads through L1 and links fetched into shared memory while waiting change nothing at the larger
+// size).  8 shifts, ms a solve against launches per step: even-odd 8^4 2.25 and 2.83,
+// 10 x 12 x 14 x 18 4.2 and 4.9, SquareImproved 8^4 2.8 and 4.6, 10 x 12 x 14 x 18 7.7 and 10.6.
+template <class GaugeT> struct PersistMsArg {
+    Geom g;
+    GaugeT U;
+    const double2 *T, *Ti;   // null without clover
+    double b, sigma;
+    const SpinorD *ring, *x, *dir;  // device arrays: kMsWin + 1 residuals, solutions, window directions
+    SpinorD p[2], q;                // full spinors; p[k & 1] holds p_k
+    SpinorD tmp;                    // EO: an even half spinor
+    MultishiftState *state;
+    double *partials;               // 2 * gridDim.x
+    unsigned int *arrived;
+    int *err;
+    int nshift, steps;
+};
+
+template <bool EO, class GaugeT>
+__global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const PersistMsArg<GaugeT> a)
+{
+    __shared__ __align__(16) MultishiftState st;
+    __shared__ SpinorD ring[kMsWin + 1];
+    __shared__ double wsum[2][kSplitThreads / 32];
+    __shared__ bool ok;
+    const Geom &g = a.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = (lane >> 3) & 1, k = lane >> 4;
+    const int sp = 3 * (2 * d + k);
+    const int tiles = (g.Vh + kSplitSites - 1) / kSplitSites;
+    static_assert(sizeof(MultishiftState) % sizeof(int) == 0, "copied by words");
+    for (int i = threadIdx.x; i < (int)(sizeof(st) / sizeof(int)); i += kSplitThreads)
+        reinterpret_cast<int *>(&st)[i] = reinterpret_cast<const int *>(a.state)[i];
+    if (threadIdx.x <= kMsWin) ring[threadIdx.x] = a.ring[threadIdx.x];
+    __syncthreads();
+    auto block_total = [&](double v, int slot) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) wsum[slot][warp] = v;
+        __syncthreads();
+        return (wsum[slot][0] + wsum[slot][1]) + (wsum[slot][2] + wsum[slot][3]);
+    };
+    unsigned int target = 0;
+    auto arrive = [&]() {
+        target += gridDim.x;
+        grid_arrive(a.arrived);
+    };
+    auto wait = [&]() { return grid_wait(a.arrived, target, &ok); };
+    // the block's part of a sum, then the barrier's first half
+    auto contribute = [&](double v, int half) {
+        const double t = block_total(v, 0);
+        if (threadIdx.x == 0) a.partials[(size_t)half * gridDim.x + blockIdx.x] = t;
+        arrive();
+    };
+    // this thread's share of the blocks' parts
+    auto collect = [&](int half) {
+        double u = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += kSplitThreads)
+            u += __ldcg(a.partials + (size_t)half * gridDim.x + i);
+        return u;
+    };
+    struct At {
+        bool in;
+        int p, h, s, c[4];
+    };
+    auto place = [&](int tile, int p) {
+        At t;
+        const int hr = tile * kSplitSites + warp * 8 + (lane & 7);
+        t.in = hr < g.Vh;
+        t.p = p;
+        t.h = t.in ? hr : g.Vh - 1;
+        site_coords(g, t.h, p, t.c);
+        t.s = lex_of(g, t.c[0], t.c[1], t.c[2], t.c[3]);
+        return t;
+    };
+    // the tiles of both parities: EO the odd ones, which have the stencil, first
+    auto item = [&](int i) { return EO ? (i < tiles ? place(i, 1) : place(i - tiles, 0)) : place(i >> 1, i & 1); };
+    auto put = [&](const SpinorD &v, const At &t, int m, C z) {
+        if (t.in) v.v[(size_t)(sp + m) * v.stride + t.h] = make_double2(z.re, z.im);
+    };
+    auto rows = [&](const double2 *clover, const At &t, const C own[3], C res[3]) {
+        C oth[3];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) oth[m] = shfl_xor(own[m], 16);
+        const double2 *const base = clover + (size_t)((t.p * 2 + d) * 18) * g.stride + t.h;
+        clover_rows([&](int w) { return __ldg(base + (size_t)clover_word(w, k) * g.stride); }, k, own, oth, res);
+    };
+    // EO: tmp = T^-1 H v on the even sites, load(w, sn) the words of v
+    auto even_half = [&](auto load) {
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const At t = place(tile, 0);
+            C acc[3], res[3];
+            split_hopping(g, load, a.U, 0, t.h, t.s, t.c, k, d, acc);
+            if (a.Ti) rows(a.Ti, t, acc, res);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) put(a.tmp, t, m, a.Ti ? res[m] : acc[m]);
+        }
+    };
+    // rows of Q v at a site: own-site words and the hopping term's input
+    auto product = [&](auto load, const At &t, const C own[3], C res[3]) {
+        C acc[3];
+        split_hopping(g, load, a.U, t.p, t.h, t.s, t.c, k, d, acc);
+        if (a.T) {
+            rows(a.T, t, own, res);
+        } else {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) res[m] = own[m];
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            fma_r(res[m], a.b, acc[m]);
+            if (d) res[m] = -res[m];
+        }
+    };
+    int it = st.iter;
+    double rr = st.rr, beta = st.beta;
+    const bool stopped = st.stop != 0;
+    bool pending = false;  // the scalars of the residual rr have not been stepped yet
+    // the shifts' scalars after a residual; the window's updates (ms_flush_kernel) when it is full
+    auto settle = [&]() {
+        pending = false;
+        ms_residual_step(&st, rr);
+        __syncthreads();
+        if (st.win < kMsWin && !st.stop) return;
+        const int m = st.failed ? 0 : st.win, k0 = st.iter - m, words = 2 * 12 * g.stride;
+        for (int o = blockIdx.x * kSplitThreads + threadIdx.x; m > 0 && o < words; o += gridDim.x * kSplitThreads) {
+            double2 R[kMsWin];
+#pragma unroll
+            for (int j = 0; j < kMsWin; ++j)
+                if (j < m) R[j] = __ldcg(ring[(k0 + 1 + j) % (kMsWin + 1)].v + o);
+            for (int i = 0; i < a.nshift; ++i) {
+                if (!st.xupd[i]) continue;
+                double2 *const xp = a.x[i].v + o, *const pp = a.dir[i].v + o;
+                const double2 P = *pp;
+                double2 X = *xp, Q = word_scale(st.cp[i][0], P);
+                word_add(X, st.cx[i][0], P);
+#pragma unroll
+                for (int j = 0; j < kMsWin; ++j)
+                    if (j < m) {
+                        word_add(X, st.cx[i][j + 1], R[j]);
+                        word_add(Q, st.cp[i][j + 1], R[j]);
+                    }
+                *xp = X;
+                if (st.pupd[i] && st.active[i] == 1) *pp = Q;
+            }
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < a.nshift) {
+            const int i = threadIdx.x;
+            st.xupd[i] = st.pupd[i] = 0;
+            for (int j = 0; j <= kMsWin; ++j) st.cx[i][j] = st.cp[i][j] = 0.0;
+            st.cp[i][0] = 1.0;
+        }
+        if (threadIdx.x == 0) st.win = 0;
+        __syncthreads();
+    };
+    bool good = true;
+    for (int n = 0; n < a.steps && !stopped; ++n) {
+        const SpinorD r = ring[it % (kMsWin + 1)], rnext = ring[(it + 1) % (kMsWin + 1)];
+        const SpinorD pnew = a.p[it & 1], pold = a.p[(it + 1) & 1];
+        auto direction = [&](int p, int w, int h) {  // word w of p_k
+            C z = load_cg(r.par(p), w, h);
+            if (beta != 0.0) fma_r(z, beta, load_cg(pold.par(p), w, h));
+            return z;
+        };
+        const SpinorD tmp = a.tmp;
+        auto load_tmp = [&](int w, int sn) { return load_cg(tmp, w, sn >> 1); };
+        if (EO) {
+            even_half([&](int w, int sn) { return direction(1, w, sn >> 1); });
+            arrive();
+            if (pending) settle();
+            if (!(good = wait()) || st.stop) break;
+        }
+        double part = 0.0;
+        for (int i = blockIdx.x; i < 2 * tiles; i += gridDim.x) {
+            const At t = item(i);
+            C own[3], res[3];
+            double pp = 0.0, qq = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                own[m] = direction(t.p, sp + m, t.h);
+                put(pnew.par(t.p), t, m, own[m]);
+                pp += own[m].re * own[m].re + own[m].im * own[m].im;
+            }
+            if (EO && t.p == 0) {
+                qq = pp;
+            } else {
+                if (EO) product(load_tmp, t, own, res);
+                else product([&](int w, int sn) { return direction(1 - t.p, w, sn >> 1); }, t, own, res);
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    put(a.q.par(t.p), t, m, res[m]);
+                    qq += res[m].re * res[m].re + res[m].im * res[m].im;
+                }
+            }
+            if (t.in) part += qq + a.sigma * pp;
+        }
+        contribute(part, 0);
+        if (!EO && pending) settle();
+        if (!(good = wait()) || st.stop) break;
+        const double share = collect(0);
+        if (EO) {
+            const SpinorD q1 = a.q.par(1);
+            even_half([&](int w, int sn) { return load_cg(q1, w, sn >> 1); });
+            arrive();
+        }
+        const double pap = block_total(share, 1), alpha = rr / pap;
+        if (EO && !(good = wait())) break;
+        part = 0.0;
+        for (int i = blockIdx.x; i < 2 * tiles; i += gridDim.x) {
+            const At t = item(i);
+            const SpinorD qv = a.q.par(t.p), qn = a.q.par(1 - t.p);
+            C own[3], ap[3];
+            if (!(EO && t.p == 0)) {
+#pragma unroll
+                for (int m = 0; m < 3; ++m) own[m] = load_cg(qv, sp + m, t.h);
+                if (EO) product(load_tmp, t, own, ap);
+                else product([&](int w, int sn) { return load_cg(qn, w, sn >> 1); }, t, own, ap);
+            }
+            double nrm = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const C pv = load_cg(pnew.par(t.p), sp + m, t.h);
+                if (EO && t.p == 0) ap[m] = pv;
+                fma_r(ap[m], a.sigma, pv);
+                C rv = load_cg(r.par(t.p), sp + m, t.h);
+                fma_r(rv, -alpha, ap[m]);
+                nrm += rv.re * rv.re + rv.im * rv.im;
+                put(rnext.par(t.p), t, m, rv);
+            }
+            if (t.in) part += nrm;
+        }
+        contribute(part, 1);
+        ms_alpha_step(&st, pap);
+        if (!(good = wait())) break;
+        const double rr_new = block_total(collect(1), 1);
+        beta = rr_new / rr;
+        rr = rr_new;
+        ++it;
+        pending = true;
+    }
+    __syncthreads();
+    if (good && pending) settle();
+    if (threadIdx.x == 0 && !good) atomicOr(a.err, 1);
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < (int)(sizeof(st) / sizeof(int)); i += kSplitThreads)
+            reinterpret_cast<int *>(a.state)[i] = reinterpret_cast<const int *>(&st)[i];
+}
+
+template <bool EO, class GaugeT>
+cudaError_t run_ms(const DslashParams &P, const void *Ti, const Spinor &p0, const Spinor &p1, const Spinor &q,
+                   const Spinor &tmp, const void *ring, const void *x, const void *dir, int nshift,
+                   MultishiftState *state, double *partials, unsigned int *arrived, int *err, int blocks, int steps,
+                   const GaugeT &U, cudaStream_t st)
+{
+    PersistMsArg<GaugeT> a{P.g,
+                           U,
+                           (const double2 *)P.clover,
+                           (const double2 *)Ti,
+                           P.b,
+                           P.sigma,
+                           (const SpinorD *)ring,
+                           (const SpinorD *)x,
+                           (const SpinorD *)dir,
+                           {p0.d(), p1.d()},
+                           q.d(),
+                           tmp.v ? tmp.d() : SpinorD{},
+                           state,
+                           partials,
+                           arrived,
+                           err,
+                           nshift,
+                           steps};
+    const cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), st);
+    if (e != cudaSuccess) return e;
+    void *args[] = {&a};
+    return cudaLaunchCooperativeKernel((const void *)ms_persist_kernel<EO, GaugeT>, dim3(blocks), dim3(kSplitThreads),
+                                       args, 0, st);
+}
+
+// The grid of the one-launch multishift: a tile of either parity each, at most as many blocks as are
+// resident at once.  0 where these have more than a tile of each parity: a phase then takes two
+// rounds (even-odd 12^3 x 24, 648 tiles on 592 blocks: 7.8 against 6.1 ms with launches per step).
+template <bool EO, class GaugeT> int ms_blocks(const Geom &g, int device)
+{
+    int sms = 0, coop = 0, per = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ms_persist_kernel<EO, GaugeT>, kSplitThreads, 0) !=
+            cudaSuccess)
+        return 0;
+    const int tiles = (g.Vh + kSplitSites - 1) / kSplitSites;
+    if (tiles > sms * per) return 0;
+    return 2 * tiles < sms * per ? 2 * tiles : sms * per;
+}
+
 }  // namespace
 
 int cg_persist_residency(const Geom &g, int rep, int device)
@@ -277,6 +593,28 @@ cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0,
     if (P.rep == REP_SU3)
         return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, steps, GaugeD18{(const double2 *)P.U->d64, s}, st);
     return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, steps, GaugeD9{(const double *)P.U->d64, s}, st);
+}
+
+int ms_persist_blocks(const Geom &g, int rep, int device, bool even_odd)
+{
+    if (rep == REP_SU3) return even_odd ? ms_blocks<true, GaugeD18>(g, device) : ms_blocks<false, GaugeD18>(g, device);
+    return even_odd ? ms_blocks<true, GaugeD9>(g, device) : ms_blocks<false, GaugeD9>(g, device);
+}
+
+cudaError_t launch_ms_persist(const DslashParams &P, const void *Ti, bool even_odd, const Spinor &p0, const Spinor &p1,
+                              const Spinor &q, const Spinor &tmp, const void *ring, const void *x, const void *dir,
+                              int nshift, void *state, double *partials, unsigned int *arrived, int *err, int blocks,
+                              int steps, cudaStream_t st)
+{
+    const int s = P.g.stride;
+    auto go = [&](const auto &U) {
+        MultishiftState *ms = (MultishiftState *)state;
+        return even_odd ? run_ms<true>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, blocks,
+                                       steps, U, st)
+                        : run_ms<false>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, blocks,
+                                        steps, U, st);
+    };
+    return P.rep == REP_SU3 ? go(GaugeD18{(const double2 *)P.U->d64, s}) : go(GaugeD9{(const double *)P.U->d64, s});
 }
 
 }  // namespace lym

@@ -418,3 +418,48 @@ def test_fused_square_cg(rep, dims, kind, oracle):
         assert rel(orc.multiply(sols[1]) + 0.3 * sols[1], b) < 1.1e-11
     finally:
         lat.close()
+
+
+@pytest.mark.parametrize("rep,dims,kind", [
+    ("su3", (2, 2, 2, 2), "SquareEvenOddImproved"), ("su2adj", (2, 6, 2, 10), "SquareEvenOddImproved"),
+    ("su3", (2, 2, 2, 2), "SquareDiracWilson"), ("su3", (4, 4, 2, 10), "SquareImproved"),
+    ("su2adj", (4, 4, 4, 6), "SquareImproved"), ("su3", (4, 4, 4, 6), "SquareDiracWilson"),
+    ("su3", (8, 8, 8, 74), "SquareEvenOddImproved"), ("su3", (8, 8, 8, 76), "SquareEvenOddImproved")])
+def test_one_launch_multishift(rep, dims, kind, oracle):
+    """The FP64 multishift in one launch: ragged and single tiles, either side of the size from which
+    its steps are launches again, step counts around the window of 8, more steps than one launch runs."""
+    kappa, csw = (0.12, 1.0) if rep == "su3" else (0.15, 1.2)
+    links = synth.fermion_links(dims, rep, 0.3, 81)
+    lat = L.Lattice(dims, rep)
+    try:
+        op = {"SquareDiracWilson": L.SquareDiracWilsonOperator, "SquareImproved": L.SquareImprovedDiracWilsonOperator,
+              "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind](lat)
+        op.setKappa(kappa)
+        clover = kind != "SquareDiracWilson"
+        if clover:
+            op.setCSW(csw)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, csw if clover else 0.0, True)
+        b = synth.gaussian_spinor(dims, 3, 82)
+        eps = 1e-22 * float(np.vdot(b, b).real)
+        ms = L.MultishiftSolver.getInstance("multishift_cg")
+        ms.setMaxSteps(3000)
+        ms.setPrecision(eps)
+        shifts, sols = [0.3, 0.02, 1e-3, 0.0, 2.0], []
+        assert ms.solve(op, b, sols, shifts)
+        for x, s in zip(sols, shifts):
+            assert rel(orc.multiply(x) + s * x, b) < 5e-11
+        if lat.V > 1000:
+            return
+        # k steps give the base system's k-th CG iterate, whatever the place within a window
+        ms.setPrecision(0.0)
+        for k in (1, 7, 8, 9):
+            ms.setMaxSteps(k)
+            assert not ms.solve(op, b, sols, shifts) and ms.stats.iterations == k
+            assert rel(sols[3], oracle.cg(orc, b, 0.0, k, guess=np.zeros_like(b))[1]) < 1e-11
+        if dims == (4, 4, 4, 6):  # |r|^2 and the shift's zeta stay far from underflow
+            ms.setMaxSteps(530)
+            assert not ms.solve(op, b, sols[:2], [0.0, 1e-6]) and ms.stats.iterations == 530
+            assert rel(orc.multiply(sols[0]), b) < 1e-12
+    finally:
+        lat.close()
