@@ -1776,7 +1776,7 @@ void apply_schur_batch(lym_context *c, const GaugeDev &U, bool clov, int prec, c
 // update with FP32 inner storage, and the fraction (1/n) of busy slots parked for their
 // updates that pauses the batched loop
 #ifndef LYM_BLOCK_DELTA2_F
-#define LYM_BLOCK_DELTA2_F 1e-4
+#define LYM_BLOCK_DELTA2_F 1e-5
 #endif
 #ifndef LYM_BLOCK_PARK_FRACTION
 #define LYM_BLOCK_PARK_FRACTION 8
@@ -2181,7 +2181,9 @@ public:
         memset(&hs, 0, sizeof(hs));
         hs.nb = nb;
         // reliable update when the recursive residual fell by 10x (FP16 inner storage) or
-        // by 100x (FP32, whose rounding drift stays far below that between updates)
+        // by 300x (FP32, whose rounding drift stays far below that between updates: 12 sources at
+        // 24^3 x 48 4-5 updates each instead of 5-6 at 100x, iterations and residuals alike; 1000x
+        // begins to cost iterations at 16^3 x 32, kappa 0.135)
         hs.delta2 = sprec == PREC_H ? 0.01 : LYM_BLOCK_DELTA2_F;
         static_assert(sizeof(BatchCGState) <= kStateBytes, "state buffer too small");
     }
