@@ -1326,7 +1326,9 @@ int shift_cg_mixed(lym_context *c, OpEntry &op, int sprec, double sigma, const S
     H.rr = rr_true;
     H.rr_max = rr_true;
     H.eps = eps;
-    H.delta2 = sprec == PREC_D ? 0.0 : 0.01;
+    // two decades between updates (after one, 12 shifts at 24^3 x 48: 43 updates and 182 ms a
+    // multishift solve, 32 and 175 ms now; the same iterations)
+    H.delta2 = sprec == PREC_D ? 0.0 : 1e-4;
     H.max_iter = iters + max_steps;
     H.iter = iters;
     push_state(c, sizeof(CGState));
@@ -2180,11 +2182,13 @@ public:
         for (BVec *v : {&xs, &rs, &ps, &aps, &tes, &tos}) CK(cudaMemsetAsync(v->s.v, 0, v->bytes, c->st));
         memset(&hs, 0, sizeof(hs));
         hs.nb = nb;
-        // reliable update when the recursive residual fell by 10x (FP16 inner storage) or
-        // by 300x (FP32, whose rounding drift stays far below that between updates: 12 sources at
-        // 24^3 x 48 4-5 updates each instead of 5-6 at 100x, iterations and residuals alike; 1000x
-        // begins to cost iterations at 16^3 x 32, kappa 0.135)
-        hs.delta2 = sprec == PREC_H ? 0.01 : LYM_BLOCK_DELTA2_F;
+        // Reliable update when the recursive residual fell by 100x (FP16 inner storage; the residual
+        // is FP32) or 300x (FP32): the rounding drift of the recursion stays below that.  FP32, 12
+        // sources at 24^3 x 48: 4-5 updates each against 5-6 at 100x, iterations and residuals
+        // alike; 1000x begins to cost iterations at 16^3 x 32, kappa 0.135.  FP16, 12 sources at
+        // 16^3 x 32: 5 updates against 9 at 10x, iterations alike, 34 against 42 ms at kappa 0.12
+        // and 66 against 76 at 0.135; 300x costs iterations there (67.6 ms).
+        hs.delta2 = sprec == PREC_H ? 1e-4 : LYM_BLOCK_DELTA2_F;
         static_assert(sizeof(BatchCGState) <= kStateBytes, "state buffer too small");
     }
     ~BlockEngine()
