@@ -1227,8 +1227,16 @@ __global__ void __launch_bounds__(kStagedThreads, MINB)
 // one pair (the grid stride is a multiple of np), its FP64 partial sums are per RHS,
 // acc[lane * NRED + k], and the last block runs Op::finalize(r, totals) for every r in
 // parallel (thread r), then Op::finalize_all().
+// Blocks per SM that the kernel's registers must leave room for: Op::kMinBlocks, 0 (the compiler's
+// choice) without one.
+template <class Op, class = void> struct BatchMinBlocks {
+    static constexpr int value = 0;
+};
+template <class Op> struct BatchMinBlocks<Op, decltype((void)Op::kMinBlocks)> {
+    static constexpr int value = Op::kMinBlocks;
+};
 template <class Op>
-__global__ void __launch_bounds__(kBlasThreads) site_batch_kernel(Op op, int vh, int lognp, double *partials,
+__global__ void __launch_bounds__(kBlasThreads, BatchMinBlocks<Op>::value) site_batch_kernel(Op op, int vh, int lognp, double *partials,
                                                                   unsigned int *counter, Gate gate)
 {
     static_assert(Op::NRED <= kBatchMaxRed, "partials hold kBatchMaxRed sums per (block, RHS)");
@@ -1573,6 +1581,9 @@ template <class ST, class SS, class SRh> struct OpBBOmega {
 // known now: alpha_r = rho_r / <what_r, p_r>), and the convergence / reliable-update decisions
 template <class SX, class SP, class SS, class ST, class SV, class SR, class SW> struct OpBBUpdate {
     static constexpr int NRED = 3;
+    // FP16 directions: 156 registers otherwise, one block per SM (14 x 10 x 12 x 22, 8 sources, 289
+    // blocks: 25.6 us in two waves, 17.1 in one); FP32 has 128 by itself
+    static constexpr int kMinBlocks = std::is_same<SP, BatchH>::value ? 2 : 0;
     SX x;
     SP p;
     SS sv;
