@@ -579,8 +579,9 @@ def run_ours(args, world, rank, local):
     lib.lym_time_stencil(ctx, opid, 1, 0, 30, C.byref(ms8))
     lib.lym_set_link_format(ctx, 12)
 
+    from oracle import ref as R
     cpu = None
-    if rank == 0 and world == 1 and not args.skip_cpu:
+    if rank == 0 and world == 1 and not args.skip_cpu and R.available("su3"):  # null where it is not built
         ref = ReferenceCPU()
         try:
             full = ref.full_solve()
