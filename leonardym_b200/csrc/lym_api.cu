@@ -1221,6 +1221,11 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     copy(c, pb, b);
     const MsViews<SpinorD> views(c, hring, hx, hp);
     const double bb = norm2_now(c, b);
+    if (!std::isfinite(bb)) {
+        c->err = "the source has non-finite entries";
+        if (st) st->last_error = bb;
+        return LYM_NOT_CONVERGED;
+    }
     // build the clover term and pool the operator's temporaries before graph capture
     op_apply(c, op, PREC_D, *ap, b, &b, C2(s0));
     MultishiftState &H = *(MultishiftState *)c->h_state;
@@ -1277,6 +1282,7 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
             run_gated_state(c, S, step, kMsWin, max_steps);
         }
         MultishiftState &R = *(MultishiftState *)c->h_state;
+        if (R.failed) c->err = "multishift CG produced a non-finite residual";  // xs: the iterates before it
         rc = R.converged ? LYM_OK : LYM_NOT_CONVERGED;
         if (st) {
             st->iterations = R.iter;

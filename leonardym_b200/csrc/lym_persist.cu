@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const Pers
         ms_residual_step(&st, rr);
         __syncthreads();
         if (st.win < kMsWin && !st.stop) return;
-        const int m = st.failed ? 0 : st.win, k0 = st.iter - m, words = 2 * 12 * g.stride;
+        const int m = st.win, k0 = ms_window_start(&st), words = 2 * 12 * g.stride;
         for (int o = blockIdx.x * kSplitThreads + threadIdx.x; m > 0 && o < words; o += gridDim.x * kSplitThreads) {
             double2 R[kMsWin];
 #pragma unroll
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const Pers
 #pragma unroll
                 for (int j = 0; j < kMsWin; ++j)
                     if (j < m) {
-                        word_add(X, st.cx[i][j + 1], R[j]);
+                        if (j < m - 1) word_add(X, st.cx[i][j + 1], R[j]);  // the last one is not in x yet
                         word_add(Q, st.cp[i][j + 1], R[j]);
                     }
                 *xp = X;

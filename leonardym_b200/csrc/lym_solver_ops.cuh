@@ -644,6 +644,10 @@ LYM_D void ms_residual_step(MultishiftState *s, double rr_new)
     if (!any || update || iter >= s->max_iter) s->stop = 1;
 }
 
+// k0 of the window's residuals R_j = r_{k0+1+j}, j < win: a residual that is not finite was counted
+// as a step but is not in the window
+LYM_D int ms_window_start(const MultishiftState *s) { return s->iter - s->win - (s->failed ? 1 : 0); }
+
 // r_{k+1} = r_k - alpha Ap with the residuals in a ring of kMsWin + 1 slots (r_k in slot
 // k mod (kMsWin + 1)), |r_{k+1}|^2, then the step's scalars and window coefficients.
 template <class SR, class SAp> struct OpMsResidualRing {
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(kMsFlushThreads) ms_flush_kernel(MsFlushArg<Vi
     const MultishiftState *s = a.s;
     const int m = s->win;
     if (m == 0) return;
-    const int k0 = s->iter - m;
+    const int k0 = ms_window_start(s);
     for (int t = threadIdx.x; t < a.nshift * (kMsWin + 1); t += blockDim.x) {
         const int i = t / (kMsWin + 1), j = t % (kMsWin + 1);
         cxs[i][j] = (R)s->cx[i][j];
@@ -758,7 +762,7 @@ __global__ void __launch_bounds__(kMsFlushThreads) ms_flush_kernel(MsFlushArg<Vi
 #pragma unroll
             for (int j = 0; j < kMsWin; ++j) {
                 if (j < m) {
-                    word_add(X, cxs[i][j + 1], Rj[j]);
+                    if (j < m - 1) word_add(X, cxs[i][j + 1], Rj[j]);  // the last one has not entered x yet
                     word_add(Q, cps[i][j + 1], Rj[j]);
                 }
             }

@@ -152,6 +152,64 @@ def test_block_solve_nonfinite_source_fails_alone(su3, algo):
         assert s.block_stats[k].converged == 1 and r <= 1e-10, (k, r)
 
 
+# V = 37888 sites and less: the FP64 multishift runs in one launch, above: launches per step
+MULTISHIFT = [((4, 4, 4, 6), "SquareEvenOddImproved"), ((4, 4, 4, 6), "SquareImproved"),
+              ((8, 8, 8, 76), "SquareEvenOddImproved"), ((8, 8, 8, 76), "SquareImproved")]
+
+
+def _multishift(dims, kind, kappa, oracle):
+    links = synth.fermion_links(dims, "su3", 0.3, 81)
+    lat = L.Lattice(dims, "su3")
+    op = {"SquareImproved": L.SquareImprovedDiracWilsonOperator,
+          "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind](lat, kappa, 1.0)
+    op.setLattice(lat.upload(links))
+    return lat, op, oracle.Operator(oracle.Geometry(dims), links, kind, kappa, 1.0, True)
+
+
+@pytest.mark.parametrize("dims,kind", MULTISHIFT)
+def test_multishift_residual_turns_nonfinite(dims, kind, oracle):
+    """Tiny sources and no threshold: |r|^2 underflows to zero and the step after it divides zero
+    by zero, at another place of the window of 8 steps for every scale.  The solutions are the last
+    finite iterates, by then solved to rounding (a window's updates left out: 1e-11 to 1e-4)."""
+    lat, op, orc = _multishift(dims, kind, 0.03, oracle)
+    try:
+        b = synth.gaussian_spinor(dims, 3, 82)
+        ms = L.MultishiftSolver.getInstance("multishift_cg")
+        ms.setPrecision(0.0)
+        scale = np.sqrt(float(np.vdot(b, b).real) / 4608.0)  # |b| as on 4^3 x 6
+        for e in (-149.5, -148.5, -147.5, -146.5):
+            v, sols = b * (10.0 ** e / scale), []
+            assert not ms.solve(op, v, sols, [0.0, 1e-6])
+            assert ms.stats.iterations < 80 and not ms.stats.converged
+            for x, s in zip(sols, (0.0, 1e-6)):
+                assert np.all(np.isfinite(x))
+                y = x / 10.0 ** e
+                r = orc.multiply(y) + s * y - b / scale
+                assert np.linalg.norm(r) <= 1e-12 * np.linalg.norm(b / scale), (e, s)
+            assert b"non-finite" in L.lib().lym_last_error(lat.handle)
+    finally:
+        lat.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("dims,kind", MULTISHIFT)
+def test_multishift_nonfinite_source_is_not_converged(dims, kind, bad, oracle):
+    lat, op, orc = _multishift(dims, kind, 0.1, oracle)
+    try:
+        b = synth.gaussian_spinor(dims, 3, 83)
+        v = b.copy()
+        v[17, 2, 1] = bad
+        ms, sols = L.MultishiftSolver.getInstance("multishift_cg"), []
+        assert not ms.solve(op, v, sols, [0.0, 0.1])
+        assert b"non-finite" in L.lib().lym_last_error(lat.handle) and not ms.stats.converged
+        assert not np.any(sols[0]) and not np.any(sols[1])
+        ms.setPrecision(1e-22 * float(np.vdot(b, b).real))
+        assert ms.solve(op, b, sols, [0.0, 0.1])  # the context goes on
+        assert np.linalg.norm(orc.multiply(sols[0]) - b) <= 2e-11 * np.linalg.norm(b)
+    finally:
+        lat.close()
+
+
 def _residual(D, b, x):
     return np.linalg.norm(b - D.multiply(x)) / np.linalg.norm(b)
 
