@@ -772,6 +772,14 @@ DslashParams square_half_params(lym_context *c, OpEntry &op, const Spinor &q, co
     return P;
 }
 
+// Held around a one-launch solver's launch: two grids that each wait for all their blocks must not
+// share a GPU's block slots.
+std::mutex &one_launch_lock(int device)
+{
+    static std::mutex locks[64];
+    return locks[device & 63];
+}
+
 // Cooperative launches go(steps, err) of at most `kOneLaunchSteps` iterations each, until the state
 // pauses.
 template <class S, class Go> void run_one_launch(lym_context *c, int max_steps, Go go, S *state)
@@ -779,11 +787,8 @@ template <class S, class Go> void run_one_launch(lym_context *c, int max_steps, 
     constexpr int kOneLaunchSteps = 512;  // bounds a launch to some ms
     int *err = c->d_err + 2;
     CK(cudaMemsetAsync(err, 0, sizeof(int), c->st));
-    // one such launch at a time in the process: two grids that each wait for all their blocks must
-    // not share the GPU's block slots
-    static std::mutex one_launch;
     for (long done = 0; done < (long)max_steps + kOneLaunchSteps; done += kOneLaunchSteps) {
-        std::lock_guard<std::mutex> lock(one_launch);
+        std::lock_guard<std::mutex> lock(one_launch_lock(c->device));
         CK(go(kOneLaunchSteps, err));
         count(c, 1);
         CK(cudaMemcpyAsync(c->h_scal, err, sizeof(int), cudaMemcpyDeviceToHost, c->st));

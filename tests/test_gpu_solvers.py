@@ -463,3 +463,57 @@ def test_one_launch_multishift(rep, dims, kind, oracle):
             assert rel(orc.multiply(sols[0]), b) < 1e-12
     finally:
         lat.close()
+
+
+def test_one_launch_solvers_of_two_threads(oracle):
+    """A CG and a multishift, each in one launch and on a context of its own, from two threads at
+    once: their grids would not fit on the GPU together, so they take turns."""
+    import threading
+
+    kappa, csw = 0.12, 1.0
+    jobs, errors = [], []
+    for dims, kind, cls in (((8, 8, 8, 8), "SquareImproved", L.SquareImprovedDiracWilsonOperator),
+                            ((8, 8, 8, 74), "SquareEvenOddImproved", L.SquareEvenOddImprovedDiracWilsonOperator)):
+        links = synth.fermion_links(dims, "su3", 0.3, 91)
+        lat = L.Lattice(dims, "su3")
+        op = cls(lat, kappa, csw)
+        op.setLattice(lat.upload(links))
+        b = synth.gaussian_spinor(dims, 3, 92)
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, csw, True)
+        jobs.append((lat, op, b, orc, 1e-22 * float(np.vdot(b, b).real)))
+    (lat_a, op_a, b_a, orc_a, eps_a), (lat_b, op_b, b_b, orc_b, eps_b) = jobs
+    x, sols = lat_a.new_vector(), []
+
+    def run_cg():
+        cg = L.ConjugateGradient()
+        cg.setPrecision(eps_a)
+        for _ in range(40):
+            if not cg.solve(op_a, b_a, x):
+                errors.append("cg")
+
+    def run_multishift():
+        ms = L.MultishiftSolver.getInstance("multishift_cg")
+        ms.setPrecision(eps_b)
+        for _ in range(6):
+            if not ms.solve(op_b, b_b, sols, [0.0, 0.3]):
+                errors.append("multishift")
+
+    def guarded(f):
+        try:
+            f()
+        except Exception as e:  # an error of the thread fails the test
+            errors.append(e)
+
+    try:
+        threads = [threading.Thread(target=guarded, args=(f,)) for f in (run_cg, run_multishift)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors
+        assert rel(orc_a.multiply(x), b_a) < 1.1e-11
+        for y, s in zip(sols, (0.0, 0.3)):
+            assert rel(orc_b.multiply(y) + s * y, b_b) < 5e-11
+    finally:
+        lat_a.close()
+        lat_b.close()
