@@ -448,6 +448,11 @@ int lym_set_link_format(lym_context *ctx, int reals);
  * involved.  A server lane fails only the request whose admission met the failure. */
 int lym_context_inject_alloc_failures(lym_context *ctx, int n);
 int lym_server_inject_alloc_failures(lym_server *server, int key, int n);
+/* The waits between the blocks of the next n one-launch solves (CG and FP64 multishift on small
+ * lattices) look for one arrival more than there are and give up after a thousand looks (tens of
+ * microseconds): the kernel ends with its error word set, and the solve runs again with launches
+ * per iteration. */
+int lym_context_inject_one_launch_give_ups(lym_context *ctx, int n);
 /* The next host check of the word in which the bulk-copy variant of the batched stencil
  * (lym_set_batch_tile codes 35, 36) records a copy wait that gave up reads it as set: the
  * call that ran the variant returns LYM_ERR_TIMEOUT and the word is cleared.  The kernels

@@ -90,6 +90,7 @@ struct lym_context {
     double engine_stats[9] = {};      // block solves: lym_context_engine_stats
     bool capturing = false;
     int inject_alloc_failures = 0;  // the next n device allocations report failure (tests)
+    int inject_give_ups = 0;        // the next n one-launch solves' waits run out (tests)
     bool inject_copy_wait = false;  // the next check of the bulk-copy wait word reports a give-up (tests)
     int link_reals = 12;            // FP32 SU(3) link format of the single-RHS stencils: 12 or 8
     int persist = 0;                // blocks per SM of the one-launch CG (lym_persist.cu), 0: not fitting
@@ -780,39 +781,51 @@ std::mutex &one_launch_lock(int device)
     return locks[device & 63];
 }
 
-// Cooperative launches go(steps, err) of at most `kOneLaunchSteps` iterations each, until the state
-// pauses.
-template <class S, class Go> void run_one_launch(lym_context *c, int max_steps, Go go, S *state)
+// Cooperative launches go(steps, wait, err) of at most `kOneLaunchSteps` iterations each, until the
+// state pauses.  False when the launch was refused or a wait between its blocks gave up (blocks that
+// found no place for about a second beside other work on the GPU): the caller then solves from the
+// start with launches per iteration.
+template <class S, class Go> bool run_one_launch(lym_context *c, int max_steps, Go go, S *state)
 {
     constexpr int kOneLaunchSteps = 512;  // bounds a launch to some ms
     int *err = c->d_err + 2;
+    BarrierWait wait;
+    if (c->inject_give_ups > 0) {  // lym_context_inject_one_launch_give_ups
+        --c->inject_give_ups;
+        wait.polls = 1 << 10;
+        wait.extra = 1;
+    }
     CK(cudaMemsetAsync(err, 0, sizeof(int), c->st));
     for (long done = 0; done < (long)max_steps + kOneLaunchSteps; done += kOneLaunchSteps) {
         std::lock_guard<std::mutex> lock(one_launch_lock(c->device));
-        CK(go(kOneLaunchSteps, err));
+        if (go(kOneLaunchSteps, wait, err) != cudaSuccess) {
+            cudaGetLastError();  // a lasting error meets the launches that follow
+            return false;
+        }
         count(c, 1);
         CK(cudaMemcpyAsync(c->h_scal, err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
         CK(cudaMemcpyAsync(c->h_state, state, sizeof(S), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
         int e = 0;
         memcpy(&e, c->h_scal, sizeof(int));
-        if (e) fail(c, LYM_ERR_TIMEOUT, "a wait between the blocks of a one-launch solver gave up");
-        if (state_paused(*(S *)c->h_state)) return;
+        if (e) return false;
+        if (state_paused(*(S *)c->h_state)) return true;
     }
-    fail(c, LYM_ERR_TIMEOUT, "solver state did not stop within %d iterations", max_steps);
+    return false;
 }
 
 // The iterations of a CG on A = op + sigma (op a squared kind on full spinors) whose state, x, r
-// and scratch p, q are set up.
-void persist_cg(lym_context *c, OpEntry &op, double sigma, const Spinor &x, const Spinor &r, const Spinor &p,
+// and scratch p, q are set up; false as run_one_launch.
+bool persist_cg(lym_context *c, OpEntry &op, double sigma, const Spinor &x, const Spinor &r, const Spinor &p,
                 const Spinor &q, int max_steps)
 {
     DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
     P.sigma = sigma;
     Vec p1(c, PREC_D, 2);
     CGState *S = cg_state(c);
-    run_one_launch(c, max_steps, [&](int steps, int *err) {
-        return launch_cg_persist(P, c->persist, p, *p1, x, r, q, S, c->spartials, c->counter + 8, err, steps, c->st);
+    return run_one_launch(c, max_steps, [&](int steps, BarrierWait wait, int *err) {
+        return launch_cg_persist(P, c->persist, p, *p1, x, r, q, S, c->spartials, c->counter + 8, err, wait, steps,
+                                 c->st);
     }, S);
 }
 
@@ -828,19 +841,22 @@ int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const 
     if (square && is_even_odd(square->kind)) te.reset(new Vec(c, PREC_D, 1));
     const Spinor half = te ? **te : Spinor();
     Vec r(c, PREC_D, nparity), p(c, PREC_D, nparity), ap(c, PREC_D, nparity);
-    copy(c, x, guess ? *guess : b);
-    matvec(*ap, x, nullptr);
-    run_site(c, OpSubNorm<SpinorD, SpinorD, SpinorD>{b.d(), (*ap).d(), (*r).d(), c->d_scal}, nparity);
-    copy(c, *p, *r);
-    CK(cudaMemcpyAsync(c->h_scal, c->d_scal, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    CGState &H = cg_host(c);
-    memset(&H, 0, sizeof(H));
-    H.rr = c->h_scal[0];
-    H.rr_max = H.rr;
-    H.eps = eps;
-    H.max_iter = max_steps;
-    push_state(c, sizeof(CGState));
+    auto start = [&]() {
+        copy(c, x, guess ? *guess : b);
+        matvec(*ap, x, nullptr);
+        run_site(c, OpSubNorm<SpinorD, SpinorD, SpinorD>{b.d(), (*ap).d(), (*r).d(), c->d_scal}, nparity);
+        copy(c, *p, *r);
+        CK(cudaMemcpyAsync(c->h_scal, c->d_scal, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        CGState &H = cg_host(c);
+        memset(&H, 0, sizeof(H));
+        H.rr = c->h_scal[0];
+        H.rr_max = H.rr;
+        H.eps = eps;
+        H.max_iter = max_steps;
+        push_state(c, sizeof(CGState));
+    };
+    start();
     CGState *S = cg_state(c);
     Gate gate{&S->pause, nullptr};
     auto step = [&]() {
@@ -859,9 +875,15 @@ int cg_solve(lym_context *c, MatVec matvec, int nparity, const Spinor &b, const 
         }
         run_site(c, OpCGDirection<SpinorD, SpinorD>{(*p).d(), (*r).d(), S}, nparity, gate);
     };
-    if (max_steps <= 0) pull_state(c, sizeof(CGState));
-    else if (square && c->persist && !is_even_odd(square->kind)) persist_cg(c, *square, sigma, x, *r, *p, *ap, max_steps);
-    else run_gated_state(c, S, step, 8, max_steps);
+    if (max_steps <= 0) {
+        pull_state(c, sizeof(CGState));
+    } else {
+        const bool one_launch = square && c->persist && !is_even_odd(square->kind);
+        if (!one_launch || !persist_cg(c, *square, sigma, x, *r, *p, *ap, max_steps)) {
+            if (one_launch) start();
+            run_gated_state(c, S, step, 8, max_steps);
+        }
+    }
     CGState &R = cg_host(c);
     if (st) {
         st->converged = R.converged;
@@ -1205,17 +1227,12 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
         return **owned.back();
     };
     std::vector<SpinorD> hring, hx, hp;
-    for (int j = 0; j <= kMsWin; ++j) {
-        const Spinor r = fresh();
-        if (j == 0) copy(c, r, b);  // r_0 = b
-        hring.push_back(r.d());
-    }
+    for (int j = 0; j <= kMsWin; ++j) hring.push_back(fresh().d());
+    const Spinor r0 = **owned[0];
     for (int i = 0; i < nshift; ++i) {
-        const Spinor p = fresh();
         zero(c, xs[i]);
-        copy(c, p, b);
         hx.push_back(xs[i].d());
-        hp.push_back(p.d());
+        hp.push_back(fresh().d());
     }
     // the base direction of the current step (the operator's input), and A p or Q p
     Vec pcur(c, PREC_D, 2), ap(c, PREC_D, 2);
@@ -1223,7 +1240,6 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     if (square && is_even_odd(op.kind)) te.reset(new Vec(c, PREC_D, 1));
     const Spinor half = te ? **te : Spinor();
     const Spinor pb = *pcur;
-    copy(c, pb, b);
     const MsViews<SpinorD> views(c, hring, hx, hp);
     const double bb = norm2_now(c, b);
     if (!std::isfinite(bb)) {
@@ -1233,22 +1249,31 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     }
     // build the clover term and pool the operator's temporaries before graph capture
     op_apply(c, op, PREC_D, *ap, b, &b, C2(s0));
-    MultishiftState &H = *(MultishiftState *)c->h_state;
-    memset(&H, 0, sizeof(H));
-    H.nshift = nshift;
-    H.base = base;
-    for (int i = 0; i < nshift; ++i) {
-        H.sigma[i] = shifts[i] - s0;
-        H.zeta[i] = H.zeta_prev[i] = 1.0;
-        H.active[i] = 1;
-        H.cp[i][0] = 1.0;
-    }
-    H.rr = bb;
-    H.alpha = 1.0;
-    H.beta = 0.0;
-    H.eps = eps;
-    H.max_iter = max_steps;
-    CK(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(MultishiftState), cudaMemcpyHostToDevice, c->st));
+    auto start = [&]() {  // x_i = 0, r_0 = p_i = b
+        copy(c, r0, b);
+        copy(c, pb, b);
+        for (int i = 0; i < nshift; ++i) {
+            zero(c, xs[i]);
+            copy(c, **owned[kMsWin + 1 + i], b);
+        }
+        MultishiftState &H = *(MultishiftState *)c->h_state;
+        memset(&H, 0, sizeof(H));
+        H.nshift = nshift;
+        H.base = base;
+        for (int i = 0; i < nshift; ++i) {
+            H.sigma[i] = shifts[i] - s0;
+            H.zeta[i] = H.zeta_prev[i] = 1.0;
+            H.active[i] = 1;
+            H.cp[i][0] = 1.0;
+        }
+        H.rr = bb;
+        H.alpha = 1.0;
+        H.beta = 0.0;
+        H.eps = eps;
+        H.max_iter = max_steps;
+        CK(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(MultishiftState), cudaMemcpyHostToDevice, c->st));
+    };
+    start();
     MultishiftState *S = (MultishiftState *)c->d_state;
     Gate gate{&S->pause, nullptr};
     int nstep = 0;
@@ -1272,6 +1297,7 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     const bool eo = is_even_odd(op.kind);
     const int blocks = square ? ms_persist_blocks(c->g, c->rep, c->device, eo) : 0;
     if (bb > 0 && max_steps > 0) {
+        bool done = false;
         if (blocks > 0) {
             DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
             P.sigma = s0;
@@ -1279,13 +1305,13 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
             const void *Ti = eo && kind_has_clover(op.kind) ? op.clover.Tinv[PREC_D] : nullptr;
             Vec p1(c, PREC_D, 2);
             DevBuf sums(c, 2 * (size_t)blocks * sizeof(double), false);
-            run_one_launch(c, max_steps, [&](int steps, int *err) {
+            done = run_one_launch(c, max_steps, [&](int steps, BarrierWait wait, int *err) {
                 return launch_ms_persist(P, Ti, eo, pb, *p1, *ap, half, views.ring, views.x, views.p, nshift, S,
-                                         (double *)sums.p, c->counter + 8, err, blocks, steps, c->st);
+                                         (double *)sums.p, c->counter + 8, err, wait, blocks, steps, c->st);
             }, S);
-        } else {
-            run_gated_state(c, S, step, kMsWin, max_steps);
+            if (!done) start();
         }
+        if (!done) run_gated_state(c, S, step, kMsWin, max_steps);
         MultishiftState &R = *(MultishiftState *)c->h_state;
         if (R.failed) c->err = "multishift CG produced a non-finite residual";  // xs: the iterates before it
         rc = R.converged ? LYM_OK : LYM_NOT_CONVERGED;
@@ -4253,6 +4279,15 @@ int lym_context_inject_alloc_failures(lym_context *c, int n)
     if (n < 0) return LYM_ERR_ARGUMENT;
     return guarded(c, [&]() {
         c->inject_alloc_failures = n;
+        return LYM_OK;
+    });
+}
+
+int lym_context_inject_one_launch_give_ups(lym_context *c, int n)
+{
+    if (n < 0) return LYM_ERR_ARGUMENT;
+    return guarded(c, [&]() {
+        c->inject_give_ups = n;
         return LYM_OK;
     });
 }

@@ -98,6 +98,13 @@ void launch_split_cg(const DslashParams &P, int mode, const Spinor &p, const Spi
 void launch_split_ms(const DslashParams &P, int mode, const Spinor &p, const void *ring, void *state, double *partials,
                      unsigned int *counter, cudaStream_t st);
 int split_partials(const Geom &g);
+// A wait of a one-launch solver between its blocks: it gives up after `polls` looks at the arrivals
+// (about a second by default).  extra: arrivals asked for beyond those that come, so that a test's
+// wait runs out.
+struct BarrierWait {
+    int polls = 1 << 21;
+    unsigned int extra = 0;
+};
 // CG on Q Q + sigma over both parities in one cooperative launch of at most `steps` iterations
 // (lym_persist.cu), where the lattice's blocks are all resident at once (cg_persist_residency
 // not 0: the argument minb).
@@ -108,7 +115,7 @@ int cg_persist_residency(const Geom &g, int rep, int device);
 int cg_persist_partials(const Geom &g);
 cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0, const Spinor &p1, const Spinor &x,
                               const Spinor &r, const Spinor &q, void *state, double *partials, unsigned int *arrived,
-                              int *err, int steps, cudaStream_t st);
+                              int *err, BarrierWait wait, int steps, cudaStream_t st);
 // The FP64 multishift CG likewise: P the operator's second (or only) stencil with the base shift,
 // Ti T^-1 of the even-odd kind (both null without clover); p0, p1, q: scratch full spinors, tmp: a
 // half spinor (even-odd); ring, x, dir: device arrays of SpinorD views; blocks:
@@ -116,8 +123,8 @@ cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0,
 int ms_persist_blocks(const Geom &g, int rep, int device, bool even_odd);
 cudaError_t launch_ms_persist(const DslashParams &P, const void *Ti, bool even_odd, const Spinor &p0, const Spinor &p1,
                               const Spinor &q, const Spinor &tmp, const void *ring, const void *x, const void *dir,
-                              int nshift, void *state, double *partials, unsigned int *arrived, int *err, int blocks,
-                              int steps, cudaStream_t st);
+                              int nshift, void *state, double *partials, unsigned int *arrived, int *err,
+                              BarrierWait wait, int blocks, int steps, cudaStream_t st);
 void launch_clover(const Geom &g, int prec, const Spinor &out, const Spinor &in, const void *clover, int parity,
                    int gamma5, cudaStream_t st);
 void launch_pack(const Geom &g, const double *aos, const Spinor &full, cudaStream_t st);

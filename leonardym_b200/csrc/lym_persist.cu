@@ -34,6 +34,7 @@ template <class GaugeT> struct PersistArg {
     double *partials;       // 2 * gridDim.x
     unsigned int *arrived;  // zero at the launch
     int *err;               // set to 1 when a barrier wait gave up
+    BarrierWait wait;
     int steps;              // iterations of this launch at most
 };
 
@@ -53,12 +54,12 @@ LYM_D void grid_arrive(unsigned int *arrived)
         atomicAdd(arrived, 1u);
     }
 }
-// target: arrivals expected so far.  The wait is bounded, about a second; false when it ran out.
-LYM_D bool grid_wait(unsigned int *arrived, unsigned int target, bool *ok)
+// target: arrivals expected so far.  The wait is bounded; false when it ran out.
+LYM_D bool grid_wait(unsigned int *arrived, unsigned int target, int polls, bool *ok)
 {
     if (threadIdx.x == 0) {
         bool done = false;
-        for (int i = 0; i < (1 << 21); ++i) {
+        for (int i = 0; i < polls; ++i) {
             unsigned int v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(arrived) : "memory");
             if (v >= target) {
@@ -72,10 +73,10 @@ LYM_D bool grid_wait(unsigned int *arrived, unsigned int target, bool *ok)
     __syncthreads();
     return *ok;
 }
-LYM_D bool grid_barrier(unsigned int *arrived, unsigned int target, bool *ok)
+LYM_D bool grid_barrier(unsigned int *arrived, unsigned int target, int polls, bool *ok)
 {
     grid_arrive(arrived);
-    return grid_wait(arrived, target, ok);
+    return grid_wait(arrived, target, polls, ok);
 }
 
 template <int MINB, class GaugeT>
@@ -141,13 +142,13 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) cg_persist_kernel(const P
         __syncthreads();
         return (wsum[slot][0] + wsum[slot][1]) + (wsum[slot][2] + wsum[slot][3]);
     };
-    unsigned int target = 0;
+    unsigned int target = a.wait.extra;
     // the block's part of a sum, then the barrier; false when it gave up
     auto contribute = [&](double v, int half) {
         const double t = block_total(in ? v : 0.0, 0);
         if (threadIdx.x == 0) a.partials[(size_t)half * gridDim.x + blockIdx.x] = t;
         target += gridDim.x;
-        return grid_barrier(a.arrived, target, &ok);
+        return grid_barrier(a.arrived, target, a.wait.polls, &ok);
     };
     // this thread's share of the blocks' parts (their sum over the block is the grid's)
     auto collect = [&](int half) {
@@ -218,8 +219,9 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) cg_persist_kernel(const P
         put(xv, m, C{x.x, x.y});
     }
     if (threadIdx.x == 0) {
-        if (!good) atomicOr(a.err, 1);
-        if (blockIdx.x == 0) {
+        if (!good) {  // the host starts the solve again with launches per iteration
+            atomicOr(a.err, 1);
+        } else if (blockIdx.x == 0) {
             CGState out = st;
             out.iter = it;
             out.rr = rr;
@@ -258,11 +260,11 @@ template <class GaugeT> int residency(const Geom &g, int device)
 
 template <class GaugeT>
 cudaError_t run(const DslashParams &P, int minb, const Spinor &p0, const Spinor &p1, const Spinor &x, const Spinor &r,
-                const Spinor &q, CGState *state, double *partials, unsigned int *arrived, int *err, int steps,
-                const GaugeT &U, cudaStream_t st)
+                const Spinor &q, CGState *state, double *partials, unsigned int *arrived, int *err, BarrierWait wait,
+                int steps, const GaugeT &U, cudaStream_t st)
 {
-    PersistArg<GaugeT> a{P.g,     U,       (const double2 *)P.clover, P.b,   P.sigma, x.d(), r.d(), q.d(), {p0.d(), p1.d()},
-                         state, partials, arrived,                   err, steps};
+    PersistArg<GaugeT> a{P.g,   U,     (const double2 *)P.clover, P.b,     P.sigma, x.d(), r.d(), q.d(), {p0.d(), p1.d()},
+                         state, partials, arrived,                   err,     wait,    steps};
     const cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
@@ -295,6 +297,7 @@ template <class GaugeT> struct PersistMsArg {
     double *partials;               // 2 * gridDim.x
     unsigned int *arrived;
     int *err;
+    BarrierWait wait;
     int nshift, steps;
 };
 
@@ -322,12 +325,12 @@ __global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const Pers
         __syncthreads();
         return (wsum[slot][0] + wsum[slot][1]) + (wsum[slot][2] + wsum[slot][3]);
     };
-    unsigned int target = 0;
+    unsigned int target = a.wait.extra;
     auto arrive = [&]() {
         target += gridDim.x;
         grid_arrive(a.arrived);
     };
-    auto wait = [&]() { return grid_wait(a.arrived, target, &ok); };
+    auto wait = [&]() { return grid_wait(a.arrived, target, a.wait.polls, &ok); };
     // the block's part of a sum, then the barrier's first half
     auto contribute = [&](double v, int half) {
         const double t = block_total(v, 0);
@@ -524,7 +527,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const Pers
     __syncthreads();
     if (good && pending) settle();
     if (threadIdx.x == 0 && !good) atomicOr(a.err, 1);
-    if (blockIdx.x == 0)
+    if (blockIdx.x == 0 && good)
         for (int i = threadIdx.x; i < (int)(sizeof(st) / sizeof(int)); i += kSplitThreads)
             reinterpret_cast<int *>(a.state)[i] = reinterpret_cast<const int *>(&st)[i];
 }
@@ -532,8 +535,8 @@ __global__ void __launch_bounds__(kSplitThreads, 4) ms_persist_kernel(const Pers
 template <bool EO, class GaugeT>
 cudaError_t run_ms(const DslashParams &P, const void *Ti, const Spinor &p0, const Spinor &p1, const Spinor &q,
                    const Spinor &tmp, const void *ring, const void *x, const void *dir, int nshift,
-                   MultishiftState *state, double *partials, unsigned int *arrived, int *err, int blocks, int steps,
-                   const GaugeT &U, cudaStream_t st)
+                   MultishiftState *state, double *partials, unsigned int *arrived, int *err, BarrierWait wait,
+                   int blocks, int steps, const GaugeT &U, cudaStream_t st)
 {
     PersistMsArg<GaugeT> a{P.g,
                            U,
@@ -551,6 +554,7 @@ cudaError_t run_ms(const DslashParams &P, const void *Ti, const Spinor &p0, cons
                            partials,
                            arrived,
                            err,
+                           wait,
                            nshift,
                            steps};
     const cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), st);
@@ -586,13 +590,14 @@ int cg_persist_partials(const Geom &g) { return 2 * persist_blocks(g); }
 
 cudaError_t launch_cg_persist(const DslashParams &P, int minb, const Spinor &p0, const Spinor &p1, const Spinor &x,
                               const Spinor &r, const Spinor &q, void *state, double *partials, unsigned int *arrived,
-                              int *err, int steps, cudaStream_t st)
+                              int *err, BarrierWait wait, int steps, cudaStream_t st)
 {
     const int s = P.g.stride;
     CGState *cs = (CGState *)state;
     if (P.rep == REP_SU3)
-        return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, steps, GaugeD18{(const double2 *)P.U->d64, s}, st);
-    return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, steps, GaugeD9{(const double *)P.U->d64, s}, st);
+        return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, wait, steps,
+                   GaugeD18{(const double2 *)P.U->d64, s}, st);
+    return run(P, minb, p0, p1, x, r, q, cs, partials, arrived, err, wait, steps, GaugeD9{(const double *)P.U->d64, s}, st);
 }
 
 int ms_persist_blocks(const Geom &g, int rep, int device, bool even_odd)
@@ -603,16 +608,16 @@ int ms_persist_blocks(const Geom &g, int rep, int device, bool even_odd)
 
 cudaError_t launch_ms_persist(const DslashParams &P, const void *Ti, bool even_odd, const Spinor &p0, const Spinor &p1,
                               const Spinor &q, const Spinor &tmp, const void *ring, const void *x, const void *dir,
-                              int nshift, void *state, double *partials, unsigned int *arrived, int *err, int blocks,
-                              int steps, cudaStream_t st)
+                              int nshift, void *state, double *partials, unsigned int *arrived, int *err,
+                              BarrierWait wait, int blocks, int steps, cudaStream_t st)
 {
     const int s = P.g.stride;
     auto go = [&](const auto &U) {
         MultishiftState *ms = (MultishiftState *)state;
-        return even_odd ? run_ms<true>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, blocks,
-                                       steps, U, st)
-                        : run_ms<false>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, blocks,
-                                        steps, U, st);
+        return even_odd ? run_ms<true>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, wait,
+                                       blocks, steps, U, st)
+                        : run_ms<false>(P, Ti, p0, p1, q, tmp, ring, x, dir, nshift, ms, partials, arrived, err, wait,
+                                        blocks, steps, U, st);
     };
     return P.rep == REP_SU3 ? go(GaugeD18{(const double2 *)P.U->d64, s}) : go(GaugeD9{(const double *)P.U->d64, s});
 }

@@ -1,8 +1,9 @@
 """Failures made on the host, never on the GPU: a source with NaN or Inf entries, a step
 limit of one, an unreachable tolerance, a BiCGStab breakdown (rho = 0), a device
 allocation that fails inside a server lane (an injected error code in place of a failing
-cudaMalloc), and a bulk-copy wait of the batched stencil reported as given up (the host's
-reading of the kernel's status word faked).  Each must end its own solve or request with a status while everything else
+cudaMalloc), a bulk-copy wait of the batched stencil reported as given up (the host's
+reading of the kernel's status word faked), and a wait between the blocks of a one-launch
+solver that looks for one arrival too many and runs out.  Each must end its own solve or request with a status while everything else
 completes within tolerance; the reference returns false on the same inputs
 (ConjugateGradient.cpp:70-73, BiConjugateGradient.cpp:381-384, 503-506), pinned here
 through its compiled code where it runs."""
@@ -304,3 +305,45 @@ def test_bulk_copy_wait_timeout_fails_the_call(su3, oracle):
         set_batch_tile(lat, -1, 0)
     for x, y in zip(xs, got):
         assert np.linalg.norm(y - D.multiply(x)) / np.linalg.norm(D.multiply(x)) < 1e-6
+
+
+def test_one_launch_wait_runs_out(oracle):
+    """A wait between the blocks of a one-launch solver looks for one arrival more than there are
+    and gives up: the kernel ends by itself, the solve runs again with launches per iteration and
+    gives the same result, and the context's next solve takes one launch again."""
+    lib = L.lib()
+
+    def launches(lat, f):
+        n = lib.lym_context_kernel_launches(lat.handle)
+        f()
+        return lib.lym_context_kernel_launches(lat.handle) - n
+
+    for kind in ("SquareImproved", "SquareEvenOddImproved"):
+        lat, op, orc = _multishift((4, 4, 4, 6), kind, 0.12, oracle)
+        try:
+            b = synth.gaussian_spinor((4, 4, 4, 6), 3, 84)
+            eps = 1e-22 * float(np.vdot(b, b).real)
+            cg, x = L.ConjugateGradient(), lat.new_vector()
+            ms, sols = L.MultishiftSolver.getInstance("multishift_cg"), []
+            cg.setPrecision(eps)
+            ms.setPrecision(eps)
+
+            def run_cg():
+                assert cg.solve(op, b, x)
+
+            def run_ms():
+                assert ms.solve(op, b, sols, [0.0, 0.3])
+
+            for run, residuals in ((run_cg, lambda: [orc.multiply(x) - b]),
+                                   (run_ms, lambda: [orc.multiply(y) + s * y - b for y, s in zip(sols, (0.0, 0.3))])):
+                if kind == "SquareEvenOddImproved" and run is run_cg:
+                    continue  # launches per iteration in any case
+                one = launches(lat, run)
+                assert lib.lym_context_inject_one_launch_give_ups(lat.handle, 1) == OK
+                again = launches(lat, run)
+                assert again > one + 100, (one, again)
+                assert max(np.linalg.norm(r) for r in residuals()) <= 5e-11 * np.linalg.norm(b)
+                assert launches(lat, run) == one
+                assert max(np.linalg.norm(r) for r in residuals()) <= 5e-11 * np.linalg.norm(b)
+        finally:
+            lat.close()
