@@ -2219,13 +2219,15 @@ public:
         for (BVec *v : {&xs, &rs, &ps, &aps, &tes, &tos}) CK(cudaMemsetAsync(v->s.v, 0, v->bytes, c->st));
         memset(&hs, 0, sizeof(hs));
         hs.nb = nb;
-        // Reliable update when the recursive residual fell by 100x (FP16 inner storage; the residual
-        // is FP32) or 300x (FP32): the rounding drift of the recursion stays below that.  FP32, 12
-        // sources at 24^3 x 48: 4-5 updates each against 5-6 at 100x, iterations and residuals
-        // alike; 1000x begins to cost iterations at 16^3 x 32, kappa 0.135.  FP16, 12 sources at
-        // 16^3 x 32: 5 updates against 9 at 10x, iterations alike, 34 against 42 ms at kappa 0.12
-        // and 66 against 76 at 0.135; 300x costs iterations there (67.6 ms).
-        hs.delta2 = sprec == PREC_H ? 1e-4 : LYM_BLOCK_DELTA2_F;
+        // Reliable update when the recursive residual fell by 30x (FP16 inner storage; the residual is
+        // FP32) or 300x (FP32).  The lines lie where the error of the solutions does not grow; against
+        // the next finer threshold, error against 64 bits (mean ratio over groups of 16 sources,
+        // three lattices), updates a source:
+        //   FP16, kappa 0.12 and 0.124: 30x against 10x 0.998 +- 0.013, 6.0 and 8.2; 100x against 10x
+        //     1.043 +- 0.014, 4.9 (and 300x costs iterations at kappa 0.135);
+        //   FP32, kappa 0.12 to 0.134: 300x against 100x 1.006 +- 0.007, 4.0 and 5.0, 34.6 iterations
+        //     either way; 1000x begins to cost iterations at 16^3 x 32, kappa 0.135.
+        hs.delta2 = sprec == PREC_H ? 1e-3 : LYM_BLOCK_DELTA2_F;
         static_assert(sizeof(BatchCGState) <= kStateBytes, "state buffer too small");
     }
     ~BlockEngine()

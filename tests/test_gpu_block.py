@@ -80,3 +80,23 @@ def test_block_bicgstab_fused_omega_matches_separate_pass(setup, minb):
         assert np.array_equal(x, y)
     for x, y in zip(a, out[1][0][0]):
         assert rel(x, y) < 1e-8
+
+
+@pytest.mark.parametrize("mode,decades", [("half", 1.6), ("single", 2.5)])
+def test_block_reliable_updates_are_close_enough(oracle, mode, decades):
+    """The recursion of a source runs over no more than 1.5 decades of the residual with FP16
+    storage (2.5 with FP32) between updates from the FP64 residual: beyond that the solutions' error
+    grows, by 4 % after two decades with FP16."""
+    dims = (8, 8, 12, 16)
+    lat = L.Lattice(dims, "su3")
+    try:
+        op = L.ImprovedDiracWilsonOperator(lat, 0.122, 1.7, gamma5=False)
+        op.setLattice(synth.fermion_links(dims, "su3", 0.25, 33))
+        srcs = [synth.gaussian_spinor(dims, 3, 200 + k) for k in range(16)]
+        s = L.EvenOddBiCGStab(mode, 1e-10)
+        ok, _ = s.solve_block(op, srcs, batch=16)
+        assert ok
+        # an update passes its threshold by part of an iteration's fall, the last one ends the solve
+        assert np.mean([st.reliable_updates for st in s.block_stats]) >= 10.0 / decades - 0.6
+    finally:
+        lat.close()
