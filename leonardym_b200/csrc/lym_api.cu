@@ -2198,8 +2198,12 @@ public:
     BlockEngine(lym_context *ctx, int sprec_, int nb_, int algo_ = ALGO_CG)
         : c(ctx), sprec(sprec_), nb(nb_), algo(algo_), te(ctx, PREC_D, 1), t1(ctx, PREC_D, 1), rS(ctx, PREC_D, 1),
           rN(ctx, PREC_D, 1), xs(ctx, PREC_F, nb_), rs(ctx, PREC_F, nb_), ps(ctx, sprec_, nb_), aps(ctx, sprec_, nb_),
-          tes(ctx, sprec_, nb_), tos(ctx, sprec_, nb_)
+          tes(ctx, sprec_, nb_), tos(ctx, sprec_, nb_), tables_mem(ctx, kTableBytes)
     {
+        // BiCGStab updates up to kUpdates parked slots together, a residual vector each, 256 MiB in all
+        if (algo == ALGO_BICGSTAB)
+            update_group = std::min<size_t>(
+                kUpdates, std::max<size_t>(1, ((size_t)256 << 20) / spinor_bytes(c->g, PREC_D, 1)));
         if (algo == ALGO_BICGSTAB) {
             svec.reset(new BVec(c, sprec, nb));
             rhat.reset(new BVec(c, PREC_F, nb));
@@ -2210,12 +2214,11 @@ public:
                 what_c[j].reset(new Vec(c, PREC_F, 1));
             }
         }
-        tables = (char *)dev_alloc(c, kTableBytes);
+        tables = (char *)tables_mem.p;
         d_b = (double *)tables;
         d_T = (const void **)(tables + kMaxBatch * sizeof(double));
         d_Ti = (const void **)(tables + 2 * kMaxBatch * sizeof(double));
         d_uniform = (int *)(tables + 3 * kMaxBatch * sizeof(double));
-        CK(cudaMemsetAsync(tables, 0, kTableBytes, c->st));
         for (BVec *v : {&xs, &rs, &ps, &aps, &tes, &tos}) CK(cudaMemsetAsync(v->s.v, 0, v->bytes, c->st));
         memset(&hs, 0, sizeof(hs));
         hs.nb = nb;
@@ -2235,7 +2238,6 @@ public:
         for (auto e : exec)
             if (e) cudaGraphExecDestroy(e);
         for (int j = 0; j < nb; ++j) delete slot[j].bp;
-        dev_free(c, tables, kTableBytes);
     }
 
     int free_slot() const
@@ -2389,8 +2391,11 @@ private:
     // rounded values), which a reliable update reads coalesced: in the pair layout one
     // right-hand side is 8 bytes of every 32-byte sector it touches
     std::unique_ptr<Vec> rhat_c[kMaxBatch], what_c[kMaxBatch];
+    static constexpr int kUpdates = 8;
+    size_t update_group = 1;                 // parked slots updated together
     std::unique_ptr<DevBuf> om_scratch;      // BiCGStab: partial omega sums of the fused stencil epilogue
     static constexpr size_t kTableBytes = 3 * kMaxBatch * sizeof(double) + 16;
+    DevBuf tables_mem;
     char *tables = nullptr;
     double *d_b = nullptr;
     const void **d_T = nullptr, **d_Ti = nullptr;
@@ -2507,17 +2512,29 @@ private:
         hs.restart[j] = 0;
         hs.active[j] = 1;
     }
+    // The residual vectors of up to n slots that are updated together: rS, and others from the pool
+    // as far as there is memory.  The pool gives them back where a new source needs the memory.
+    std::vector<std::unique_ptr<Vec>> more_residuals(size_t n)
+    {
+        std::vector<std::unique_ptr<Vec>> v;
+        const std::string err = c->err;
+        try {
+            while (v.size() + 1 < n) v.emplace_back(new Vec(c, PREC_D, 1));
+        } catch (const LymError &e) {
+            if (e.code != LYM_ERR_MEMORY) throw;
+            c->err = err;
+            update_group = v.size() + 1;  // not asked for again
+        }
+        return v;
+    }
     // The reliable updates of several parked slots together: their true residuals, then, for
     // those that go on, the continuation of the recursion, with one host round trip each.
-    static constexpr int kUpdates = 8;  // at most; a residual vector each
-    void reliable_updates_bicg(const std::vector<int> &js)
+    void reliable_updates_bicg(const std::vector<int> &js, const std::vector<std::unique_ptr<Vec>> &more)
     {
         const int n = (int)js.size();
-        std::vector<std::unique_ptr<Vec>> more;  // the first slot's residual is rS
         std::vector<Spinor> res;
         for (int i = 0; i < n; ++i) {
-            if (i > 0) more.emplace_back(new Vec(c, PREC_D, 1));
-            res.push_back(i > 0 ? **more.back() : *rS);
+            res.push_back(i > 0 ? **more[i - 1] : *rS);
             const int j = js[i];
             Slot &s = slot[j];
             // x += the FP32 accumulator (unless a non-finite recursion (restart 2) drops it); the
@@ -2602,17 +2619,16 @@ private:
         std::vector<int> parked;
         for (int j = 0; j < nb; ++j)
             if (slot[j].busy && !slot[j].finished && hs.need_update[j]) parked.push_back(j);
-        // BiCGStab: as many together as there is scratch for (a residual each, 256 MiB in all)
-        const size_t most = std::max<size_t>(1, ((size_t)256 << 20) / spinor_bytes(c->g, PREC_D, 1));
-        const size_t group = algo == ALGO_BICGSTAB ? std::min<size_t>(kUpdates, most) : 1;
-        for (size_t i = 0; i < parked.size(); i += group) {
-            const std::vector<int> js(parked.begin() + i, parked.begin() + std::min(parked.size(), i + group));
-            if (algo == ALGO_BICGSTAB) reliable_updates_bicg(js);
+        for (size_t i = 0; i < parked.size();) {
+            const auto more = more_residuals(std::min(update_group, parked.size() - i));
+            const std::vector<int> js(parked.begin() + i, parked.begin() + i + 1 + more.size());
+            if (algo == ALGO_BICGSTAB) reliable_updates_bicg(js, more);
             else reliable_update(js[0]);
             for (int j : js) {
                 c->engine_stats[6] += 1;
                 if (!slot[j].finished && hs.its[j] >= slot[j].max_iter) finish(j);
             }
+            i += js.size();
         }
         c->engine_stats[1] += wall() - t0;
     }

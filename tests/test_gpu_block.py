@@ -100,3 +100,28 @@ def test_block_reliable_updates_are_close_enough(oracle, mode, decades):
         assert np.mean([st.reliable_updates for st in s.block_stats]) >= 10.0 / decades - 0.6
     finally:
         lat.close()
+
+
+def test_block_updates_go_on_without_memory(setup):
+    """Identical sources all wait for their reliable update at once, and updates done together take a
+    vector each: where no memory is left for these, the updates go one by one and the solve ends as
+    ever.  (One step with all sources first, so that nothing else is left to allocate.)"""
+    lat, b = setup["lat"], setup["srcs"][4]
+    s = L.EvenOddBiCGStab("single", 1e-10)
+    L.lib().lym_context_trim(lat.handle)
+    s.maxSteps = 1
+    assert not s.solve_block(setup["op"], [b] * 16, batch=16)[0]
+    s.maxSteps = 20000
+    held = L.lib().lym_context_device_bytes(lat.handle)
+    try:
+        assert L.lib().lym_context_inject_alloc_failures(lat.handle, 1000) == 0
+        ok, sols = s.solve_block(setup["op"], [b] * 16, batch=16)
+    finally:
+        L.lib().lym_context_inject_alloc_failures(lat.handle, 0)
+    assert ok
+    for x in sols:
+        assert np.linalg.norm(b - setup["D"].multiply(x)) <= 1e-10 * np.linalg.norm(b)
+    assert L.lib().lym_context_device_bytes(lat.handle) == held
+    # with memory the next solve does take the vectors
+    assert s.solve_block(setup["op"], [b] * 16, batch=16)[0]
+    assert L.lib().lym_context_device_bytes(lat.handle) > held
