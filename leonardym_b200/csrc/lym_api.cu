@@ -1180,24 +1180,17 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
 // accumulators) and the directions
 template <class View> struct MsViews {
     lym_context *c;
+    DevBuf mem;
     View *ring, *x, *p;
     static constexpr size_t kBytes = (kMsWin + 1 + 2 * kMaxShifts) * sizeof(View);
     MsViews(lym_context *ctx, const std::vector<View> &hring, const std::vector<View> &hx, const std::vector<View> &hp)
-        : c(ctx), ring((View *)dev_alloc(ctx, kBytes)), x(ring + kMsWin + 1), p(x + kMaxShifts)
+        : c(ctx), mem(ctx, kBytes, false), ring((View *)mem.p), x(ring + kMsWin + 1), p(x + kMaxShifts)
     {
-        try {
-            CK(cudaMemcpyAsync(ring, hring.data(), hring.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(x, hx.data(), hx.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(p, hp.data(), hp.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
-            CK(cudaStreamSynchronize(c->st));
-        } catch (...) {
-            dev_free(c, ring, kBytes);
-            throw;
-        }
+        CK(cudaMemcpyAsync(ring, hring.data(), hring.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(x, hx.data(), hx.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(p, hp.data(), hp.size() * sizeof(View), cudaMemcpyHostToDevice, c->st));
+        CK(cudaStreamSynchronize(c->st));
     }
-    ~MsViews() { dev_free(c, ring, kBytes); }
-    MsViews(const MsViews &) = delete;
-    MsViews &operator=(const MsViews &) = delete;
     // the window's updates of every shift, then a new window (words: of one vector)
     template <class W, class R> void flush(MultishiftState *S, int nshift, int words) const
     {
@@ -1211,7 +1204,9 @@ template <class View> struct MsViews {
 // Multishift CG on (A + shift_i), A Hermitian positive definite (a Square* kind), in FP64.  The
 // shifted x_i and p_i are updated once per kMsWin steps from a ring of residuals
 // (multishift_cg_mixed tells how): 4 of their vectors move per window instead of per step.  Small
-// lattices run all steps in one launch (lym_persist.cu).
+// lattices run all steps in one launch (lym_persist.cu).  Where there is no memory for the ring and
+// a base direction of its own, every entry of the ring is the one residual, which a step updates in
+// place, the window is one step, and the base direction is that of its shift.
 int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts, double eps, int max_steps,
                   const Spinor &b, std::vector<Spinor> &xs, lym_solve_stats *st)
 {
@@ -1220,41 +1215,62 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
     for (int i = 1; i < nshift; ++i)
         if (shifts[i] < shifts[base]) base = i;
     const double s0 = shifts[base];
-    const bool square = is_hermitian_square(op);
-    std::vector<std::unique_ptr<Vec>> owned;
-    auto fresh = [&]() {
-        owned.emplace_back(new Vec(c, PREC_D, 2));
-        return **owned.back();
-    };
-    std::vector<SpinorD> hring, hx, hp;
-    for (int j = 0; j <= kMsWin; ++j) hring.push_back(fresh().d());
-    const Spinor r0 = **owned[0];
-    for (int i = 0; i < nshift; ++i) {
-        zero(c, xs[i]);
-        hx.push_back(xs[i].d());
-        hp.push_back(fresh().d());
-    }
-    // the base direction of the current step (the operator's input), and A p or Q p
-    Vec pcur(c, PREC_D, 2), ap(c, PREC_D, 2);
-    std::unique_ptr<Vec> te;
-    if (square && is_even_odd(op.kind)) te.reset(new Vec(c, PREC_D, 1));
-    const Spinor half = te ? **te : Spinor();
-    const Spinor pb = *pcur;
-    const MsViews<SpinorD> views(c, hring, hx, hp);
+    for (int i = 0; i < nshift; ++i) zero(c, xs[i]);
     const double bb = norm2_now(c, b);
     if (!std::isfinite(bb)) {
         c->err = "the source has non-finite entries";
         if (st) st->last_error = bb;
         return LYM_NOT_CONVERGED;
     }
-    // build the clover term and pool the operator's temporaries before graph capture
-    op_apply(c, op, PREC_D, *ap, b, &b, C2(s0));
+    const bool square = is_hermitian_square(op), eo = is_even_odd(op.kind);
+    std::vector<std::unique_ptr<Vec>> dirs, more;  // more: residuals 1..kMsWin, the base direction
+    for (int i = 0; i < nshift; ++i) dirs.emplace_back(new Vec(c, PREC_D, 2));
+    Vec r0(c, PREC_D, 2), ap(c, PREC_D, 2);  // ap: A p or Q p
+    std::unique_ptr<Vec> te, p1;
+    if (square && eo) te.reset(new Vec(c, PREC_D, 1));
+    const Spinor half = te ? **te : Spinor();
+    std::unique_ptr<DevBuf> sums;
+    std::unique_ptr<MsViews<SpinorD>> view_mem;
+    const int blocks = square ? ms_persist_blocks(c->g, c->rep, c->device, eo) : 0;
+    auto set_up = [&]() {
+        std::vector<SpinorD> hring, hx, hp;
+        for (int j = 0; j <= kMsWin; ++j) hring.push_back(j > 0 && !more.empty() ? (**more[j - 1]).d() : (*r0).d());
+        for (int i = 0; i < nshift; ++i) {
+            hx.push_back(xs[i].d());
+            hp.push_back((**dirs[i]).d());
+        }
+        view_mem.reset(new MsViews<SpinorD>(c, hring, hx, hp));
+        // build the clover term and pool the operator's temporaries before graph capture
+        if (!square) op_apply(c, op, PREC_D, *ap, b, &b, C2(s0));
+        else if (kind_has_clover(op.kind)) ensure_clover(c, op);
+    };
+    const std::string err = c->err;
+    try {
+        for (int j = 0; j <= kMsWin; ++j) more.emplace_back(new Vec(c, PREC_D, 2));
+        if (blocks > 0) {
+            p1.reset(new Vec(c, PREC_D, 2));
+            sums.reset(new DevBuf(c, 2 * (size_t)blocks * sizeof(double), false));
+        }
+        set_up();
+    } catch (const LymError &e) {
+        if (e.code != LYM_ERR_MEMORY) throw;
+        c->err = err;
+        more.clear();
+        p1.reset();
+        sums.reset();
+        set_up();
+    }
+    const MsViews<SpinorD> &views = *view_mem;
+    const bool windowed = !more.empty();
+    const int win = windowed ? kMsWin : 1;
+    // the base direction of the current step (the operator's input)
+    const Spinor pb = windowed ? **more[kMsWin] : **dirs[base];
     auto start = [&]() {  // x_i = 0, r_0 = p_i = b
-        copy(c, r0, b);
+        copy(c, *r0, b);
         copy(c, pb, b);
         for (int i = 0; i < nshift; ++i) {
             zero(c, xs[i]);
-            copy(c, **owned[kMsWin + 1 + i], b);
+            copy(c, **dirs[i], b);
         }
         MultishiftState &H = *(MultishiftState *)c->h_state;
         memset(&H, 0, sizeof(H));
@@ -1290,24 +1306,20 @@ int multishift_cg(lym_context *c, OpEntry &op, int nshift, const double *shifts,
             run_site(c, OpMsAlpha<SpinorD, SpinorD>{pb.d(), (*ap).d(), S}, 2, Gate{&S->stop, nullptr, &S->pause});
             run_site(c, OpMsResidualRing<SpinorD, SpinorD>{views.ring, (*ap).d(), S}, 2, Gate{&S->stop, nullptr});
         }
-        run_site(c, OpMsBaseDirection<SpinorD, SpinorD>{views.ring, pb.d(), S}, 2, gate);
-        if (++nstep % kMsWin == 0) views.template flush<double2, double>(S, nshift, 2 * 12 * c->g.stride);
+        if (windowed) run_site(c, OpMsBaseDirection<SpinorD, SpinorD>{views.ring, pb.d(), S}, 2, gate);
+        if (++nstep % win == 0) views.template flush<double2, double>(S, nshift, 2 * 12 * c->g.stride);
     };
     int rc = LYM_OK;
-    const bool eo = is_even_odd(op.kind);
-    const int blocks = square ? ms_persist_blocks(c->g, c->rep, c->device, eo) : 0;
     if (bb > 0 && max_steps > 0) {
         bool done = false;
-        if (blocks > 0) {
+        if (blocks > 0 && windowed) {
             DslashParams P = full_params(c, op, PREC_D, 1, C2(0.0), nullptr);
             P.sigma = s0;
             if (eo) P.b = -op.kappa * op.kappa;
             const void *Ti = eo && kind_has_clover(op.kind) ? op.clover.Tinv[PREC_D] : nullptr;
-            Vec p1(c, PREC_D, 2);
-            DevBuf sums(c, 2 * (size_t)blocks * sizeof(double), false);
             done = run_one_launch(c, max_steps, [&](int steps, BarrierWait wait, int *err) {
-                return launch_ms_persist(P, Ti, eo, pb, *p1, *ap, half, views.ring, views.x, views.p, nshift, S,
-                                         (double *)sums.p, c->counter + 8, err, wait, blocks, steps, c->st);
+                return launch_ms_persist(P, Ti, eo, pb, **p1, *ap, half, views.ring, views.x, views.p, nshift, S,
+                                         (double *)sums->p, c->counter + 8, err, wait, blocks, steps, c->st);
             }, S);
             if (!done) start();
         }

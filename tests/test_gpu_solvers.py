@@ -517,3 +517,55 @@ def test_one_launch_solvers_of_two_threads(oracle):
     finally:
         lat_a.close()
         lat_b.close()
+
+
+@pytest.mark.parametrize("kind", ["SquareEvenOddImproved", "SquareImproved"])
+def test_multishift_without_memory_for_its_window(kind, oracle):
+    """Where there is no memory for the ring of residuals, the FP64 multishift updates its shifted
+    vectors every step: the same iterates and solutions from ten vectors less.  (A solve with one
+    shift first leaves 15 full vectors behind; four shifts take 11 without the ring.)"""
+    dims, kappa, csw = (4, 4, 4, 6), 0.12, 1.0
+    links = synth.fermion_links(dims, "su3", 0.3, 85)
+    lat = L.Lattice(dims, "su3")
+    lib = L.lib()
+    try:
+        op = {"SquareImproved": L.SquareImprovedDiracWilsonOperator,
+              "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind](lat, kappa, csw)
+        op.setLattice(lat.upload(links))
+        orc = oracle.Operator(oracle.Geometry(dims), links, kind, kappa, csw, True)
+        b = synth.gaussian_spinor(dims, 3, 86)
+        eps = 1e-22 * float(np.vdot(b, b).real)
+        ms = L.MultishiftSolver.getInstance("multishift_cg")
+
+        def solve(shifts):
+            sols, n = [], lib.lym_context_kernel_launches(lat.handle)
+            ok = ms.solve(op, b, sols, shifts)
+            return ok, sols, lib.lym_context_kernel_launches(lat.handle) - n
+
+        shifts = [0.3, 0.02, 1e-3, 0.0]
+        for eps_k, steps in ((eps, 3000), (0.0, 1), (0.0, 7), (0.0, 8), (0.0, 9)):
+            lib.lym_context_trim(lat.handle)
+            ms.setPrecision(eps)
+            ms.setMaxSteps(3000)
+            one = solve([0.0])[2]
+            ms.setPrecision(eps_k)
+            ms.setMaxSteps(steps)
+            try:
+                assert lib.lym_context_inject_alloc_failures(lat.handle, 1000) == 0
+                ok, sols, launches = solve(shifts)
+            finally:
+                lib.lym_context_inject_alloc_failures(lat.handle, 0)
+            assert launches > one + 8  # not the one-launch form
+            if eps_k > 0.0:
+                assert ok
+                for x, s in zip(sols, shifts):
+                    assert rel(orc.multiply(x) + s * x, b) < 5e-11
+            else:
+                assert not ok and ms.stats.iterations == steps
+                xo = oracle.cg(orc, b, 0.0, steps, guess=np.zeros_like(b))[1]
+                assert rel(sols[3], xo) < 1e-11
+            again = solve(shifts)[1]  # with memory: the window's updates
+            for x, y in zip(sols, again):
+                assert rel(x, y) < (1e-9 if ok else 1e-11)
+    finally:
+        lat.close()
