@@ -91,3 +91,28 @@ def test_chiral_condensate(setup, oracle):
         assert np.max(np.abs(got - ref)) <= 1e-8 * np.max(np.abs(ref))
     est = res["estimators"]
     assert abs(res["condensate"]["re"] - est[:, 0].mean()) < 1e-14 * abs(est[:, 0]).max()
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 8, 4), (16, 16, 32, 2), (2, 2, 2, 66), (4, 8, 16, 130)])
+def test_slice_sums_keep_small_terms(dims):
+    """The sites of a time slice are added in short chains: one site of value 1 and q everywhere else,
+    q just under half a unit in the last place of 1, which a chain that starts from the 1 loses
+    whole.  Bound: the additions of the longest chain, each to half a unit."""
+    lat = L.Lattice(dims, "su3")
+    try:
+        lines, Lt = lat.V // dims[3], dims[3]
+        props = [np.zeros((lat.V, 4, 3), np.complex128) for _ in range(12)]
+        root = 43.0 / 32.0 * 2.0 ** -27  # its square is exact
+        props[0][:, 0, 0] = root
+        props[0][:Lt, 0, 0] = 1.0
+        out = [np.zeros(Lt) for _ in range(3)]
+        rc = L.lib().lym_meson_contractions(lat.handle, (C.c_void_p * 12)(*[p.ctypes.data for p in props]),
+                                            *[o.ctypes.data_as(C.c_void_p) for o in out])
+        assert rc == 0
+        groups = 256 // min(Lt, 64)
+        chain = np.ceil(np.ceil(lines / min(lines, 128)) / groups) + np.ceil(np.log2(groups)) + 9
+        q = root * root
+        # 1 + (lines - 1) q without rounding the excess over 1
+        assert np.max(np.abs((out[0] - 1.0) - (lines - 1) * q)) <= chain * 2.0 ** -53
+    finally:
+        lat.close()
