@@ -3105,8 +3105,14 @@ int lym_operator_destroy(lym_context *c, int op_id)
 // An operator application reads the caller's AoS input straight into the stencil up to this many
 // sites, instead of packing it first: a launch less, but a 32-byte sector per 16 bytes asked for.
 // us a call, packed and direct: 8^4 21.7 and 17.1, 8^3 x 16 22.5 and 20.0, 12^4 27.4 and 26.3
-// (adjoint 26.7 and 28.5), 12^3 x 24 34.4 and 39.8.
+// (adjoint 26.7 and 28.5), 12^3 x 24 34.4 and 39.8.  Extents are even: across an odd one the
+// packed stencil takes the neighbour from the other parity's half-sites, the AoS vector holds the
+// neighbour itself, and an application is the operator that the solvers use.
 constexpr int kAosInputSites = 12288;
+static bool reads_aos_input(const Geom &g)
+{
+    return g.V <= kAosInputSites && !((g.L[0] | g.L[1] | g.L[2] | g.L[3]) & 1);
+}
 
 static int do_multiply(lym_context *c, int op_id, int prec, double *out, const double *v1, const double *v2,
                        double2 alpha, bool device_ptr)
@@ -3131,7 +3137,7 @@ static int do_multiply(lym_context *c, int op_id, int prec, double *out, const d
                 CK(cudaMemcpyAsync(staging(c, 1), v2, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
                 add = c->aos[1];
             }
-            if ((op.kind == LYM_OP_DIRAC_WILSON || op.kind == LYM_OP_IMPROVED) && c->g.V <= kAosInputSites &&
+            if ((op.kind == LYM_OP_DIRAC_WILSON || op.kind == LYM_OP_IMPROVED) && reads_aos_input(c->g) &&
                 !(device_ptr && overlap(v1, out))) {
                 // one launch, from AoS vector to AoS vector
                 const double *src = v1;

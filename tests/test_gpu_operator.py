@@ -304,3 +304,52 @@ def test_input_read_in_place_or_packed(kind, rep, dims, oracle):
             assert rel(out.cpu().numpy(), ref) < 1e-13
     finally:
         lat.close()
+
+
+@pytest.mark.parametrize("dims", [(3, 2, 4, 6), (4, 5, 2, 4), (2, 2, 3, 10), (3, 5, 7, 2), (4, 2, 6, 4)])
+@pytest.mark.parametrize("kind", ["DiracWilson", "Improved", "SquareImproved"])
+def test_odd_extents_are_one_operator(kind, dims):
+    """With odd space extents too every way of applying an operator gives the same vector: apart,
+    over the input (packed first), with an added vector that overlaps the result (the general
+    path), and twice for the square."""
+    import ctypes as C
+
+    import torch
+    links = synth.fermion_links(dims, "su3", 0.4, 51)
+    lat = L.Lattice(dims, "su3")
+    try:
+        gid = lat.upload(links)
+
+        def make(kind):
+            op = GPU_CLASS[kind](lat)
+            op.setKappa(0.14)
+            if kind != "DiracWilson":
+                op.setCSW(1.1)
+            op.setLattice(gid)
+            return op
+
+        op = make(kind)
+        x = synth.gaussian_spinor(dims, 3, 52)
+
+        def call(op, out, v, add=None):
+            torch.cuda.synchronize()
+            p = [C.c_void_p(t.data_ptr()) for t in (out, v)]
+            if add is None:
+                rc = L.lib().lym_multiply_device(lat.handle, op.op_id, *p)
+            else:
+                rc = L.lib().lym_multiply_add_device(lat.handle, op.op_id, *p, C.c_void_p(add.data_ptr()), 0.0, 0.0)
+            assert rc == 0
+            return out.cpu().numpy()
+
+        dx = torch.from_numpy(x).cuda()
+        apart = call(op, torch.empty_like(dx), dx)
+        over = torch.from_numpy(x).cuda()
+        buf = torch.zeros((lat.V + 1, 4, 3), dtype=torch.complex128, device="cuda")
+        assert rel(call(op, over, over), apart) < 1e-14
+        assert rel(call(op, buf[:-1], dx, buf[1:]), apart) < 1e-14
+        if kind == "SquareImproved":
+            d = make("Improved")
+            once = call(d, torch.empty_like(dx), dx)
+            assert rel(call(d, torch.empty_like(dx), torch.from_numpy(once).cuda()), apart) < 1e-13
+    finally:
+        lat.close()
