@@ -313,12 +313,11 @@ void copy(lym_context *c, const Spinor &dst, const Spinor &src)
     launch_convert(c->g, dst, src, c->st);
 }
 
-// the FP64 x of one parity plus an accumulator of another precision, which starts again from zero
+// the FP64 x of one parity plus an accumulator (FP64 or FP32), which starts again from zero
 void fold(lym_context *c, const Spinor &acc, const Spinor &x)
 {
     if (acc.prec == PREC_D) run_site(c, OpFoldClear<SpinorD, SpinorD>{acc.d(), x.d()}, 1);
-    else if (acc.prec == PREC_F) run_site(c, OpFoldClear<SpinorF, SpinorD>{acc.f(), x.d()}, 1);
-    else run_site(c, OpFoldClear<SpinorH, SpinorD>{acc.h(), x.d()}, 1);
+    else run_site(c, OpFoldClear<SpinorF, SpinorD>{acc.f(), x.d()}, 1);
 }
 
 // CG going on after a reliable update with the FP64 residual rt: r = rt, p = rt + b p (r FP32
