@@ -569,3 +569,81 @@ def test_multishift_without_memory_for_its_window(kind, oracle):
                 assert rel(x, y) < (1e-9 if ok else 1e-11)
     finally:
         lat.close()
+
+
+# CG on the squared kinds takes one launch of 2 blocks per SM up to 148 * 64 = 9472 sites, of 4 up to
+# 18944, and launches per iteration above; the FP64 multishift one launch up to 37888 sites.
+@pytest.mark.parametrize("rep", ["su3", "su2adj"])
+@pytest.mark.parametrize("dims", [(8, 8, 8, 18), (8, 8, 8, 20), (6, 8, 14, 28), (8, 8, 8, 38)])
+@pytest.mark.parametrize("kind", ["SquareDiracWilson", "SquareImproved"])
+def test_square_cg_of_every_size(rep, dims, kind, oracle):
+    kappa, csw = (0.12, 1.0) if rep == "su3" else (0.15, 1.2)
+    lat, op, orc = _square_operator(dims, rep, kind, kappa, csw, 95, oracle)
+    try:
+        b = synth.gaussian_spinor(dims, 3, 96)
+        eps = 1e-22 * float(np.vdot(b, b).real)
+        cg = L.ConjugateGradient()
+        cg.setPrecision(eps)
+        x, n = lat.new_vector(), L.lib().lym_context_kernel_launches(lat.handle)
+        assert cg.solve(op, b, x)
+        n = L.lib().lym_context_kernel_launches(lat.handle) - n
+        assert (n < cg.stats.iterations) == (lat.V <= 18944)
+        assert rel(orc.multiply(x), b) < 1.1e-11
+        cg.setPrecision(0.0)
+        for k in (1, 6):
+            cg.setMaximumSteps(k)
+            assert not cg.solve(op, b, x)
+            assert rel(x, oracle.cg(orc, b, 0.0, k)[1]) < 1e-12
+        # with a shift, from the guess of the solver that starts at the previous shift's solution
+        ms = L.MultishiftSolver.getInstance("mass_estrapolation")
+        ms.setPrecision(eps)
+        sols = []
+        assert ms.solve(op, b, sols, [0.05, 0.3])
+        for y, s in zip(sols, (0.05, 0.3)):
+            assert rel(orc.multiply(y) + s * y, b) < 1.1e-11
+    finally:
+        lat.close()
+
+
+@pytest.mark.parametrize("rep,dims,kind", [
+    ("su3", (8, 8, 8, 40), "SquareImproved"), ("su2adj", (8, 8, 8, 40), "SquareDiracWilson"),
+    ("su3", (8, 8, 8, 74), "SquareImproved"), ("su2adj", (8, 8, 8, 74), "SquareImproved"),
+    ("su3", (8, 8, 8, 76), "SquareImproved"), ("su2adj", (8, 8, 8, 76), "SquareDiracWilson"),
+    ("su2adj", (8, 8, 8, 74), "SquareEvenOddImproved"), ("su2adj", (8, 8, 8, 76), "SquareEvenOddImproved")])
+def test_multishift_of_every_size(rep, dims, kind, oracle):
+    """Blocks that walk one tile or several, and launches per step, whose steps around the window of
+    8 are checked against the oracle's."""
+    kappa, csw = (0.12, 1.0) if rep == "su3" else (0.15, 1.2)
+    lat, op, orc = _square_operator(dims, rep, kind, kappa, csw, 97, oracle)
+    try:
+        b = synth.gaussian_spinor(dims, 3, 98)
+        eps = 1e-22 * float(np.vdot(b, b).real)
+        ms = L.MultishiftSolver.getInstance("multishift_cg")
+        ms.setMaxSteps(3000)
+        ms.setPrecision(eps)
+        shifts, sols, n = [0.3, 1e-3, 0.0], [], L.lib().lym_context_kernel_launches(lat.handle)
+        assert ms.solve(op, b, sols, shifts)
+        n = L.lib().lym_context_kernel_launches(lat.handle) - n
+        assert (n < ms.stats.iterations) == (lat.V <= 37888)
+        for x, s in zip(sols, shifts):
+            assert rel(orc.multiply(x) + s * x, b) < 5e-11
+        ms.setPrecision(0.0)
+        for k in (7, 8, 9):
+            ms.setMaxSteps(k)
+            assert not ms.solve(op, b, sols, shifts) and ms.stats.iterations == k
+            assert rel(sols[2], oracle.cg(orc, b, 0.0, k, guess=np.zeros_like(b))[1]) < 1e-11
+    finally:
+        lat.close()
+
+
+def _square_operator(dims, rep, kind, kappa, csw, seed, oracle):
+    links = synth.fermion_links(dims, rep, 0.3, seed)
+    lat = L.Lattice(dims, rep)
+    op = {"SquareDiracWilson": L.SquareDiracWilsonOperator, "SquareImproved": L.SquareImprovedDiracWilsonOperator,
+          "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind](lat)
+    op.setKappa(kappa)
+    clover = kind != "SquareDiracWilson"
+    if clover:
+        op.setCSW(csw)
+    op.setLattice(lat.upload(links))
+    return lat, op, oracle.Operator(oracle.Geometry(dims), links, kind, kappa, csw if clover else 0.0, True)
