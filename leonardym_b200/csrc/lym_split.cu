@@ -87,6 +87,14 @@ LYM_D C load_aos(const double2 *v, int word, int s)
     return C{w.x, w.y};
 }
 
+// a word of a vector that the same launch writes (load1 reads through the path for data that nothing
+// writes meanwhile)
+LYM_D C load_own(const SpinorD &v, int word, int h)
+{
+    const double2 w = v.v[(size_t)word * v.stride + h];
+    return C{w.x, w.y};
+}
+
 template <int EPI, bool AOS, int IN, class GaugeT, class Fin>
 __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<GaugeT> arg, const Fin fin)
 {
@@ -222,29 +230,40 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
         if constexpr (EPI == SPLIT_CG_UPDATE) {
             const double2 al2 = *arg.alpha;
             const C al = {al2.x, al2.y};
+            C pv[3], xv[3], rv[3];  // all read before the first is written
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
-                const C pv = load1(arg.v2[p], sp + m, h);
-                C xv = load1(arg.x[p], sp + m, h), ap = identity ? pv : res[m];
-                fma_c(xv, al, pv);
-                fma_r(ap, arg.sigma, pv);
-                const C rv = load1(arg.r[p], sp + m, h) - al * ap;
-                part += rv.re * rv.re + rv.im * rv.im;
-                put(arg.x[p], m, xv);
-                put(arg.r[p], m, rv);
+                pv[m] = load1(arg.v2[p], sp + m, h);
+                xv[m] = load_own(arg.x[p], sp + m, h);
+                rv[m] = load_own(arg.r[p], sp + m, h);
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                C ap = identity ? pv[m] : res[m];
+                fma_c(xv[m], al, pv[m]);
+                fma_r(ap, arg.sigma, pv[m]);
+                rv[m] = rv[m] - al * ap;
+                part += rv[m].re * rv[m].re + rv[m].im * rv[m].im;
+                put(arg.x[p], m, xv[m]);
+                put(arg.r[p], m, rv[m]);
             }
         } else if constexpr (EPI == SPLIT_MS_RESIDUAL) {
             const int it = arg.ms->iter;
             const SpinorD rin = arg.ring[it % (kMsWin + 1)].par(p), rout = arg.ring[(it + 1) % (kMsWin + 1)].par(p);
             const double al = arg.ms->alpha;
+            C pv[3], rv[3];  // rin may be rout
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
-                const C pv = load1(arg.v2[p], sp + m, h);
-                C ap = identity ? pv : res[m], rv = load1(rin, sp + m, h);
-                fma_r(ap, arg.sigma, pv);
-                fma_r(rv, -al, ap);
-                part += rv.re * rv.re + rv.im * rv.im;
-                put(rout, m, rv);
+                pv[m] = load1(arg.v2[p], sp + m, h);
+                rv[m] = load_own(rin, sp + m, h);
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                C ap = identity ? pv[m] : res[m];
+                fma_r(ap, arg.sigma, pv[m]);
+                fma_r(rv[m], -al, ap);
+                part += rv[m].re * rv[m].re + rv[m].im * rv[m].im;
+                put(rout, m, rv[m]);
             }
         } else {
             double pp = 0.0;
