@@ -445,7 +445,9 @@ int lym_set_link_format(lym_context *ctx, int reals);
  * The next n device allocations of the context (of the server lane holding gauge field
  * `key`) report failure as a cudaMalloc that returned cudaErrorMemoryAllocation would:
  * the call that needed the memory returns LYM_ERR_MEMORY.  No device memory or kernel is
- * involved.  A server lane fails only the request whose admission met the failure. */
+ * involved.  A server lane fails only the request whose admission met the failure.
+ * n < 0 (context only): the next -n allocations fail at first and succeed when they are tried
+ * again, after the context has given back its idle buffers, as it does when memory is short. */
 int lym_context_inject_alloc_failures(lym_context *ctx, int n);
 int lym_server_inject_alloc_failures(lym_server *server, int key, int n);
 /* The waits between the blocks of the next n one-launch solves (CG and FP64 multishift on small

@@ -81,6 +81,7 @@ struct lym_context {
     double *h_scal = nullptr;
     // host-layout staging buffers (V * 24 doubles)
     double *aos[3] = {nullptr, nullptr, nullptr};
+    bool aos_held[3] = {false, false, false};  // in use by the call that runs
     std::vector<Spinor> pool;
     // idle per-call device buffers (batched vectors, staging rings, scratch) kept for the
     // next call of the same size, like the spinor pool: given back by trim_pool
@@ -89,7 +90,8 @@ struct lym_context {
     unsigned long long launches = 0;  // kernels enqueued (graph replays count their nodes)
     double engine_stats[9] = {};      // block solves: lym_context_engine_stats
     bool capturing = false;
-    int inject_alloc_failures = 0;  // the next n device allocations report failure (tests)
+    // tests: the next n device allocations report failure; -n: fail at first, and are tried again
+    int inject_alloc_failures = 0;
     int inject_give_ups = 0;        // the next n one-launch solves' waits run out (tests)
     bool inject_copy_wait = false;  // the next check of the bulk-copy wait word reports a give-up (tests)
     int link_reals = 12;            // FP32 SU(3) link format of the single-RHS stencils: 12 or 8
@@ -153,7 +155,7 @@ void trim_pool(lym_context *c)
     }
     c->blocks.clear();
     for (int k = 0; k < 3; ++k)
-        if (c->aos[k]) {
+        if (c->aos[k] && !c->aos_held[k]) {
             cudaFree(c->aos[k]);
             c->bytes -= (size_t)c->g.V * 24 * sizeof(double);
             c->aos[k] = nullptr;
@@ -167,9 +169,11 @@ void *dev_alloc(lym_context *c, size_t bytes)
         fail(c, LYM_ERR_MEMORY, "device allocation of %zu bytes failed: injected failure", bytes);
     }
     void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
+    const bool fails_first = c->inject_alloc_failures < 0;
+    if (fails_first) ++c->inject_alloc_failures;
+    cudaError_t e = fails_first ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
     if (e == cudaErrorMemoryAllocation && !c->capturing &&
-        (!c->pool.empty() || !c->blocks.empty() || c->aos[0] || c->aos[1] || c->aos[2])) {
+        (fails_first || !c->pool.empty() || !c->blocks.empty() || c->aos[0] || c->aos[1] || c->aos[2])) {
         // the idle pooled spinors are a cache: give them back and try once more
         cudaGetLastError();
         trim_pool(c);
@@ -626,6 +630,18 @@ double *staging(lym_context *c, int k)
     if (!c->aos[k]) c->aos[k] = (double *)dev_alloc(c, (size_t)c->g.V * 24 * sizeof(double));
     return c->aos[k];
 }
+
+// A staging buffer that stays while this lives: an allocation that finds no memory gives the others
+// back (trim_pool).
+struct HeldStaging {
+    lym_context *c;
+    int k;
+    double *p;
+    HeldStaging(lym_context *ctx, int slot) : c(ctx), k(slot), p(staging(ctx, slot)) { c->aos_held[k] = true; }
+    ~HeldStaging() { c->aos_held[k] = false; }
+    HeldStaging(const HeldStaging &) = delete;
+    HeldStaging &operator=(const HeldStaging &) = delete;
+};
 
 void upload_vec(lym_context *c, const Spinor &dst, const double *src, bool device_ptr, int slot)
 {
@@ -3130,19 +3146,23 @@ static int do_multiply(lym_context *c, int op_id, int prec, double *out, const d
             upload_vec(c, **a, v1, device_ptr, 0);
         };
         if (prec == PREC_D && !parts) {
-            double *dst = device_ptr ? out : staging(c, 2);
+            std::unique_ptr<HeldStaging> result, added, input;
+            if (!device_ptr) result.reset(new HeldStaging(c, 2));
+            double *dst = device_ptr ? out : result->p;
             const double *add = v2;
             if (v2 && !device_ptr) {
-                CK(cudaMemcpyAsync(staging(c, 1), v2, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
-                add = c->aos[1];
+                added.reset(new HeldStaging(c, 1));
+                add = added->p;
+                CK(cudaMemcpyAsync(added->p, v2, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
             }
             if ((op.kind == LYM_OP_DIRAC_WILSON || op.kind == LYM_OP_IMPROVED) && reads_aos_input(c->g) &&
                 !(device_ptr && overlap(v1, out))) {
                 // one launch, from AoS vector to AoS vector
                 const double *src = v1;
                 if (!device_ptr) {
-                    CK(cudaMemcpyAsync(staging(c, 0), v1, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
-                    src = c->aos[0];
+                    input.reset(new HeldStaging(c, 0));
+                    src = input->p;
+                    CK(cudaMemcpyAsync(input->p, v1, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
                 }
                 DslashParams P = full_params(c, op, PREC_D, op.gamma5, alpha, nullptr);
                 P.parity = 2;
@@ -4311,7 +4331,6 @@ int lym_set_link_format(lym_context *c, int reals)
 
 int lym_context_inject_alloc_failures(lym_context *c, int n)
 {
-    if (n < 0) return LYM_ERR_ARGUMENT;
     return guarded(c, [&]() {
         c->inject_alloc_failures = n;
         return LYM_OK;

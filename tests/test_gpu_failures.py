@@ -1,7 +1,7 @@
 """Failures made on the host, never on the GPU: a source with NaN or Inf entries, a step
 limit of one, an unreachable tolerance, a BiCGStab breakdown (rho = 0), a device
 allocation that fails inside a server lane (an injected error code in place of a failing
-cudaMalloc), a bulk-copy wait of the batched stencil reported as given up (the host's
+cudaMalloc) or that succeeds only after idle buffers were given back, a bulk-copy wait of the batched stencil reported as given up (the host's
 reading of the kernel's status word faked), and a wait between the blocks of a one-launch
 solver that looks for one arrival too many and runs out.  Each must end its own solve or request with a status while everything else
 completes within tolerance; the reference returns false on the same inputs
@@ -280,6 +280,49 @@ def test_server_allocation_failure_fails_one_request(oracle):
         assert _residual(D3, srcs[0], solD[0]) <= 1e-10
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4, 6), (8, 8, 8, 26)])
+@pytest.mark.parametrize("kind", ["DiracWilson", "Improved", "SquareImproved", "EvenOddImproved",
+                                  "SquareEvenOddImproved"])
+def test_application_while_idle_buffers_are_given_back(kind, dims, oracle):
+    """Every allocation finds no memory at first and is tried again once the idle buffers are given
+    back: those that the application already holds stay.  Vectors read in place and packed, on the
+    host and on the device."""
+    import torch
+    cls = {"DiracWilson": L.DiracWilsonOperator, "Improved": L.ImprovedDiracWilsonOperator,
+           "SquareImproved": L.SquareImprovedDiracWilsonOperator,
+           "EvenOddImproved": L.EvenOddImprovedDiracWilsonOperator,
+           "SquareEvenOddImproved": L.SquareEvenOddImprovedDiracWilsonOperator}[kind]
+    links = synth.fermion_links(dims, "su3", 0.4, 61)
+    csw = 0.0 if kind == "DiracWilson" else 1.1
+    orc = oracle.Operator(oracle.Geometry(dims), links, kind, 0.13, csw, True)
+    x, y = (synth.gaussian_spinor(dims, 3, 62 + k) for k in range(2))
+    ref, lib = orc.multiply(x), L.lib()
+    for device in (False, True):
+        for add in (False, True):
+            if add and kind == "EvenOddImproved":
+                continue
+            lat = L.Lattice(dims, "su3")
+            try:
+                op = cls(lat)
+                op.setKappa(0.13)
+                if csw:
+                    op.setCSW(csw)
+                op.setLattice(lat.upload(links))
+                out = np.zeros_like(x)
+                arrays = [torch.from_numpy(a).cuda() for a in (out, x, y)] if device else [out, x, y]
+                torch.cuda.synchronize()
+                p = [C.c_void_p(a.data_ptr() if device else a.ctypes.data) for a in arrays]
+                name = "lym_multiply" + ("_add" if add else "") + ("_device" if device else "")
+                args = (*p, 0.3, -0.2) if add else p[:2]
+                assert lib.lym_context_inject_alloc_failures(lat.handle, -1000) == OK
+                assert getattr(lib, name)(lat.handle, op.op_id, *args) == OK
+                got = arrays[0].cpu().numpy() if device else out
+                want = ref + (0.3 - 0.2j) * y if add else ref
+                assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want), (device, add)
+            finally:
+                lat.close()
 
 
 def test_bulk_copy_wait_timeout_fails_the_call(su3, oracle):
