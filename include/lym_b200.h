@@ -232,7 +232,9 @@ int lym_solve_block_device(lym_context *ctx, int op_id, int solver, double preci
 /* ---- multishift -------------------------------------------------------------------
  * MultishiftSolver::solve(dirac, source, solutions, shifts) -> bool
  * (inverters/MultishiftSolver.h:28); the operator must be Hermitian positive
- * definite (a Square* kind).  solutions[i] receives (A + shifts[i])^{-1} source. */
+ * definite (a Square* kind).  solutions[i] receives (A + shifts[i])^{-1} source.
+ * multishift_cg: a source with non-finite entries is LYM_NOT_CONVERGED with zero solutions; after a
+ * residual that is not finite the solutions are the iterates before it. */
 int lym_multishift(lym_context *ctx, int op_id, int algorithm, int nshift, const double *shifts, double precision,
                    int max_steps, const double *source, double **solutions, lym_solve_stats *stats);
 int lym_multishift_device(lym_context *ctx, int op_id, int algorithm, int nshift, const double *shifts,

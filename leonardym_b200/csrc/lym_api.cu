@@ -1094,7 +1094,8 @@ int eo_cg(lym_context *c, OpEntry &op, int sprec, const Spinor &b, const Spinor 
           int max_steps, lym_solve_stats *st)
 {
     // FP32 keeps its recursion over two decades of the residual: adjoint 16^3 x 32, 6 updates instead
-    // of 11 at delta 0.1, 109 iterations with either
+    // of 11 at delta 0.1, 109 iterations and the same error of the solution with either (mean ratio
+    // 0.99 +- 0.01 over 24 solves).  FP16 needs more iterations from delta 0.03 on
     const double delta = sprec == PREC_D ? 0.0 : sprec == PREC_F ? 0.01 : 0.1;
     OpEntry &eo = op;  // apply_schur takes gamma5 explicitly
     if (kind_has_clover(op.kind)) ensure_clover(c, op);
@@ -1391,7 +1392,8 @@ int shift_cg_mixed(lym_context *c, OpEntry &op, int sprec, double sigma, const S
     H.rr_max = rr_true;
     H.eps = eps;
     // two decades between updates (after one, 12 shifts at 24^3 x 48: 43 updates and 182 ms a
-    // multishift solve, 32 and 175 ms now; the same iterations)
+    // multishift solve, 32 and 175 ms now; the same iterations, and the same error of the solutions
+    // to 1e-3 of it in both storages, 12^3 x 24, kappa 0.125 and 0.1365, adjoint 0.17)
     H.delta2 = sprec == PREC_D ? 0.0 : 1e-4;
     H.max_iter = iters + max_steps;
     H.iter = iters;

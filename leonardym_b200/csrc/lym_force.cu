@@ -108,8 +108,10 @@ LYM_D void subtract(double2 *out, const Mat<C> &F)
 // copies are contiguous 192-byte pieces); warps 0..3 then add the pair to M of direction mu =
 // warp, warps 4 and 5 to the P_k of one chirality (27 reals a thread).  The +t neighbour of a
 // site is the next site of the tile, except at the end of a t line or of the tile: only those
-// are copied for it.  Bound by shared memory (8 x 192 bytes written and 36 x 96 read per site
-// and pair), so the next pair's copies run during this pair's sums, two blocks per SM; the
+// are copied for it.  Bound by shared memory traffic (8 x 192 bytes written and 36 x 96 read per
+// site and pair: L1 and shared memory at half of their rate, DRAM at 43 %, FP64 at 22 %) and its
+// latency at 12 warps per SM, so the next pair's copies run during this pair's sums, two blocks
+// per SM; the
 // order of the tiles (x slowest, or columns that keep the +x neighbours in L2) made no
 // difference.  Reading the AoS spinors straight into registers instead costs one 32-byte sector
 // per lane and load, with 48 loads per pair, site and direction.
@@ -390,8 +392,9 @@ LYM_D void add_staple(const ForceArg &a, const Gauge &U, const int c[4], const i
 
 // One thread per (half-site, mu); a block's four warps take the four directions of 32
 // consecutive half-sites, whose links and plane matrices they share through L1.  Bound by FP64
-// arithmetic (about 20k fused multiply-adds per site, 0.8 ms of the chip at 24^3 x 48), so it
-// runs at 255 registers, two blocks per SM, rather than spill: 1.51 ms there (11 link products
+// arithmetic (about 20k fused multiply-adds per site, 0.8 ms of the chip at 24^3 x 48; the FP64 pipe
+// is busy half of the time with 8 warps per SM), so it runs at 252 registers, two blocks per SM,
+// rather than spill: 1.51 ms there (11 link products
 // and 10 with plane matrices per staple pair before, most of 18.9 ms).  The lower staples come
 // first: their sum L enters as -(U L U)^+.
 template <class Gauge> __global__ void __launch_bounds__(128, 2) clover_force_kernel(ForceArg a, Gauge U)

@@ -32,8 +32,8 @@ __device__ __forceinline__ double re_conj_mul(double2 a, double2 b) { return a.x
 // pieces); warp c * 3 + d then takes the 4 x 4 spin block of source colour c and sink colour d
 // of every site, and the nine warps' sums are added in order.  HBM bound: 2304 bytes a site.
 // Read straight from the AoS vectors by one thread per site, each sector of 32 bytes was
-// fetched for 16 of its bytes at a time: 377 us against 242 us at 24^3 x 48, and 62 us for
-// the time slices' sums in 48 strided blocks against 25 us.
+// fetched for 16 of its bytes at a time: 377 us against 241 us at 24^3 x 48, and 62 us for
+// the time slices' sums in 48 strided blocks against 13.5 and 2.4 us.
 constexpr int kMesonSites = 32, kMesonThreads = 288;
 constexpr int kMesonWord = 13;  // 12 words of a site, 1 of padding: conflict-free reads
 constexpr int kMesonSmem = 12 * kMesonSites * kMesonWord * 16;

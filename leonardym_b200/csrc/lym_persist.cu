@@ -12,7 +12,11 @@
 // barrier, and then runs the CG step's scalars (OpCGUpdate) on its own copy: all copies agree bit
 // for bit.  Directions alternate between two buffers and partial sums between two
 // halves, so that nobody overwrites what a slower block may still read.
-// PERSIST_TIMES
+//
+// ms a solve to 1e-10 (SquareImproved, kappa 0.12, 106 to 120 iterations), in one launch and with
+// launches per iteration (after a launch made to give up at once, about 0.1 ms): 8^4 1.17 and 2.80, 8^3 x 18 1.62 and 3.36; with 4 blocks per SM 8^3 x 20
+// 2.01 and 3.57, 6 x 8 x 14 x 28 2.63 and 4.21.  8^4 is 9.9 us an iteration: two barriers and two
+// chains of L2 loads.
 #include "lym_blas.cuh"
 #include "lym_internal.h"
 #include "lym_solver_ops.cuh"
@@ -283,8 +287,9 @@ cudaError_t run(const DslashParams &P, int minb, const Spinor &p0, const Spinor 
 // of x_i and P_i run while a block waits for the others.
 // Latency bound (a stencil phase 7 us with 128 registers a thread; polling without the acquire,
 // reads through L1 and links fetched into shared memory while waiting change nothing at the larger
-// size).  8 shifts, ms a solve against launches per step: even-odd 8^4 2.25 and 2.83,
-// 10 x 12 x 14 x 18 4.2 and 4.9, SquareImproved 8^4 2.8 and 4.6, 10 x 12 x 14 x 18 7.7 and 10.6.
+// size).  8 shifts to 1e-10, ms a solve in one launch and with launches per step as above: even-odd, kappa
+// 0.1365, 8^4 3.6 and 4.8, 10 x 12 x 14 x 18 9.4 and 11.5; SquareImproved, kappa 0.13, 8^4 3.6 and
+// 6.2, 10 x 12 x 14 x 18 10.6 and 14.9.
 template <class GaugeT> struct PersistMsArg {
     Geom g;
     GaugeT U;
@@ -566,7 +571,7 @@ cudaError_t run_ms(const DslashParams &P, const void *Ti, const Spinor &p0, cons
 
 // The grid of the one-launch multishift: a tile of either parity each, at most as many blocks as are
 // resident at once.  0 where these have more than a tile of each parity: a phase then takes two
-// rounds (even-odd 12^3 x 24, 648 tiles on 592 blocks: 7.8 against 6.1 ms with launches per step).
+// rounds (even-odd 12^3 x 24, 648 tiles on 592 blocks: 1.28 times the launches per step).
 template <bool EO, class GaugeT> int ms_blocks(const Geom &g, int device)
 {
     int sms = 0, coop = 0, per = 0;

@@ -113,8 +113,9 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split_kernel(const SplitArg<
     int p, hr;
     if (kReduce && arg.even_identity) {
         // the stencil's blocks, 32 odd half-sites each, then those of the even sites, which only
-        // stream: with both parities in a block half of its warps would idle (10 x 12 x 14 x 18:
-        // norm 15.6 against 16.6 us, residual 19.7 against 21.7)
+        // stream: with both parities in a block half of its warps would idle (10 x 12 x 14 x 18,
+        // multishift: 1.0 us of the norm's launch and 2.0 us of the residual's; these take 15.1 and
+        // 16.7 us at 12^3 x 24)
         const int odd = (g.Vh + kSplitSites - 1) / kSplitSites, blk = blockIdx.x;
         p = blk < odd ? 1 : 0;
         hr = (p ? blk : blk - odd) * kSplitSites + warp * 8 + (lane & 7);
